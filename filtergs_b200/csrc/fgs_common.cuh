@@ -398,9 +398,63 @@ __device__ __forceinline__ float3 sh_to_rgb(int deg, const float* __restrict__ s
 struct __align__(16) PairRecord {
     float4 a;  // x, y, conic.x, conic.y
     float4 b;  // conic.z, opacity, r, g
-    float4 c;  // b, gaussian id (bits), 0, 0
+    float4 c;  // b, gaussian id (bits); per Gaussian: view depth, 0; per sorted pair: quad_mask, emission index (bits)
 };
 static_assert(sizeof(PairRecord) == 48, "record size");
+
+__device__ __forceinline__ float sqrt_approx(float v)
+{
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// The 8x8 quads of the tile at (tx0, ty0) in which a Gaussian can reach alpha >= 1/255
+// at a pixel centre: bit 2 r + c for the quad of columns tx0 + 8 c .. + 7 and rows
+// ty0 + 8 r .. + 7; and kWild when its colour or position is not finite or too large for
+// arithmetic that multiplies unreached pixels by zero.  A quad outside the mask has no
+// pixel that the per-pixel tests of the compositing accept, so skipping it changes no
+// output.
+//
+// alpha >= 1/255 needs Q(d) = a dx^2 + 2 b dx dy + c dy^2 <= t0 = 2 ln(255 o).  The test
+// uses the ellipse Q <= t, t = 1.02 t0 + 0.1.  Within a strip of rows its right edge
+// x(dy) = (-b dy + sqrt(a t - det dy^2)) / a is concave with its top at
+// dy = -b x_max / c, x_max = sqrt(t c / det), so the strip's largest x is at that dy
+// clamped to the strip and to |dy| <= sqrt(t a / det); the left edge is its mirror image.
+// With det >= 2.5e-4 a c (kappa = a c / det <= 4000) the rounding of the per-pixel Q
+// (under 12 eps kappa t < 0.3%), of det (eps kappa) and of the square roots stays far
+// inside the 2% + 0.1; every quad for a conic beyond that, and for one that is not
+// positive definite.
+constexpr uint32_t kWild = 16u;
+__device__ __forceinline__ uint32_t quad_mask(const PairRecord& g, float tx0, float ty0)
+{
+    const float mx = g.a.x, my = g.a.y, a = g.a.z, b = g.a.w, c = g.b.x, o = g.b.y;
+    const bool tame = fabsf(mx) < 1e7f && fabsf(my) < 1e7f && fabsf(g.b.z) < 1e15f && fabsf(g.b.w) < 1e15f &&
+                      fabsf(g.c.x) < 1e15f;
+    const uint32_t wild = tame ? 0u : kWild;
+    if (!(o >= 1.0f / 255.0f)) return wild;  // alpha <= o
+    const float ac = a * c, det = ac - b * b;
+    const float t = 1.02f * (2.f * __logf(255.f * o)) + 0.1f;
+    const float s = __fdividef(t, det), ra = __fdividef(1.f, a);
+    const float xmax = sqrt_approx(s * c), ymax = sqrt_approx(s * a);
+    if (!(tame && a > 0.f && c > 0.f && det >= 2.5e-4f * ac && xmax < 1e7f && ymax < 1e7f && ra < 1e30f &&
+          a * t < 1e30f))
+        return wild | 15u;
+    const float ytop = -__fdividef(b * xmax, c);  // where the right edge is furthest; -ytop for the left one
+    const float X = tx0 - mx, at = a * t;
+    uint32_t m = 0;
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        const float lo = fmaxf(ty0 + 8 * r - my, -ymax), hi = fminf(ty0 + 8 * r + 7 - my, ymax);
+        const float yr = fminf(fmaxf(ytop, lo), hi), yl = fminf(fmaxf(-ytop, lo), hi);
+        const float xr = (sqrt_approx(fmaxf(at - det * yr * yr, 0.f)) - b * yr) * ra + 0.01f;
+        const float xl = -(sqrt_approx(fmaxf(at - det * yl * yl, 0.f)) + b * yl) * ra - 0.01f;
+        const bool rows = lo <= hi + 0.01f;
+        if (rows && xr >= X && xl <= X + 7.f) m |= 1u << (2 * r);
+        if (rows && xr >= X + 8.f && xl <= X + 15.f) m |= 2u << (2 * r);
+    }
+    return m;
+}
 
 // ---------------------------------------------------------------- warp helpers
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31; }

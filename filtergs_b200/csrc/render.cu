@@ -2,12 +2,21 @@
 // (antialias/cuda_rasterizer/forward.cu:406-567, backward.cu:399-557).
 //
 // One CTA per 16x16 tile.  The tile's sorted pairs are contiguous 48-byte
-// records (written by the last sort pass), so each 256-record batch is ONE
-// bulk copy (cp.async.bulk, the TMA engine's 1-D form) into shared memory,
-// completed on an mbarrier.  Three record buffers keep two batches in flight
-// while the current one is composited.  A thread owns PPT pixels of one
-// column (16 x 2*PPT pixels per warp); a warp whose pixels have all
-// saturated (T < 1e-4) stops evaluating and only joins the per-batch barrier.
+// records (written by the last sort pass), so each record batch is ONE bulk copy
+// (cp.async.bulk, the TMA engine's 1-D form) into shared memory, completed on an
+// mbarrier.  Three record buffers keep two batches in flight while the current
+// one is composited.  A warp owns a block of 8 columns x 4 PPT rows (PPT pixels of
+// one column per lane, 4 rows apart), and a record carries the mask of the tile's
+// four 8x8 quads it can reach (quad_mask, written by the sort): one ballot per 32
+// records tells a warp which of them to composite.
+//
+// Both directions are bound by instruction issue (86% and 73% of the issue slots of
+// 1080p views), so two pixels of a lane are composited per instruction with packed
+// fma / mul / add.f32x2, which round each half as the scalar operation does, and a
+// record's masks are formed once, not once per warp and direction.  Sixteen 1080p views
+// (27.9M pairs) at the best shape: forward 4.81 -> 3.68 ms, backward 7.81 -> 6.55 ms; one
+// such view: 361 -> 284 and 505 -> 372 us; 10,000 Gaussians at 256x256: 72 -> 44 and
+// 93 -> 58 us at 2 pixels per lane.
 //
 // Per-Gaussian outputs that the reference updates from every pixel (the
 // racy out_point_weight max, the KPC statistics, the backward's 9 gradient
@@ -89,41 +98,67 @@ __device__ __forceinline__ float warp_sum(float v)
     return v;
 }
 
-// Conservative test used to skip (warp, record) pairs: can a Gaussian with mean
-// (mx, my), conic (a, b, c) and opacity o reach alpha >= 1/255 at any pixel
-// centre of [x0,x1] x [y0,y1]?  alpha <= o (power <= 0), so o < 1/255 never
-// contributes; otherwise alpha >= 1/255 needs Q = a dx^2 + 2b dx dy + c dy^2
-// <= 2 ln(255 o), and Q's minimum over the rectangle is 0 when the mean is
-// inside, else on the boundary (one clamped 1-D minimum per edge).  The margin
-// covers float rounding of the per-pixel evaluation by a wide factor; a
-// non-positive-definite conic is never skipped.  Skipping only removes work
-// that the per-pixel tests would reject, so every output is unchanged.
-__device__ __forceinline__ bool may_touch(float mx, float my, float a, float b, float c, float o, float x0, float x1,
-                                          float y0, float y1)
+// ---------------------------------------------------------------- two floats per instruction
+// A pair of float32 in one 64-bit register; each half of an operation is rounded to
+// nearest as the scalar operation is.
+typedef unsigned long long F2;
+
+__device__ __forceinline__ F2 f2(float lo, float hi)
 {
-    if (!(o >= 1.0f / 255.0f)) return false;
-    if (!(a > 0.f && c > 0.f && a * c - b * b > 0.f)) return true;
-    const float X0 = x0 - mx, X1 = x1 - mx, Y0 = y0 - my, Y1 = y1 - my;
-    if (X0 <= 0.f && X1 >= 0.f && Y0 <= 0.f && Y1 >= 0.f) return true;
-    const float thr = 2.f * __logf(255.f * o);
-    float q = 3.4e38f;
-    // edges x = X0, X1
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const float X = i ? X1 : X0;
-        const float dy = fminf(fmaxf(-b * X / c, Y0), Y1);
-        q = fminf(q, a * X * X + 2.f * b * X * dy + c * dy * dy);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const float Y = i ? Y1 : Y0;
-        const float dx = fminf(fmaxf(-b * Y / a, X0), X1);
-        q = fminf(q, a * dx * dx + 2.f * b * dx * Y + c * Y * Y);
-    }
-    const float mX = fmaxf(fabsf(X0), fabsf(X1)), mY = fmaxf(fabsf(Y0), fabsf(Y1));
-    const float mag = a * mX * mX + c * mY * mY + 2.f * fabsf(b) * mX * mY;
-    return q <= thr + 0.05f + 1e-5f * mag;
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
 }
+__device__ __forceinline__ F2 f2(float v) { return f2(v, v); }
+__device__ __forceinline__ float f2_lo(F2 v)
+{
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return a;
+}
+__device__ __forceinline__ float f2_hi(F2 v)
+{
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return b;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// The block of pixels of this thread's warp: 8 columns x 4 PPT rows of the tile, lane
+// (x, y) = (lane & 7, lane >> 3), its pixel k at row y + 4 k.
+template <int PPT>
+struct WarpBlock {
+    int px, py0, col, quad_row;  // first pixel; the block's column of quads and its first row of quads
+    __device__ __forceinline__ WarpBlock(int bx, int by)
+    {
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        col = w & 1;
+        const int row = (w >> 1) * 4 * PPT;
+        quad_row = row >> 3;
+        px = bx * kTileX + 8 * col + (lane & 7);
+        py0 = by * kTileY + row + (lane >> 3);
+    }
+};
+// Quads of 8x8 pixels one warp's block covers (a block of PPT = 1 is half a quad).
+template <int PPT>
+constexpr int warp_quads() { return PPT == 4 ? 2 : 1; }
 
 // ---------------------------------------------------------------- per-view render descriptors
 // Everything one tile needs, for the plain launch (one view, one tile per CTA)
@@ -141,19 +176,23 @@ struct FwdSmem {
     uint32_t kcnt[2][kBatch];
 };
 
-// Per-record gradient sums of a batch: warps 2s and 2s+1 add their warp totals
-// into slot s.  A slot starts at zero and takes at most two additions, and
-// float addition is commutative, so its value does not depend on which warp
-// came first; the slots are then summed in slot order.  The result is the same
-// on every run (no order-dependent float atomics anywhere in the backward).
+// Per-record gradient sums of a batch, [record][component] so that the nine lanes
+// that store a record's totals hit nine banks.  With two warps per tile (PPT = 4)
+// each has a slot of its own, stores its totals (no read-modify-write; a record the
+// warp did not touch is told by `live`), and the slots are added in warp order.  With
+// more warps, warps 2s and 2s+1 add into slot s: a slot starts at zero and takes at
+// most two additions, and float addition is commutative, so its value does not depend
+// on which warp came first.  Either way the result is the same on every run (no
+// order-dependent float atomics anywhere in the backward).
 template <int PPT>
-constexpr int bwd_slots() { return (256 / PPT / 32) / 2 > 0 ? (256 / PPT / 32) / 2 : 1; }
+constexpr int bwd_slots() { return PPT == 4 ? 2 : (256 / PPT / 32) / 2; }
 
 template <int kBatch, int kSlots>
 struct BwdSmem {
     PairRecord rec[kBufs][kBatch];
     uint64_t bar[kBufs];
-    float acc[kSlots][9][kBatch];
+    float acc[kSlots][kBatch][9];
+    uint32_t live[2][kBatch / 32];
     uint32_t max_last;
 };
 
@@ -207,40 +246,100 @@ __device__ __forceinline__ float fwd_accumulate(float alpha, const float4 rb, co
     return w;
 }
 
-// fwd_alpha + fwd_accumulate in one pass with early exits (the tile path: no
-// record is evaluated ahead), the same arithmetic.  A contribution also goes into
-// the caller's per-record sums (max weight, weight sum, count).
-__device__ __forceinline__ void fwd_pixel_step(const float4 ra, const float4 rb, const PairRecord& rec, float pxf,
-                                               float pyf, uint32_t position, float& T, float (&C)[3], float& wmax,
-                                               int& maxid, uint32_t& last, bool& done, float& wj, float& ksum,
-                                               uint32_t& kc)
+// What a forward launch keeps beside the image: nothing (a batched view without these
+// outputs), point_id / point_weight_pixel / point_weight, or those and the statistics.
+enum { kImage = 0, kWeights = 1, kStats = 2 };
+
+// One pixel's state between records: T, colour and the strongest contributor as in
+// fwd_accumulate; amin is the smallest alpha that still counts: 1/255, or 2 (no alpha
+// reaches it) once the pixel is done or when it lies outside the image.
+constexpr float kAlphaMin = 1.0f / 255.0f, kDone = 2.0f;
+
+// One record on one pixel, with branches: the form for one pixel per lane, and for a
+// record whose colour or position is too large for the packed form (kWild), where a
+// pixel the record does not reach must not see 0 * inf.  Returns the weight T * alpha
+// the record took, 0 when it did not contribute.
+__device__ __forceinline__ float fwd_pixel_step(const float4 ra, const float4 rb, float c2, int id, float pxf,
+                                                float pyf, uint32_t position, float& T, float& C0, float& C1,
+                                                float& C2, float& wmax, int& maxid, uint32_t& last, float& amin)
 {
-    if (done) return;
-    const float dx = ra.x - pxf, dy = ra.y - pyf;
-    const float q = __fmaf_rn(__fmul_rn(ra.z, dx), dx, __fmul_rn(__fmul_rn(rb.x, dy), dy));
-    const float power = __fmaf_rn(-0.5f, q, -__fmul_rn(__fmul_rn(ra.w, dx), dy));
-    if (power > 0.0f) return;
-    const float alpha = fminf(0.99f, __fmul_rn(rb.y, expf(power)));
-    if (alpha < 1.0f / 255.0f) return;
+    const float alpha = fwd_alpha(ra, rb, pxf, pyf);
+    if (!(alpha >= amin)) return 0.f;
     const float test_T = __fmul_rn(T, 1.0f - alpha);
     if (test_T < 0.0001f) {
-        done = true;
-        return;
+        amin = kDone;
+        return 0.f;
     }
-    const float4 rc = rec.c;
-    C[0] = __fmaf_rn(__fmul_rn(rb.z, alpha), T, C[0]);
-    C[1] = __fmaf_rn(__fmul_rn(rb.w, alpha), T, C[1]);
-    C[2] = __fmaf_rn(__fmul_rn(rc.x, alpha), T, C[2]);
+    C0 = __fmaf_rn(__fmul_rn(rb.z, alpha), T, C0);
+    C1 = __fmaf_rn(__fmul_rn(rb.w, alpha), T, C1);
+    C2 = __fmaf_rn(__fmul_rn(c2, alpha), T, C2);
     const float w = __fmul_rn(T, alpha);
     if (w > wmax) {
         wmax = w;
-        maxid = __float_as_int(rc.y);
+        maxid = id;
     }
-    wj = fmaxf(wj, w);
-    ksum += w;
-    kc += 1;
     T = test_T;
     last = position;
+    return w;
+}
+
+// The pixels of one lane in pairs (k = 2q, 2q + 1).
+template <int NP>
+struct FwdPixels {
+    F2 T[NP], C[NP][3], wmax[NP], npy[NP];  // npy: -row
+    float amin[2 * NP];
+    int maxid[2 * NP];
+    uint32_t last[2 * NP];
+};
+
+// One record on one pair of pixels, without branches: a pixel the record does not
+// reach takes alpha 0, which leaves T, the colours and the weight as they are (T * 1,
+// C + 0 * T).  The same operations, in the same order and rounding, as fwd_alpha and
+// fwd_accumulate.  Returns the larger of the two weights (kImage: alphas): > 0 when
+// either pixel took something.
+template <int kOut, int NP>
+__device__ __forceinline__ float fwd_pair_step(FwdPixels<NP>& s, int q, const float4 ra, const float4 rb, float c2,
+                                               int id, float dx, float sx, float nbx, uint32_t position, F2& wsum,
+                                               uint32_t& wcount)
+{
+    const F2 dy = f2_add(f2(ra.y), s.npy[q]);
+    const F2 qf = f2_fma(f2(sx), f2(dx), f2_mul(f2_mul(f2(rb.x), dy), dy));
+    const F2 power = f2_fma(f2(-0.5f), qf, f2_mul(f2(nbx), dy));
+    const F2 oG = f2_mul(f2(rb.y), f2(expf(f2_lo(power)), expf(f2_hi(power))));
+    const float a0 = fminf(0.99f, f2_lo(oG)), a1 = fminf(0.99f, f2_hi(oG));
+    float& m0 = s.amin[2 * q];
+    float& m1 = s.amin[2 * q + 1];
+    const bool ok0 = !(f2_lo(power) > 0.f) && a0 >= m0, ok1 = !(f2_hi(power) > 0.f) && a1 >= m1;
+    F2 alpha = f2(ok0 ? a0 : 0.f, ok1 ? a1 : 0.f);
+    const F2 keep = f2_fma(alpha, f2(-1.f), f2(1.f));  // 1 - alpha
+    const F2 test_T = f2_mul(s.T[q], keep);
+    // (a pixel that takes nothing keeps T >= 1e-4 and cannot end here)
+    const bool end0 = ok0 && f2_lo(test_T) < 0.0001f, end1 = ok1 && f2_hi(test_T) < 0.0001f;
+    m0 = end0 ? kDone : m0;
+    m1 = end1 ? kDone : m1;
+    const float e0 = end0 ? 0.f : f2_lo(alpha), e1 = end1 ? 0.f : f2_hi(alpha);
+    alpha = f2(e0, e1);
+    s.C[q][0] = f2_fma(f2_mul(f2(rb.z), alpha), s.T[q], s.C[q][0]);
+    s.C[q][1] = f2_fma(f2_mul(f2(rb.w), alpha), s.T[q], s.C[q][1]);
+    s.C[q][2] = f2_fma(f2_mul(f2(c2), alpha), s.T[q], s.C[q][2]);
+    s.last[2 * q] = e0 > 0.f ? position : s.last[2 * q];
+    s.last[2 * q + 1] = e1 > 0.f ? position : s.last[2 * q + 1];
+    float took = fmaxf(e0, e1);
+    if constexpr (kOut != kImage) {
+        const F2 w = f2_mul(s.T[q], alpha);
+        const float w0 = f2_lo(w), w1 = f2_hi(w);
+        const bool g0 = w0 > f2_lo(s.wmax[q]), g1 = w1 > f2_hi(s.wmax[q]);
+        s.wmax[q] = f2(g0 ? w0 : f2_lo(s.wmax[q]), g1 ? w1 : f2_hi(s.wmax[q]));
+        s.maxid[2 * q] = g0 ? id : s.maxid[2 * q];
+        s.maxid[2 * q + 1] = g1 ? id : s.maxid[2 * q + 1];
+        took = fmaxf(w0, w1);
+        if constexpr (kOut == kStats) {
+            wsum = f2_add(wsum, w);
+            wcount += (e0 > 0.f) + (e1 > 0.f);
+        }
+    }
+    s.T[q] = f2(end0 ? f2_lo(s.T[q]) : f2_lo(test_T), end1 ? f2_hi(s.T[q]) : f2_hi(test_T));
+    return took;
 }
 
 // One tile.  Callers guarantee every thread of the CTA is synchronised on
@@ -248,22 +347,23 @@ __device__ __forceinline__ void fwd_pixel_step(const float4 ra, const float4 rb,
 // this CTA has ever waited for: batch g lives in buffer g % 3 and completes
 // phase (g / 3) & 1 of that buffer's mbarrier, so the barriers are initialised
 // once per CTA and keep their phase across tiles.
-template <int PPT, int kBatch>
+template <int PPT, int kBatch, int kOut>
 __device__ __forceinline__ void render_fwd_tile(FwdSmem<kBatch>& sm, const TileArgs& a, int tile, uint32_t& gb,
-                                                uint32_t split_min, bool stats_smem, unsigned* err)
+                                                uint32_t split_min, unsigned* err)
 {
     constexpr int NT = 256 / PPT;
+    constexpr int NP = PPT > 1 ? PPT / 2 : 1;
+    constexpr int kQuads = warp_quads<PPT>();
     const int tid = threadIdx.x;
     const int W = a.W, H = a.H;
     const int gx = (W + kTileX - 1) / kTileX;
     const int bx = tile % gx, by = tile / gx;
-    const int lx = tid & 15, ly0 = (tid >> 4) * PPT;
-    const int px = bx * kTileX + lx;
+    const WarpBlock<PPT> blk(bx, by);
+    const int px = blk.px;
     const uint2 range = a.ranges[tile];
     const uint32_t n = range.y - range.x;
     if (split_min && n >= split_min) return;  // rendered in bands (render_long_tile)
     const int nb = (int)((n + kBatch - 1) / kBatch);
-    const bool stats = stats_smem && a.kv_sum != nullptr;  // the sums exist only in a launch that has them
     const PairRecord* recs = a.recs;
 
     if (tid == 0) {
@@ -273,112 +373,139 @@ __device__ __forceinline__ void render_fwd_tile(FwdSmem<kBatch>& sm, const TileA
         }
     }
 
-    float T[PPT], C[PPT][3], wmax[PPT];
-    uint32_t last[PPT];
-    int maxid[PPT];
-    bool done[PPT];
-    float pyf[PPT];
+    FwdPixels<NP> s;
 #pragma unroll
-    for (int k = 0; k < PPT; k++) {
-        T[k] = 1.0f;
-        C[k][0] = C[k][1] = C[k][2] = 0.f;
-        wmax[k] = 0.f;
-        last[k] = 0;
-        maxid[k] = -1;
-        const int py = by * kTileY + ly0 + k;
-        done[k] = !(px < W && py < H);
-        pyf[k] = (float)py;
+    for (int q = 0; q < NP; q++) {
+        s.T[q] = f2(1.f);
+        s.C[q][0] = s.C[q][1] = s.C[q][2] = f2(0.f);
+        s.wmax[q] = f2(0.f);
+        s.npy[q] = f2(-(float)(blk.py0 + 8 * q), -(float)(blk.py0 + 8 * q + 4));
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const bool inside = px < W && blk.py0 + 8 * q + 4 * h < H && 2 * q + h < PPT;
+            s.amin[2 * q + h] = inside ? kAlphaMin : kDone;
+            s.last[2 * q + h] = 0;
+            s.maxid[2 * q + h] = -1;
+        }
     }
     const float pxf = (float)px;
-    // this warp's pixel rectangle: 16 columns x 2*PPT rows
-    const float rx0 = (float)(bx * kTileX), rx1 = rx0 + (kTileX - 1);
-    const float ry0 = (float)(by * kTileY + (tid >> 5) * 2 * PPT), ry1 = ry0 + (2 * PPT - 1);
-    bool all_done = true;
+    auto all_done = [&] {
+        bool d = true;
 #pragma unroll
-    for (int k = 0; k < PPT; k++) all_done = all_done && done[k];
+        for (int k = 0; k < PPT; k++) d = d && s.amin[k] > 1.f;
+        return d;
+    };
+    const int qbit0 = 2 * blk.quad_row + blk.col;
 
     int issued = nb < 2 ? nb : 2;
     uint32_t contributor = 0;
+    bool stop = __all_sync(0xffffffffu, all_done());  // warp-uniform: no pixel of the warp takes any more
     for (int b = 0; b < nb; b++) {
         const uint32_t g = gb + b;
         const int buf = (int)(g % kBufs);
         const int acc = b & 1;
         const uint32_t cnt = min((uint32_t)kBatch, n - b * kBatch);
-        if (!mbar_wait(&sm.bar[buf], (g / kBufs) & 1, err)) all_done = true;
+        // (a copy that never lands: every thread gives up on the tile, the error is recorded)
+        if (__any_sync(0xffffffffu, !mbar_wait(&sm.bar[buf], (g / kBufs) & 1, err))) stop = true;
         const PairRecord* R = sm.rec[buf];
-        const bool warp_live = !__all_sync(0xffffffffu, all_done);
-        if (warp_live) {
-            bool stop = false;
-            for (uint32_t k0 = 0; k0 < cnt && !stop; k0 += 32) {
-                // which of these 32 records can reach alpha >= 1/255 inside this warp's pixels
-                const uint32_t e = k0 + (tid & 31);
-                bool t = false;
-                if (e < cnt) {
-                    const float4 ea = R[e].a, eb = R[e].b;
-                    t = may_touch(ea.x, ea.y, ea.z, ea.w, eb.x, eb.y, rx0, rx1, ry0, ry1);
-                }
-                uint32_t live = __ballot_sync(0xffffffffu, t);
-                while (live) {
-                    const uint32_t j = k0 + (uint32_t)(__ffs(live) - 1);
-                    live &= live - 1;
-                    const uint32_t position = contributor + j + 1;
-                    const float4 ra = R[j].a;
-                    const float4 rb = R[j].b;
-                    float wj = 0.f, ksum = 0.f;
-                    uint32_t kc = 0;
+        for (uint32_t k0 = 0; k0 < cnt && !stop; k0 += 32) {
+            // which of these 32 records reach this warp's quads
+            const uint32_t e = k0 + (tid & 31);
+            const uint32_t mask = e < cnt ? __float_as_uint(R[e].c.z) >> qbit0 : 0u;
+            uint32_t quad[kQuads], live = 0;
 #pragma unroll
-                    for (int k = 0; k < PPT; k++)
-                        fwd_pixel_step(ra, rb, R[j], pxf, pyf[k], position, T[k], C[k], wmax[k], maxid[k], last[k],
-                                       done[k], wj, ksum, kc);
-                    bool ad = true;
+            for (int q = 0; q < kQuads; q++) {
+                quad[q] = __ballot_sync(0xffffffffu, (mask >> (2 * q)) & 1u);
+                live |= quad[q];
+            }
+            while (live) {
+                const uint32_t bit = (uint32_t)(__ffs(live) - 1);
+                const uint32_t j = k0 + bit;
+                live &= live - 1;
+                const uint32_t position = contributor + j + 1;
+                const float4 ra = R[j].a;
+                const float4 rb = R[j].b;
+                const float4 rc = R[j].c;
+                float wj = 0.f;
+                F2 wsum = f2(0.f);
+                uint32_t kc = 0;
+                if (PPT == 1 || (__float_as_uint(rc.z) & kWild)) {
 #pragma unroll
-                    for (int k = 0; k < PPT; k++) ad = ad && done[k];
-                    all_done = ad;
-                    // per-Gaussian max weight (and statistics): warp, then CTA
-                    if (__any_sync(0xffffffffu, wj > 0.f)) {
-                        const uint32_t wm = __reduce_max_sync(0xffffffffu, __float_as_uint(wj));
-                        float ks = 0.f;
-                        uint32_t kcs = 0;
-                        if (stats) {
-                            ks = warp_sum(ksum);
-                            kcs = __reduce_add_sync(0xffffffffu, kc);
-                        }
-                        if ((tid & 31) == 0) {
-                            atomicMax(&sm.wmax[acc][j], wm);
-                            if (stats) {
-                                atomicAdd(&sm.ksum[acc][j], ks);
-                                atomicAdd(&sm.kcnt[acc][j], kcs);
-                            }
-                        }
+                    for (int k = 0; k < PPT; k++) {
+                        const int q = k >> 1;
+                        float T = (k & 1) ? f2_hi(s.T[q]) : f2_lo(s.T[q]);
+                        float C[3], wm = (k & 1) ? f2_hi(s.wmax[q]) : f2_lo(s.wmax[q]);
+#pragma unroll
+                        for (int c = 0; c < 3; c++) C[c] = (k & 1) ? f2_hi(s.C[q][c]) : f2_lo(s.C[q][c]);
+                        const float pyf = -((k & 1) ? f2_hi(s.npy[q]) : f2_lo(s.npy[q]));
+                        const float w = fwd_pixel_step(ra, rb, rc.x, __float_as_int(rc.y), pxf, pyf, position, T, C[0],
+                                                       C[1], C[2], wm, s.maxid[k], s.last[k], s.amin[k]);
+                        wj = fmaxf(wj, w);
+                        wsum = f2_add(wsum, f2(w, 0.f));
+                        kc += w > 0.f;
+                        s.T[q] = (k & 1) ? f2(f2_lo(s.T[q]), T) : f2(T, f2_hi(s.T[q]));
+                        s.wmax[q] = (k & 1) ? f2(f2_lo(s.wmax[q]), wm) : f2(wm, f2_hi(s.wmax[q]));
+#pragma unroll
+                        for (int c = 0; c < 3; c++)
+                            s.C[q][c] = (k & 1) ? f2(f2_lo(s.C[q][c]), C[c]) : f2(C[c], f2_hi(s.C[q][c]));
                     }
-                    if (__all_sync(0xffffffffu, all_done)) {
-                        stop = true;
-                        break;
+                } else {
+                    const float dx = ra.x - pxf;
+                    const float sx = __fmul_rn(ra.z, dx), nbx = -__fmul_rn(ra.w, dx);
+#pragma unroll
+                    for (int q = 0; q < NP; q++)
+                        if (kQuads == 1 || ((quad[q] >> bit) & 1u))
+                            wj = fmaxf(wj, fwd_pair_step<kOut, NP>(s, q, ra, rb, rc.x, __float_as_int(rc.y), dx, sx,
+                                                                    nbx, position, wsum, kc));
+                }
+                if (!__any_sync(0xffffffffu, wj > 0.f)) {
+                    // a record that nobody took: perhaps because every pixel is done
+                    stop = __all_sync(0xffffffffu, all_done());
+                    if (stop) break;
+                    continue;
+                }
+                if constexpr (kOut != kImage) {
+                    // per-Gaussian max weight (and statistics): warp, then CTA
+                    const uint32_t wm = __reduce_max_sync(0xffffffffu, __float_as_uint(wj));
+                    float ks = 0.f;
+                    uint32_t kcs = 0;
+                    if constexpr (kOut == kStats) {
+                        ks = warp_sum(f2_lo(wsum) + f2_hi(wsum));
+                        kcs = __reduce_add_sync(0xffffffffu, kc);
+                    }
+                    if ((tid & 31) == 0) {
+                        atomicMax(&sm.wmax[acc][j], wm);
+                        if constexpr (kOut == kStats) {
+                            atomicAdd(&sm.ksum[acc][j], ks);
+                            atomicAdd(&sm.kcnt[acc][j], kcs);
+                        }
                     }
                 }
             }
+            if (!stop) stop = __all_sync(0xffffffffu, all_done());
         }
         contributor += cnt;
-        const int ndone = __syncthreads_count(all_done);
-        for (uint32_t e = tid; e < cnt; e += NT) {
-            const uint32_t wm = sm.wmax[acc][e];
-            if (wm) {
-                const int id = __float_as_int(R[e].c.y);
-                if (a.out_point_weight) atomicMax(reinterpret_cast<unsigned*>(a.out_point_weight) + id, wm);
-                sm.wmax[acc][e] = 0;
+        const int ndone = __syncthreads_count(stop);
+        if constexpr (kOut != kImage)
+            for (uint32_t e = tid; e < cnt; e += NT) {
+                const uint32_t wm = sm.wmax[acc][e];
+                if (wm) {
+                    const int id = __float_as_int(R[e].c.y);
+                    if (a.out_point_weight) atomicMax(reinterpret_cast<unsigned*>(a.out_point_weight) + id, wm);
+                    sm.wmax[acc][e] = 0;
+                }
+                if constexpr (kOut == kStats) {
+                    a.kv_sum[range.x + b * kBatch + e] = sm.ksum[acc][e];
+                    a.kv_cnt[range.x + b * kBatch + e] = sm.kcnt[acc][e];
+                    sm.ksum[acc][e] = 0.f;
+                    sm.kcnt[acc][e] = 0;
+                }
             }
-            if (stats) {
-                a.kv_sum[range.x + b * kBatch + e] = sm.ksum[acc][e];
-                a.kv_cnt[range.x + b * kBatch + e] = sm.kcnt[acc][e];
-                sm.ksum[acc][e] = 0.f;
-                sm.kcnt[acc][e] = 0;
-            }
-        }
         if (ndone == NT) {
             // drain the copy still in flight before the buffers are reused or the CTA exits
             if (tid == 0 && b + 1 < nb)
                 mbar_wait(&sm.bar[(g + 1) % kBufs], ((g + 1) / kBufs) & 1, err);
-            if (stats) {
+            if constexpr (kOut == kStats) {
                 // pairs never reached contribute nothing
                 for (uint32_t e = (b + 1) * kBatch + tid; e < n; e += NT) {
                     a.kv_sum[range.x + e] = 0.f;
@@ -400,16 +527,20 @@ __device__ __forceinline__ void render_fwd_tile(FwdSmem<kBatch>& sm, const TileA
 
 #pragma unroll
     for (int k = 0; k < PPT; k++) {
-        const int py = by * kTileY + ly0 + k;
+        const int py = blk.py0 + 4 * k, q = k >> 1;
+        auto half = [&](F2 v) { return (k & 1) ? f2_hi(v) : f2_lo(v); };
         if (px < W && py < H) {
             const int pix = W * py + px;
-            a.final_T[pix] = T[k];
-            a.n_contrib[pix] = last[k];
-            a.out_color[pix] = __fmaf_rn(T[k], a.bg[0], C[k][0]);
-            a.out_color[H * W + pix] = __fmaf_rn(T[k], a.bg[1], C[k][1]);
-            a.out_color[2 * H * W + pix] = __fmaf_rn(T[k], a.bg[2], C[k][2]);
-            if (a.out_point_id) a.out_point_id[pix] = maxid[k];
-            if (a.out_pw_pixel) a.out_pw_pixel[pix] = wmax[k];
+            const float T = half(s.T[q]);
+            a.final_T[pix] = T;
+            a.n_contrib[pix] = s.last[k];
+            a.out_color[pix] = __fmaf_rn(T, a.bg[0], half(s.C[q][0]));
+            a.out_color[H * W + pix] = __fmaf_rn(T, a.bg[1], half(s.C[q][1]));
+            a.out_color[2 * H * W + pix] = __fmaf_rn(T, a.bg[2], half(s.C[q][2]));
+            if constexpr (kOut != kImage) {
+                if (a.out_point_id) a.out_point_id[pix] = s.maxid[k];
+                if (a.out_pw_pixel) a.out_pw_pixel[pix] = half(s.wmax[q]);
+            }
         }
     }
 }
@@ -439,16 +570,15 @@ __device__ __forceinline__ void fwd_smem_init(FwdSmem<kBatch>& sm, int NT, bool 
 template <int PPT>
 constexpr int fwd_min_ctas() { return PPT == 1 ? 3 : (PPT == 2 ? 8 : 16); }
 
-template <int PPT, int kBatch>
+template <int PPT, int kBatch, int kOut>
 __global__ void __launch_bounds__(256 / PPT, fwd_min_ctas<PPT>())
     render_fwd_kernel(TileArgs a, uint32_t split_min, unsigned* err)
 {
     extern __shared__ __align__(128) unsigned char fwd_dyn[];
     FwdSmem<kBatch>& sm = *reinterpret_cast<FwdSmem<kBatch>*>(fwd_dyn);
-    const bool stats_smem = a.kv_sum != nullptr;  // the launch sized the shared memory from the same test
-    fwd_smem_init(sm, 256 / PPT, stats_smem);
+    fwd_smem_init(sm, 256 / PPT, kOut == kStats);
     uint32_t gb = 0;
-    render_fwd_tile<PPT, kBatch>(sm, a, blockIdx.x, gb, split_min, stats_smem, err);
+    render_fwd_tile<PPT, kBatch, kOut>(sm, a, blockIdx.x, gb, split_min, err);
 }
 
 // Persistent multi-view forward: CTAs pop work items from one queue; item i is
@@ -478,7 +608,11 @@ __global__ void __launch_bounds__(256 / PPT, fwd_min_ctas<PPT>())
         if (item >= total) break;
         const int v = view_of(begin, nviews, item);
         const TileArgs& a = views[v];  // fields read where used, not held in registers
-        render_fwd_tile<PPT, kBatch>(sm, a, (int)(item - begin[v]), gb, split_min, false, err);
+        // (from the device descriptors: a captured graph follows fgs_batch_set_view_outputs)
+        if (a.out_point_weight || a.out_point_id || a.out_pw_pixel)
+            render_fwd_tile<PPT, kBatch, kWeights>(sm, a, (int)(item - begin[v]), gb, split_min, err);
+        else
+            render_fwd_tile<PPT, kBatch, kImage>(sm, a, (int)(item - begin[v]), gb, split_min, err);
         __syncthreads();
     }
 }
@@ -817,6 +951,139 @@ __global__ void __launch_bounds__(LongTile<BW, BH>::kThreads)
 }
 
 // ---------------------------------------------------------------- backward
+// The pixels of one lane in the backward, in pairs (k = 2q, 2q + 1).  The reference's
+// accum_rec recurrence (the colour composited behind the current Gaussian,
+// backward.cu:513-520) enters dL/dalpha only through its dot product with dL/dpixel,
+// so a pixel carries that dot product (acc): one value instead of six.  bgT: the
+// numerator -T_final (bg . dL/dpixel) of the background term of dL/dalpha.
+template <int NP>
+struct BwdPixels {
+    F2 T[NP], acc[NP], d[NP][3], bgT[NP], npy[NP];
+    uint32_t last[2 * NP];
+};
+
+// A record's sums over a lane's pixels: alpha T dL/dpixel (c) and w, w dy, w dy dy (s)
+// with w = G dL/dalpha.  All of a lane's pixels share a column, so the products with dx
+// are formed from these once per column (warp_column_sum9) instead of once per pixel.
+struct BwdSums {
+    F2 c[3], s[3];
+};
+
+// One record on one pixel, with branches (see fwd_pixel_step for when).  The values of
+// the pixel are passed one by one; sums go into the low halves.
+template <bool kConsistent>
+__device__ __forceinline__ bool bwd_pixel_step(const float4 ra, const float4 rb, float c2, float pxf, float pyf,
+                                               bool before_last, float& T, float& acc, float d0, float d1, float d2,
+                                               float bgT, BwdSums& g)
+{
+    if (!before_last) return false;
+    const float dx = ra.x - pxf, dy = ra.y - pyf;
+    const float qf = __fmaf_rn(__fmul_rn(ra.z, dx), dx, __fmul_rn(__fmul_rn(rb.x, dy), dy));
+    const float power = __fmaf_rn(-0.5f, qf, -__fmul_rn(__fmul_rn(ra.w, dx), dy));
+    if (power > 0.0f) return false;
+    const float G = expf(power);
+    const float oG = __fmul_rn(rb.y, G);
+    const float alpha = fminf(0.99f, oG);
+    if (alpha < 1.0f / 255.0f) return false;
+    const float inv = __fdividef(1.f, 1.f - alpha);
+    T = T * inv;
+    const float wc = alpha * T;
+    g.c[0] = f2_add(g.c[0], f2(wc * d0, 0.f));
+    g.c[1] = f2_add(g.c[1], f2(wc * d1, 0.f));
+    g.c[2] = f2_add(g.c[2], f2(wc * d2, 0.f));
+    const float cdot = rb.z * d0 + rb.w * d1 + c2 * d2;
+    const float diff = cdot - acc;
+    float dL_dalpha = diff * T;
+    if (bgT != 0.f) dL_dalpha += bgT * inv;
+    if (kConsistent && oG > 0.99f) dL_dalpha = 0.f;
+    acc += alpha * diff;
+    const float w = G * dL_dalpha, v = w * dy;
+    g.s[0] = f2_add(g.s[0], f2(w, 0.f));
+    g.s[1] = f2_add(g.s[1], f2(v, 0.f));
+    g.s[2] = f2_add(g.s[2], f2(v * dy, 0.f));
+    return true;
+}
+
+// One record on one pair of pixels, without branches: a pixel the record does not
+// reach (or that ended before it) takes alpha 0, which leaves its T and acc as they are,
+// and w 0.  G and alpha are formed with the forward's operations and rounding, so this
+// pass skips exactly the (pixel, record) pairs the forward skipped.  All values are
+// below 1e15 here (kWild records and warps take bwd_pixel_step), so no 0 * inf arises.
+template <bool kConsistent, int NP>
+__device__ __forceinline__ bool bwd_pair_step(BwdPixels<NP>& s, int q, const float4 ra, const float4 rb, float c2,
+                                              float dx, float sx, float nbx, uint32_t contributor, BwdSums& g)
+{
+    const F2 dy = f2_add(f2(ra.y), s.npy[q]);
+    const F2 qf = f2_fma(f2(sx), f2(dx), f2_mul(f2_mul(f2(rb.x), dy), dy));
+    const F2 power = f2_fma(f2(-0.5f), qf, f2_mul(f2(nbx), dy));
+    const F2 G = f2(expf(f2_lo(power)), expf(f2_hi(power)));
+    const F2 oG = f2_mul(f2(rb.y), G);
+    const float a0 = fminf(0.99f, f2_lo(oG)), a1 = fminf(0.99f, f2_hi(oG));
+    const bool ok0 = contributor < s.last[2 * q] && !(f2_lo(power) > 0.f) && !(a0 < 1.0f / 255.0f);
+    const bool ok1 = contributor < s.last[2 * q + 1] && !(f2_hi(power) > 0.f) && !(a1 < 1.0f / 255.0f);
+    const F2 alpha = f2(ok0 ? a0 : 0.f, ok1 ? a1 : 0.f);
+    const F2 rem = f2_fma(alpha, f2(-1.f), f2(1.f));
+    // (fast reciprocal: 1 - alpha >= 0.01)
+    const F2 inv = f2(__fdividef(1.f, f2_lo(rem)), __fdividef(1.f, f2_hi(rem)));
+    s.T[q] = f2_mul(s.T[q], inv);  // transmittance before this Gaussian
+    const F2 wc = f2_mul(alpha, s.T[q]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) g.c[c] = f2_fma(wc, s.d[q][c], g.c[c]);
+    const F2 cdot = f2_fma(f2(c2), s.d[q][2], f2_fma(f2(rb.w), s.d[q][1], f2_mul(f2(rb.z), s.d[q][0])));
+    const F2 diff = f2_fma(s.acc[q], f2(-1.f), cdot);
+    s.acc[q] = f2_fma(alpha, diff, s.acc[q]);
+    const F2 dL_dalpha = f2_fma(s.bgT[q], inv, f2_mul(diff, s.T[q]));
+    F2 w = f2_mul(G, dL_dalpha);
+    const bool w0 = ok0 && !(kConsistent && f2_lo(oG) > 0.99f), w1 = ok1 && !(kConsistent && f2_hi(oG) > 0.99f);
+    w = f2(w0 ? f2_lo(w) : 0.f, w1 ? f2_hi(w) : 0.f);
+    const F2 v = f2_mul(w, dy);
+    g.s[0] = f2_add(g.s[0], w);
+    g.s[1] = f2_add(g.s[1], v);
+    g.s[2] = f2_fma(v, dy, g.s[2]);
+    return ok0 || ok1;
+}
+
+// The nine sums of a record over a warp's block (8 columns x 4 rows of lanes) from each
+// lane's BwdSums.  The lanes of a column (lane distances 16 and 8) are added first: at
+// distance 16 the upper lanes keep s and the lower ones c; after distance 8 every lane
+// has its column's three totals, and the lanes with bit 3 of the upper half turn theirs
+// into the dx products (w dx, w dx dx, w dy dx).  Then the eight columns: 3 -> 2 -> 1
+// values over distances 4 and 2, and a plain step over distance 1.  10 shuffles.
+// Lane l ends with the total of component column_sum9_component(l) of
+// c0 c1 c2 | w dx, w dy | w dx dx, w dx dy, w dy dy | w.
+__device__ __forceinline__ float warp_column_sum9(const BwdSums& g, float dx)
+{
+    const unsigned lane = threadIdx.x & 31;
+    const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4, b2 = lane & 2;
+    float v[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const float c = f2_lo(g.c[i]) + f2_hi(g.c[i]), s = f2_lo(g.s[i]) + f2_hi(g.s[i]);
+        v[i] = (b16 ? s : c) + __shfl_xor_sync(0xffffffffu, b16 ? c : s, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 8);
+    const bool expand = b16 && b8;
+    const float x0 = v[0] * dx, x1 = x0 * dx, x2 = v[1] * dx;
+    v[0] = expand ? x0 : v[0];
+    v[1] = expand ? x1 : v[1];
+    v[2] = expand ? x2 : v[2];
+    const float r0 = (b4 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, b4 ? v[0] : v[2], 4);
+    const float r1 = v[1] + __shfl_xor_sync(0xffffffffu, v[1], 4);
+    const float t = (b2 ? r1 : r0) + __shfl_xor_sync(0xffffffffu, b2 ? r0 : r1, 2);
+    return t + __shfl_xor_sync(0xffffffffu, t, 1);
+}
+
+// Which component warp_column_sum9 leaves on `lane`; 15 for the lanes whose copy is not
+// stored (odd lanes, the second copies).
+__device__ __forceinline__ int column_sum9_component(unsigned lane)
+{
+    const int part = (lane >> 3) & 3, pick = (lane & 2) ? 1 : ((lane & 4) ? 2 : 0);
+    if ((lane & 1) || part == 1 || ((lane & 2) && (lane & 4))) return 15;
+    // parts (three nibbles each): 0 colours, 2 (w, w dy, w dy dy), 3 (w dx, w dx dx, w dx dy)
+    return (int)((0x653748fff210ull >> (4 * (3 * part + pick))) & 15u);
+}
+
 // kConsistent: the exact-gradient backward mode (FGS_BACKWARD_CONSISTENT), a
 // compile-time switch so that the reference mode pays nothing for it per pixel.
 template <int PPT, int kBatch, bool kConsistent>
@@ -824,54 +1091,57 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()
                                                 uint32_t& gb, unsigned* err)
 {
     constexpr int kSlots = bwd_slots<PPT>();
+    constexpr bool kOwnSlot = PPT == 4;
     constexpr int NT = 256 / PPT;
+    constexpr int NP = PPT > 1 ? PPT / 2 : 1;
+    constexpr int kQuads = warp_quads<PPT>();
     constexpr int NG = 9;  // dcolor r,g,b ; dmean2D x,y ; dconic x,y,w ; dopacity
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5;
     const int W = a.W, H = a.H;
     const int gx = (W + kTileX - 1) / kTileX;
     const int bx = tile % gx, by = tile / gx;
-    const int lx = tid & 15, ly0 = (tid >> 4) * PPT;
-    const int px = bx * kTileX + lx;
+    const WarpBlock<PPT> blk(bx, by);
+    const int px = blk.px;
     const uint2 range = a.ranges[tile];
     const PairRecord* recs = a.recs;
 
-    // Per pixel: the reference's accum_rec recurrence (the colour composited behind
-    // the current Gaussian, backward.cu:513-520) enters dL/dalpha only through its
-    // dot product with dL/dpixel, so the pixel carries that dot product (acc_dot)
-    // and the previous contributor's colour dotted the same way (last_dot): the
-    // same sums, regrouped, in 2 values instead of 6.
-    float T[PPT], dpix[PPT][3], acc_dot[PPT], last_dot[PPT], last_alpha[PPT];
-    uint32_t last[PPT];
-    // the background term of dL/dalpha, -T_final (bg . dL/dpixel) / (1 - alpha): its
-    // numerator per pixel (zero for a black background, and then skipped)
-    float bgT[PPT];
+    BwdPixels<NP> s;
     const float bg0 = a.bg[0], bg1 = a.bg[1], bg2 = a.bg[2];
     uint32_t my_max = 0;
+    bool tame = true;
 #pragma unroll
-    for (int k = 0; k < PPT; k++) {
-        const int py = by * kTileY + ly0 + k;
-        const bool inside = px < W && py < H;
-        const int pix = W * py + px;
-        T[k] = inside ? a.final_T[pix] : 0.f;
-        last[k] = inside ? a.n_contrib[pix] : 0;
-        my_max = max(my_max, last[k]);
+    for (int q = 0; q < NP; q++) {
+        float T[2], d[2][3], bgT[2];
 #pragma unroll
-        for (int c = 0; c < 3; c++) dpix[k][c] = inside ? a.dL_dpix[c * H * W + pix] : 0.f;
-        acc_dot[k] = 0.f;
-        last_dot[k] = 0.f;
-        last_alpha[k] = 0.f;
-        bgT[k] = -T[k] * (bg0 * dpix[k][0] + bg1 * dpix[k][1] + bg2 * dpix[k][2]);
+        for (int h = 0; h < 2; h++) {
+            const int py = blk.py0 + 8 * q + 4 * h;
+            const bool inside = px < W && py < H && 2 * q + h < PPT;
+            const int pix = W * py + px;
+            T[h] = inside ? a.final_T[pix] : 0.f;
+            s.last[2 * q + h] = inside ? a.n_contrib[pix] : 0;
+            my_max = max(my_max, s.last[2 * q + h]);
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                d[h][c] = inside ? a.dL_dpix[c * H * W + pix] : 0.f;
+                tame = tame && fabsf(d[h][c]) < 1e15f;
+            }
+            bgT[h] = -T[h] * (bg0 * d[h][0] + bg1 * d[h][1] + bg2 * d[h][2]);
+            tame = tame && fabsf(bgT[h]) < 1e30f;
+        }
+        s.T[q] = f2(T[0], T[1]);
+        s.bgT[q] = f2(bgT[0], bgT[1]);
+        s.acc[q] = f2(0.f);
+        s.npy[q] = f2(-(float)(blk.py0 + 8 * q), -(float)(blk.py0 + 8 * q + 4));
+#pragma unroll
+        for (int c = 0; c < 3; c++) s.d[q][c] = f2(d[0][c], d[1][c]);
     }
+    // a gradient too large for the packed form (or not finite) sends the warp the other way
+    const uint32_t wild_warp = __all_sync(0xffffffffu, tame) ? 0u : kWild;
     const float pxf = (float)px;
-    const float rx0 = (float)(bx * kTileX), rx1 = rx0 + (kTileX - 1);
-    const float ry0 = (float)(by * kTileY + (tid >> 5) * 2 * PPT), ry1 = ry0 + (2 * PPT - 1);
+    const int qbit0 = 2 * blk.quad_row + blk.col;
     const float ddelx_dx = 0.5 * W;
     const float ddely_dy = 0.5 * H;
-    // The per-pixel loop sums w = G dL/dalpha and its products with dx, dy; the
-    // factors common to all of a pair's pixels (opacity, conic, -W/2, -H/2, -1/2 of
-    // backward.cu:537-551) are applied once per pair when the batch is flushed.
-    // Each warp total sits on the lanes of its component.
-    const int q_lane = (tid & 1) ? 15 : sum9_component((unsigned)tid);
+    const int q_lane = column_sum9_component((unsigned)tid & 31u);
 
     if (tid == 0) sm.max_last = 0;
     __syncthreads();
@@ -898,15 +1168,16 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()
         mbar_wait(&sm.bar[buf], (g / kBufs) & 1, err);
         const PairRecord* R = sm.rec[buf];
         for (int k0 = (int)((cnt - 1) & ~31u); k0 >= 0; k0 -= 32) {
-            // records of this chunk that sit before some pixel's last contributor and can
-            // reach alpha >= 1/255 inside this warp's pixels, walked back to front
+            // records of this chunk that sit before some pixel's last contributor and reach
+            // this warp's quads, walked back to front
             const uint32_t e = (uint32_t)k0 + (tid & 31);
-            bool t = false;
-            if (e < cnt && lo + e < warp_last) {
-                const float4 ea = R[e].a, eb = R[e].b;
-                t = may_touch(ea.x, ea.y, ea.z, ea.w, eb.x, eb.y, rx0, rx1, ry0, ry1);
+            const uint32_t mask = e < cnt && lo + e < warp_last ? __float_as_uint(R[e].c.z) >> qbit0 : 0u;
+            uint32_t quad[kQuads], live = 0, touched = 0;
+#pragma unroll
+            for (int q = 0; q < kQuads; q++) {
+                quad[q] = __ballot_sync(0xffffffffu, (mask >> (2 * q)) & 1u);
+                live |= quad[q];
             }
-            uint32_t live = __ballot_sync(0xffffffffu, t);
             while (live) {
                 const int bit = 31 - __clz(live);
                 live &= ~(1u << bit);
@@ -914,72 +1185,60 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()
                 const uint32_t contributor = lo + (uint32_t)j;  // 0-based position in the tile list
                 const float4 ra = R[j].a;
                 const float4 rb = R[j].b;
-                float gr[NG];
+                const float2 rc = make_float2(R[j].c.x, R[j].c.z);
+                BwdSums sums;
 #pragma unroll
-                for (int q = 0; q < NG; q++) gr[q] = 0.f;
+                for (int i = 0; i < 3; i++) sums.c[i] = sums.s[i] = f2(0.f);
+                const float dx = ra.x - pxf;
                 bool any = false;
+                if (PPT == 1 || ((__float_as_uint(rc.y) | wild_warp) & kWild)) {
 #pragma unroll
-                for (int k = 0; k < PPT; k++) {
-                    if (contributor >= last[k]) continue;
-                    // G and alpha in the forward's arithmetic (fwd_alpha): the same
-                    // bits, so this pass skips exactly the pairs the forward skipped
-                    const float dx = ra.x - pxf, dy = ra.y - (float)(by * kTileY + ly0 + k);
-                    const float qf = __fmaf_rn(__fmul_rn(ra.z, dx), dx, __fmul_rn(__fmul_rn(rb.x, dy), dy));
-                    const float power = __fmaf_rn(-0.5f, qf, -__fmul_rn(__fmul_rn(ra.w, dx), dy));
-                    if (power > 0.0f) continue;
-                    const float G = expf(power);
-                    const float oG = __fmul_rn(rb.y, G);
-                    const float alpha = fminf(0.99f, oG);
-                    if (alpha < 1.0f / 255.0f) continue;
-                    // transmittance before this Gaussian (fast reciprocal: 1 - alpha >= 0.01)
-                    const float inv_1ma = __fdividef(1.f, 1.f - alpha);
-                    T[k] = T[k] * inv_1ma;
-                    const float dchannel_dcolor = alpha * T[k];
-                    const float c2 = R[j].c.x;
-                    gr[0] += dchannel_dcolor * dpix[k][0];
-                    gr[1] += dchannel_dcolor * dpix[k][1];
-                    gr[2] += dchannel_dcolor * dpix[k][2];
-                    const float cdot = rb.z * dpix[k][0] + rb.w * dpix[k][1] + c2 * dpix[k][2];
-                    acc_dot[k] += last_alpha[k] * (last_dot[k] - acc_dot[k]);
-                    last_dot[k] = cdot;
-                    last_alpha[k] = alpha;
-                    float dL_dalpha = (cdot - acc_dot[k]) * T[k];
-                    // background term; exactly zero (and skipped) for a black background
-                    if (bgT[k] != 0.f) dL_dalpha += bgT[k] * inv_1ma;
-                    if (kConsistent && oG > 0.99f) dL_dalpha = 0.f;
-                    // w = G dL/dalpha = dL/dopacity; w dx and w dy give dL/dmean2D,
-                    // w dx dx, w dx dy and w dy dy dL/dconic (times the pair's factors)
-                    const float w = G * dL_dalpha;
-                    const float u = w * dx, v = w * dy;
-                    gr[3] += u;
-                    gr[4] += v;
-                    gr[5] += u * dx;
-                    gr[6] += u * dy;
-                    gr[7] += v * dy;
-                    gr[8] += w;
-                    any = true;
+                    for (int k = 0; k < PPT; k++) {
+                        const int q = k >> 1;
+                        auto half = [&](F2 v) { return (k & 1) ? f2_hi(v) : f2_lo(v); };
+                        float T = half(s.T[q]), acc = half(s.acc[q]);
+                        any |= bwd_pixel_step<kConsistent>(ra, rb, rc.x, pxf, -half(s.npy[q]), contributor < s.last[k],
+                                                           T, acc, half(s.d[q][0]), half(s.d[q][1]), half(s.d[q][2]),
+                                                           half(s.bgT[q]), sums);
+                        s.T[q] = (k & 1) ? f2(f2_lo(s.T[q]), T) : f2(T, f2_hi(s.T[q]));
+                        s.acc[q] = (k & 1) ? f2(f2_lo(s.acc[q]), acc) : f2(acc, f2_hi(s.acc[q]));
+                    }
+                } else {
+                    const float sx = __fmul_rn(ra.z, dx), nbx = -__fmul_rn(ra.w, dx);
+#pragma unroll
+                    for (int q = 0; q < NP; q++)
+                        if (kQuads == 1 || ((quad[q] >> bit) & 1u))
+                            any |= bwd_pair_step<kConsistent, NP>(s, q, ra, rb, rc.x, dx, sx, nbx, contributor, sums);
                 }
                 if (__any_sync(0xffffffffu, any)) {
-                    const float tot = warp_transpose_sum9(gr);
-                    if (q_lane < NG) atomicAdd(&sm.acc[(tid >> 5) >> 1][q_lane][j], tot);
+                    const float tot = warp_column_sum9(sums, dx);
+                    if constexpr (kOwnSlot) {
+                        touched |= 1u << bit;
+                        if (q_lane < NG) sm.acc[warp][j][q_lane] = tot;
+                    } else {
+                        if (q_lane < NG) atomicAdd(&sm.acc[warp >> 1][j][q_lane], tot);
+                    }
                 }
             }
+            if constexpr (kOwnSlot)
+                if ((tid & 31) == 0) sm.live[warp][k0 >> 5] = touched;
         }
         __syncthreads();
-        // this batch's per-pair gradients, at each pair's emission index: the slot
-        // sums times the pair's own factors
+        // this batch's per-pair gradients, at each pair's emission index: the slot sums times
+        // the pair's own factors (opacity, conic, -W/2, -H/2, -1/2 of backward.cu:537-551)
         for (uint32_t e = tid; e < cnt; e += NT) {
             float* dst = a.pgrad + (size_t)__float_as_uint(R[e].c.w) * NG;
             float sum[NG];
 #pragma unroll
-            for (int q = 0; q < NG; q++) {
-                float v = 0.f;
+            for (int q = 0; q < NG; q++) sum[q] = 0.f;
 #pragma unroll
-                for (int sl = 0; sl < kSlots; sl++) {
-                    v += sm.acc[sl][q][e];
-                    sm.acc[sl][q][e] = 0.f;
+            for (int sl = 0; sl < kSlots; sl++) {
+                if (kOwnSlot && !((sm.live[sl][e >> 5] >> (e & 31)) & 1u)) continue;
+#pragma unroll
+                for (int q = 0; q < NG; q++) {
+                    sum[q] += sm.acc[sl][e][q];
+                    if (!kOwnSlot) sm.acc[sl][e][q] = 0.f;
                 }
-                sum[q] = v;
             }
             const float4 ea = R[e].a, eb = R[e].b;  // conic (ea.z, ea.w, eb.x), opacity eb.y
             const float o = eb.y;
@@ -1154,8 +1413,11 @@ void fwd_launch(int grid, const ImageState& im, const BinState& b, long long K, 
         launch_long_kernel(band_shape, a, im.long_list, im.long_ctr, (uint32_t)grid, s);
         note_launches(2);
     }
-    render_fwd_kernel<PPT, B><<<grid, 256 / PPT, fwd_smem_bytes<B>(stats), s>>>(a, (uint32_t)(split > 0 ? split : 0),
-                                                                                err);
+    const uint32_t split_min = (uint32_t)(split > 0 ? split : 0);
+    if (stats)
+        render_fwd_kernel<PPT, B, kStats><<<grid, 256 / PPT, fwd_smem_bytes<B>(true), s>>>(a, split_min, err);
+    else
+        render_fwd_kernel<PPT, B, kWeights><<<grid, 256 / PPT, fwd_smem_bytes<B>(false), s>>>(a, split_min, err);
 }
 
 // Dynamic shared memory of a backward kernel instantiation (opted in once per process
