@@ -160,6 +160,7 @@ def profile_read(reset=True):
 
 
 def set_render_config(fwd_ppt=2, fwd_batch=256, bwd_ppt=2, bwd_batch=256):
+    """Fix the compositing shapes (until the first call the library chooses them per launch)."""
     check(lib().fgs_set_render_config(int(fwd_ppt), int(fwd_batch), int(bwd_ppt), int(bwd_batch)),
           "fgs_set_render_config")
 

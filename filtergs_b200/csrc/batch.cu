@@ -62,6 +62,7 @@ struct Batch {
     TileArgs* d_args_bwd;
     std::vector<TileArgs> h_args;  // host copy of d_args_fwd ++ d_args_bwd (sources of pointer updates)
     uint32_t* d_begin;
+    std::vector<uint32_t> h_begin;  // host copy of d_begin
     uint32_t* d_queue;
     uint32_t* d_long;  // long-tile bins [32][total_tiles], then their 34 counters
     unsigned* d_err;
@@ -244,6 +245,7 @@ void* fgs_batch_create(const fgs_raster_args* shared, int nviews, const fgs_view
         TileArgs f{};
         f.ranges = s.im.ranges; f.recs = s.b.rec; f.W = va.width; f.H = va.height; f.bg = shared->background;
         f.out_color = va.out_color; f.final_T = s.im.final_T; f.n_contrib = s.im.n_contrib;
+        f.totals = s.g.total;
         TileArgs bk = f;
         bk.out_color = nullptr;
         bk.dL_dpix = va.dL_dout_color;
@@ -254,6 +256,7 @@ void* fgs_batch_create(const fgs_raster_args* shared, int nviews, const fgs_view
         B->views.push_back(s);
     }
     B->total_tiles = begin[nviews];
+    B->h_begin = begin;
     std::vector<FoldView> fold(nviews);
     for (int v = 0; v < nviews; v++) {
         const ViewState& s = B->views[v];
@@ -340,6 +343,9 @@ int fgs_batch_forward(void* handle, void* stream)
         const PreParams& p0 = B->views[0].pre;
         launch_pack_gaussians(B->P, p0.means, p0.opac, p0.scales, p0.rots, B->packed, s);
     }
+    const RenderConfig rc = get_render_config();
+    uint32_t* long_ctr = B->d_long + 32 * (size_t)B->total_tiles;
+    if (rc.rule_long()) cudaMemsetAsync(long_ctr, 0, 34 * sizeof(uint32_t), s);  // the views' ranges add to it
     if (cudaEventRecord(B->forked, s) != cudaSuccess) return FGS_ERR_CUDA;
     for (int i = 0; i < ns; i++) cudaStreamWaitEvent(B->aux[i], B->forked, 0);
     for (int vi = 0; vi < B->V; vi++) {
@@ -365,7 +371,10 @@ int fgs_batch_forward(void* handle, void* stream)
             launch_tile_sort(v.g, v.b, v.cap, v.tile_bits, v.pre.W, v.pre.H, vs, v.g.total);
         }
         StageTimer t(FGS_STAGE_RANGES, vs);
-        launch_ranges(v.b, v.im, v.cap, v.num_tiles, vs, v.g.total);
+        LongList lng{};
+        if (rc.rule_long())
+            lng = LongList{B->d_long, long_ctr, B->total_tiles, B->h_begin[vi], v.g.total, nullptr, nullptr};
+        launch_ranges(v.b, v.im, v.cap, v.num_tiles, vs, v.g.total, lng);
     }
     for (int i = 0; i < ns; i++) {
         cudaEventRecord(B->joined[i], B->aux[i]);
@@ -375,8 +384,8 @@ int fgs_batch_forward(void* handle, void* stream)
     zero_point_weight_kernel<<<dim3((unsigned)((B->P + 255) / 256 < 592 ? (B->P + 255) / 256 : 592), (unsigned)B->V),
                                256, 0, s>>>(B->d_args_fwd, B->P);
     note_launches(1);
-    launch_render_fwd_multi(B->d_args_fwd, B->d_begin, B->V, B->total_tiles, B->d_queue, B->d_long,
-                            B->d_long + 32 * (size_t)B->total_tiles, B->d_err, s);
+    launch_render_fwd_multi(rc, B->d_args_fwd, B->d_begin, B->V, B->total_tiles, B->d_queue, B->d_long, long_ctr,
+                            B->d_err, s);
     return cudaGetLastError() == cudaSuccess ? FGS_OK : FGS_ERR_CUDA;
 }
 
@@ -389,7 +398,7 @@ int fgs_batch_backward(void* handle, void* stream)
     if (!B->g_means3D || !B->g_opacity) return FGS_ERR_ARG;
     {
         StageTimer t(FGS_STAGE_RENDER_BWD, s);
-        launch_render_bwd_multi(B->d_args_bwd, B->d_begin, B->V, B->total_tiles, B->d_queue + 1, B->consistent,
+        launch_render_bwd_multi(B->d_args_bwd, B->d_begin, B->h_begin.data(), B->V, B->d_queue + 1, B->consistent,
                                 B->d_err, s);
     }
     StageTimer t(FGS_STAGE_PREPROCESS_BWD, s);

@@ -178,6 +178,17 @@ int make_params(const fgs_raster_args* a, PreParams& p, bool backward)
     return FGS_OK;
 }
 
+// The launch rule's long-tile list of one view (counters zeroed here), or none when the caller set
+// a shape or a split.
+LongList long_list_of(const RenderConfig& c, const ImageState& im, int num_tiles, const unsigned long long* totals,
+                      const BinState* stats, cudaStream_t s)
+{
+    if (!c.rule_long()) return LongList{};
+    cudaMemsetAsync(im.long_ctr, 0, 34 * sizeof(uint32_t), s);
+    return LongList{im.long_list, im.long_ctr, (uint32_t)num_tiles, 0u, totals, stats ? stats->kv_sum : nullptr,
+                    stats ? stats->kv_cnt : nullptr};
+}
+
 namespace {
 
 // rasterizer_impl.cu:44-55
@@ -415,6 +426,7 @@ int fgs_forward_render(const fgs_raster_args* a, void* geom, void* image, void* 
     GeomState g = geom_views(geom, p.P);
     ImageState im = image_views(image, W, H);
     BinCarve bc = carve_bin(binning, K, p.P);
+    const RenderConfig rc = get_render_config();
     const bool stats = a->ogfs_enable_stats != 0;
     if (stats && stats_host && stats_len < 9 + 2 * FGS_STATS_SLOTS) return FGS_ERR_ARG;
     if (p.P > 0) cudaMemsetAsync(out_point_weight, 0, sizeof(float) * (size_t)p.P, s);
@@ -430,11 +442,11 @@ int fgs_forward_render(const fgs_raster_args* a, void* geom, void* image, void* 
     }
     {
         StageTimer t(FGS_STAGE_RANGES, s);
-        launch_ranges(bc.b, im, K, num_tiles, s);
+        launch_ranges(bc.b, im, K, num_tiles, s, nullptr, long_list_of(rc, im, num_tiles, g.total, stats ? &bc.b : nullptr, s));
     }
     {
         StageTimer t_render(FGS_STAGE_RENDER_FWD, s);
-        launch_render_fwd(W, H, im, bc.b, K, a->background, out_color, out_point_id, out_point_weight_pixel,
+        launch_render_fwd(rc, W, H, im, bc.b, K, g.total, a->background, out_color, out_point_id, out_point_weight_pixel,
                           out_point_weight, stats && K > 0, g.err, s);
     }
     if ((st = check_launch())) return st;
@@ -702,7 +714,7 @@ int fgs_debug_lookback_fault(unsigned int skip_chunk, unsigned long long wait_ns
 int fgs_set_render_config(int fwd_ppt, int fwd_batch, int bwd_ppt, int bwd_batch)
 {
     const RenderConfig cur = get_render_config();
-    const RenderConfig c{fwd_ppt, fwd_batch, bwd_ppt, bwd_batch, cur.fwd_split, cur.fwd_band};
+    const RenderConfig c{fwd_ppt, fwd_batch, bwd_ppt, bwd_batch, cur.fwd_split, cur.fwd_band, true, cur.own_split};
     if (!valid_render_config(c)) return FGS_ERR_ARG;
     set_render_config(c);
     return FGS_OK;
@@ -713,6 +725,7 @@ int fgs_set_render_split(int min_records, int band_shape)
     RenderConfig c = get_render_config();
     c.fwd_split = min_records;
     c.fwd_band = band_shape;
+    c.own_split = true;
     if (!valid_render_config(c)) return FGS_ERR_ARG;
     set_render_config(c);
     return FGS_OK;

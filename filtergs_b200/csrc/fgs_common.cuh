@@ -456,6 +456,22 @@ __device__ __forceinline__ uint32_t quad_mask(const PairRecord& g, float tx0, fl
     return m;
 }
 
+// The launch rule's long tiles: tiles with at least this many records are rendered in
+// units of 8x4 pixels (render.cu); totals = {pairs K, visible Gaussians V} of the view.
+// With K <= 2 V the splats are small (most touch one tile: a distant level of detail) and
+// sit in few tiles: units pay from 256 records on (8M-node LoD views at 1080p, 1.1M to
+// 8.5M pairs: 0.47 to 1.08 ms against 1.1 to 5.6 ms without; 1M nodes at 720p: 0.14 to
+// 0.34 against 0.29 to 1.43; in the earlier bands 256 beat 1024 on all of them).  Larger
+// splats touch most of a tile's units, which then do more work together than the tile's
+// own warps (2M-Gaussian view at 1080p, tiles of at most 561 records: 0.30 ms without,
+// 0.34 in bands from 512, 0.88 from 256), so only a tile that would outlast the rest is split: one
+// longer than 1024 records and twice the mean load of the 1184 tile blocks resident.
+__device__ __forceinline__ uint32_t auto_split_min(const unsigned long long* totals)
+{
+    const unsigned long long K = __ldg(totals), V = __ldg(totals + 1);
+    return K <= 2 * V ? 256u : max(1024u, (uint32_t)(min(K, 1ull << 30) / 592));
+}
+
 // ---------------------------------------------------------------- warp helpers
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31; }
 

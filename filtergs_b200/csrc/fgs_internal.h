@@ -114,12 +114,26 @@ int sort_chunk_size();
 // K is the pair count, or the capacity when n_dev (device-side count) is given.
 void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int tile_bits, int W, int H, cudaStream_t s,
                       const unsigned long long* n_dev = nullptr);
+struct RenderConfig;
+// Where the tiles that the launch rule renders in bands are listed (render.cu): list [32][cap]
+// binned by log2(records), ctr [34] (zeroed by the caller) and the first id of this view's tiles.
+// totals: the view's {pairs, visible} on the device; kv_*: zeroed for the listed tiles when given.
+struct LongList {
+    uint32_t* list;
+    uint32_t* ctr;
+    uint32_t cap, id_base;
+    const unsigned long long* totals;
+    float* kv_sum;
+    uint32_t* kv_cnt;
+};
+// Tile ranges of the K sorted pairs; lists the long tiles when lng.list is set.
 void launch_ranges(const BinState& b, const ImageState& im, long long K, int num_tiles, cudaStream_t s,
-                   const unsigned long long* n_dev = nullptr);
-// K: the pair count (or capacity) of b, for the statistics' zeroing when long tiles are split.
-void launch_render_fwd(int W, int H, const ImageState& im, const BinState& b, long long K, const float* bg,
-                       float* out_color, int* point_id, float* pw_pixel, float* point_weight, bool stats,
-                       unsigned* err, cudaStream_t s);
+                   const unsigned long long* n_dev, const LongList& lng);
+// K: the pair count (or capacity) of b, for the statistics' zeroing when long tiles are split;
+// totals as in LongList (the long tiles are in im when the launch rule is in force).
+void launch_render_fwd(const RenderConfig& c, int W, int H, const ImageState& im, const BinState& b, long long K,
+                       const unsigned long long* totals, const float* bg, float* out_color, int* point_id,
+                       float* pw_pixel, float* point_weight, bool stats, unsigned* err, cudaStream_t s);
 void launch_render_bwd(int W, int H, const ImageState& im, const BinState& b, const float* bg,
                        const float* dL_dpix, int consistent, unsigned* err, cudaStream_t s);
 // Densification statistics a training step keeps per Gaussian (null pointers: off).
@@ -193,6 +207,7 @@ struct TileArgs {
     float* out_point_weight;
     float* kv_sum;
     uint32_t* kv_cnt;
+    const unsigned long long* totals;  // {pairs, visible}: the launch rule's long tiles (auto_split_min)
     // backward input / output
     const float* dL_dpix;
     float* pgrad;  // [K][9] per-pair gradients, indexed by the record's emission index
@@ -201,10 +216,13 @@ struct TileArgs {
 // Persistent multi-view compositing over the tiles of `nviews` views; begin[v]
 // is the first work item of view v (begin[nviews] == total_tiles); queue is a
 // device counter (zeroed here).
-// long_list: [32 * total_tiles] scratch, long_ctr: [34] scratch (bands of long tiles; statistics must be off).
-void launch_render_fwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
-                             uint32_t* queue, uint32_t* long_list, uint32_t* long_ctr, unsigned* err, cudaStream_t s);
-void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
+// long_list: [32 * total_tiles], long_ctr: [34] (bands of long tiles; statistics must be off): scratch, or
+// filled by the views' launch_ranges when the launch rule is in force.
+void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const uint32_t* begin, int nviews,
+                             uint32_t total_tiles, uint32_t* queue, uint32_t* long_list, uint32_t* long_ctr,
+                             unsigned* err, cudaStream_t s);
+// host_begin: the values of begin; queue: two counters.
+void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, const uint32_t* host_begin, int nviews,
                              uint32_t* queue, int consistent, unsigned* err, cudaStream_t s);
 
 // Render kernel shape: pixels per thread {1,2,4} and records per shared-memory batch {64,128,256}.
@@ -212,7 +230,13 @@ struct RenderConfig {
     int fwd_ppt, fwd_batch, bwd_ppt, bwd_batch;
     int fwd_split;  // forward: tiles with at least this many records are rendered in bands (0: never)
     int fwd_band;   // band shape: 0 = 16x2, 1 = 8x4, 2 = 4x4, 3 = 4x2 pixels per warp
+    // Until a caller sets them, the shapes and the split are chosen per launch (render.cu):
+    bool own_shape;  // the four shape fields were set (fgs_set_render_config)
+    bool own_split;  // the split fields were set (fgs_set_render_split)
+    bool rule_long() const { return !own_shape && !own_split; }  // long tiles by the launch rule
 };
+LongList long_list_of(const RenderConfig& c, const ImageState& im, int num_tiles, const unsigned long long* totals,
+                      const BinState* stats, cudaStream_t s);
 bool valid_render_config(const RenderConfig& c);
 void set_render_config(const RenderConfig& c);
 RenderConfig get_render_config();

@@ -351,6 +351,7 @@ template <int PPT, int kBatch, int kOut>
 __device__ __forceinline__ void render_fwd_tile(FwdSmem<kBatch>& sm, const TileArgs& a, int tile, uint32_t& gb,
                                                 uint32_t split_min, unsigned* err)
 {
+    // (every thread of the CTA takes the same way here)
     constexpr int NT = 256 / PPT;
     constexpr int NP = PPT > 1 ? PPT / 2 : 1;
     constexpr int kQuads = warp_quads<PPT>();
@@ -902,35 +903,11 @@ __device__ __forceinline__ bool next_long_tile(uint32_t* ctr, const uint32_t* __
 }
 
 template <int BW, int BH>
-__global__ void __launch_bounds__(LongTile<BW, BH>::kThreads)
-    render_fwd_long_kernel(TileArgs a, const uint32_t* __restrict__ list, uint32_t* ctr, uint32_t cap)
+__device__ __forceinline__ void long_tile_loop(unsigned char* dyn, const TileArgs* __restrict__ views,
+                                               const uint32_t* __restrict__ begin, int nviews,
+                                               const uint32_t* __restrict__ list, uint32_t* ctr, uint32_t cap)
 {
-    extern __shared__ __align__(128) unsigned char long_dyn[];
-    auto& sm = *reinterpret_cast<LongSmem<LongTile<BW, BH>::kChunk>*>(long_dyn);
-    __shared__ uint32_t s_id;
-    __shared__ int s_ok, s_group;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            uint32_t id = 0;
-            int group = 0;
-            s_ok = next_long_tile<LongTile<BW, BH>::kGroups>(ctr, list, cap, id, group);
-            s_id = id;
-            s_group = group;
-        }
-        __syncthreads();
-        if (!s_ok) break;
-        render_long_tile<BW, BH>(sm, a, (int)s_id, s_group);
-        __syncthreads();  // s_id / s_group / s_ok are rewritten for the next item
-    }
-}
-
-template <int BW, int BH>
-__global__ void __launch_bounds__(LongTile<BW, BH>::kThreads)
-    render_fwd_long_multi_kernel(const TileArgs* __restrict__ views, const uint32_t* __restrict__ begin, int nviews,
-                                 const uint32_t* __restrict__ list, uint32_t* ctr, uint32_t cap)
-{
-    extern __shared__ __align__(128) unsigned char long_dyn[];
-    auto& sm = *reinterpret_cast<LongSmem<LongTile<BW, BH>::kChunk>*>(long_dyn);
+    auto& sm = *reinterpret_cast<LongSmem<LongTile<BW, BH>::kChunk>*>(dyn);
     __shared__ uint32_t s_id;
     __shared__ int s_ok, s_group;
     for (;;) {
@@ -944,8 +921,269 @@ __global__ void __launch_bounds__(LongTile<BW, BH>::kThreads)
         __syncthreads();
         if (!s_ok) break;
         const uint32_t id = s_id;
-        const int v = view_of(begin, nviews, id);
-        render_long_tile<BW, BH>(sm, views[v], (int)(id - begin[v]), s_group);
+        const int v = begin ? view_of(begin, nviews, id) : 0;
+        render_long_tile<BW, BH>(sm, views[v], (int)(begin ? id - begin[v] : id), s_group);
+        __syncthreads();  // s_id / s_group / s_ok are rewritten for the next item
+    }
+}
+
+template <int BW, int BH>
+__global__ void __launch_bounds__(LongTile<BW, BH>::kThreads)
+    render_fwd_long_kernel(TileArgs a, const uint32_t* __restrict__ list, uint32_t* ctr, uint32_t cap)
+{
+    extern __shared__ __align__(128) unsigned char long_dyn[];
+    long_tile_loop<BW, BH>(long_dyn, &a, nullptr, 1, list, ctr, cap);
+}
+
+template <int BW, int BH>
+__global__ void __launch_bounds__(LongTile<BW, BH>::kThreads)
+    render_fwd_long_multi_kernel(const TileArgs* __restrict__ views, const uint32_t* __restrict__ begin, int nviews,
+                                 const uint32_t* __restrict__ list, uint32_t* ctr, uint32_t cap)
+{
+    extern __shared__ __align__(128) unsigned char long_dyn[];
+    long_tile_loop<BW, BH>(long_dyn, views, begin, nviews, list, ctr, cap);
+}
+
+// ---------------------------------------------------------------- long tiles by quads
+// The launch rule's form of a long tile: a CTA renders a unit of 8x4 pixels, four warps
+// with a 4x2 band each, and stages only the records whose quad_mask has the unit's quad.
+// What bounds a tile of thousands of small splats is staging, not compositing: with
+// every record staged and tested by each of the tile's eight CTAs, two thirds of the
+// time went there.  Here a CTA reads the 4-byte masks of kUnitIn records (the next ones
+// in flight meanwhile), compacts the survivors (about a quarter) in order, loads only
+// those records and tests only those against the bands.  Per pixel the same records in
+// the same order with the same arithmetic as on the tile path.  8M-node LoD views at
+// 1080p with 2.7M / 6.4M / 8.5M pairs: 0.60 / 1.08 / 1.06 ms; in bands that stage every
+// record 0.78 / 1.42 / 1.36; one CTA per tile 1.66 / 2.63 / 5.59.
+constexpr int kUnitIn = 512, kUnitRecs = 256, kUnits = 8, kUnitThreads = 128;
+
+struct UnitSmem {
+    PairRecord rec[kUnitRecs];
+    uint32_t mask[kUnitRecs];  // the unit's bands each record can reach (bit = warp)
+    uint32_t wmax[kUnitRecs];  // as in LongSmem
+    float ksum[kUnitRecs];
+    uint32_t kcnt[kUnitRecs];
+    uint16_t idx[kUnitIn];     // survivors of the kUnitIn records
+    uint32_t cnt[kUnitIn / 32];
+};
+
+__device__ __forceinline__ void render_unit(UnitSmem& sm, const TileArgs& a, int tile, int unit)
+{
+    constexpr int kPix = 8, kSlots = 4, kPer = kUnitIn / kUnitThreads;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int W = a.W, H = a.H;
+    const int gx = (W + kTileX - 1) / kTileX;
+    const int bx = tile % gx, by = tile / gx, ux = unit & 1, uy = unit >> 1;
+    const float tx0 = (float)(bx * kTileX), ty0 = (float)(by * kTileY);
+    const int band0 = 8 * uy + 2 * ux;  // the unit's bands in band_mask<4, 2>: band0 + {0, 1, 4, 5}
+    const int qbit = 2 * (uy >> 1) + ux;
+    const int pix_lane = lane % kPix, slot = lane / kPix;
+    const int px = bx * kTileX + 8 * ux + 4 * (warp & 1) + pix_lane % 4;
+    const int py = by * kTileY + 4 * uy + 2 * (warp >> 1) + pix_lane / 4;
+    const bool mine = lane < kPix;  // the pixel's owner lane keeps its state
+    const uint2 range = a.ranges[tile];
+    const uint32_t n = range.y - range.x;
+    const bool stats = a.kv_sum != nullptr;
+    const PairRecord* recs = a.recs + range.x;
+    const float pxf = (float)px, pyf = (float)py;
+    float T = 1.0f, C[3] = {0.f, 0.f, 0.f}, wmax = 0.f;
+    uint32_t last = 0;
+    int maxid = -1;
+    bool done = !(mine && px < W && py < H);
+    const unsigned lt = (1u << lane) - 1u;
+
+    uint32_t m[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+        const uint32_t e = (uint32_t)(i * kUnitThreads + tid);
+        m[i] = e < n ? __float_as_uint(__ldg(&recs[e].c.z)) : 0u;
+    }
+    bool all_done = false;
+    for (uint32_t c0 = 0; c0 < n && !all_done; c0 += kUnitIn) {
+        uint32_t b[kPer];
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {
+            b[i] = __ballot_sync(0xffffffffu, (m[i] >> qbit) & 1u);
+            if (lane == 0) sm.cnt[i * (kUnitThreads / 32) + warp] = __popc(b[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {  // the next masks, in flight while these records are composited
+            const uint32_t e = c0 + kUnitIn + (uint32_t)(i * kUnitThreads + tid);
+            m[i] = e < n ? __float_as_uint(__ldg(&recs[e].c.z)) : 0u;
+        }
+        __syncthreads();
+        uint32_t total = 0;
+#pragma unroll
+        for (int i = 0; i < kPer; i++)
+#pragma unroll
+            for (int w = 0; w < kUnitThreads / 32; w++) {
+                if (w == warp && ((b[i] >> lane) & 1u))
+                    sm.idx[total + __popc(b[i] & lt)] = (uint16_t)(i * kUnitThreads + tid);
+                total += sm.cnt[i * (kUnitThreads / 32) + w];
+            }
+        __syncthreads();
+        for (uint32_t s0 = 0; s0 < total && !all_done; s0 += kUnitRecs) {
+            const uint32_t cnt = min((uint32_t)kUnitRecs, total - s0);
+#pragma unroll
+            for (int q = 0; q < kUnitRecs / kUnitThreads; q++) {
+                const int e = q * kUnitThreads + tid;
+                uint32_t bits = 0;
+                if ((uint32_t)e < cnt) {
+                    const PairRecord r = recs[c0 + sm.idx[s0 + e]];
+                    const uint32_t all = band_mask<4, 2>(r.a, r.b, tx0, ty0) >> band0;
+                    bits = (all & 3u) | ((all >> 2) & 12u);
+                    sm.rec[e] = r;
+                }
+                sm.mask[e] = bits;
+                sm.wmax[e] = 0u;
+                if (stats) {
+                    sm.ksum[e] = 0.f;
+                    sm.kcnt[e] = 0u;
+                }
+            }
+            __syncthreads();
+            for (uint32_t k = 0; k < cnt && !__all_sync(0xffffffffu, done); k += 32) {
+                uint32_t live = __ballot_sync(0xffffffffu, (sm.mask[k + lane] >> warp) & 1u);
+                const PairRecord* R = sm.rec + k;
+                while (live) {
+                    // the next kSlots live records, in order (32: none); lanes of slot s
+                    // evaluate record js[s] at their pixel
+                    uint32_t js[kSlots];
+                    uint32_t mj = 32u;
+#pragma unroll
+                    for (int s = 0; s < kSlots; s++) {
+                        js[s] = live ? (uint32_t)(__ffs(live) - 1) : 32u;
+                        live &= live - 1;
+                        if (s == slot) mj = js[s];
+                    }
+                    const bool pdone = __shfl_sync(0xffffffffu, done, pix_lane);
+                    const float al = (mj < 32u && !pdone) ? fwd_alpha(R[mj].a, R[mj].b, pxf, pyf) : 0.f;
+#pragma unroll
+                    for (int s = 0; s < kSlots; s++) {
+                        const float as = __shfl_sync(0xffffffffu, al, s * kPix + pix_lane);
+                        const uint32_t j = js[s];
+                        if (j < 32u) {
+                            const float w = fwd_accumulate(as, R[j].b, R[j], c0 + sm.idx[s0 + k + j] + 1, T, C, wmax,
+                                                           maxid, last, done);
+                            if (w > 0.f) {
+                                atomicMax(&sm.wmax[k + j], __float_as_uint(w));
+                                if (stats) {
+                                    atomicAdd(&sm.ksum[k + j], w);
+                                    atomicAdd(&sm.kcnt[k + j], 1u);
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+            // (every pixel of this unit done: no later record can contribute)
+            all_done = __syncthreads_and(done);
+#pragma unroll
+            for (int q = 0; q < kUnitRecs / kUnitThreads; q++) {
+                const uint32_t e = (uint32_t)(q * kUnitThreads + tid);
+                const uint32_t wm = e < cnt ? sm.wmax[e] : 0u;
+                if (!wm) continue;
+                if (a.out_point_weight)
+                    atomicMax(reinterpret_cast<unsigned*>(a.out_point_weight) + __float_as_int(sm.rec[e].c.y), wm);
+                if (stats) {
+                    const uint32_t at = range.x + c0 + sm.idx[s0 + e];
+                    atomicAdd(a.kv_sum + at, sm.ksum[e]);
+                    atomicAdd(a.kv_cnt + at, sm.kcnt[e]);
+                }
+            }
+        }
+    }
+    if (mine && px < W && py < H) {
+        const int pix = W * py + px;
+        a.final_T[pix] = T;
+        a.n_contrib[pix] = last;
+        a.out_color[pix] = __fmaf_rn(T, a.bg[0], C[0]);
+        a.out_color[H * W + pix] = __fmaf_rn(T, a.bg[1], C[1]);
+        a.out_color[2 * H * W + pix] = __fmaf_rn(T, a.bg[2], C[2]);
+        if (a.out_point_id) a.out_point_id[pix] = maxid;
+        if (a.out_pw_pixel) a.out_pw_pixel[pix] = wmax;
+    }
+}
+
+// Units of long tiles from the queue until it is empty (all threads of the CTA).
+__device__ __forceinline__ void unit_loop(unsigned char* dyn, const TileArgs* __restrict__ views,
+                                          const uint32_t* __restrict__ begin, int nviews,
+                                          const uint32_t* __restrict__ list, uint32_t* ctr, uint32_t cap)
+{
+    UnitSmem& sm = *reinterpret_cast<UnitSmem*>(dyn);
+    __shared__ uint32_t s_id;
+    __shared__ int s_ok, s_unit;
+    for (;;) {
+        if (threadIdx.x == 0) {
+            uint32_t id = 0;
+            int unit = 0;
+            s_ok = next_long_tile<kUnits>(ctr, list, cap, id, unit);
+            s_id = id;
+            s_unit = unit;
+        }
+        __syncthreads();
+        if (!s_ok) break;
+        const uint32_t id = s_id;
+        const int v = begin ? view_of(begin, nviews, id) : 0;
+        render_unit(sm, views[v], (int)(begin ? id - begin[v] : id), s_unit);
+        __syncthreads();  // s_id / s_unit / s_ok are rewritten for the next item
+    }
+}
+
+// ---------------------------------------------------------------- the launch rule's forward
+// Used until a caller sets a shape or a split: 2 pixels per lane and 128-record batches
+// (over all shapes within 5% of the best on views of 256x256 to 1080p, one or sixteen),
+// and the long tiles (listed by ranges_kernel) in units by the same launch: its first
+// blocks, one resident set, take them from the queue before the tiles' own blocks start,
+// so a view without long tiles pays for no second kernel and no listing pass (10 us of
+// 300), only for blocks that leave at once.
+constexpr int kRulePpt = 2, kRuleBatch = 128;
+static_assert(kUnitThreads == 256 / kRulePpt, "one block size for tiles and units");
+static_assert(sizeof(UnitSmem) <= offsetof(FwdSmem<kRuleBatch>, ksum), "shared memory");
+
+template <int kOut>
+__global__ void __launch_bounds__(256 / kRulePpt, fwd_min_ctas<kRulePpt>())
+    render_fwd_rule_kernel(TileArgs a, int long_ctas, const uint32_t* __restrict__ list, uint32_t* ctr, uint32_t cap,
+                           unsigned* err)
+{
+    extern __shared__ __align__(128) unsigned char fwd_dyn[];
+    if ((int)blockIdx.x < long_ctas) {
+        if (*(volatile uint32_t*)ctr) unit_loop(fwd_dyn, &a, nullptr, 1, list, ctr, cap);
+        return;
+    }
+    FwdSmem<kRuleBatch>& sm = *reinterpret_cast<FwdSmem<kRuleBatch>*>(fwd_dyn);
+    fwd_smem_init(sm, 256 / kRulePpt, kOut == kStats);
+    uint32_t gb = 0;
+    render_fwd_tile<kRulePpt, kRuleBatch, kOut>(sm, a, (int)blockIdx.x - long_ctas, gb, auto_split_min(a.totals), err);
+}
+
+__global__ void __launch_bounds__(256 / kRulePpt, fwd_min_ctas<kRulePpt>())
+    render_fwd_multi_rule_kernel(const TileArgs* __restrict__ views, const uint32_t* __restrict__ begin, int nviews,
+                                 uint32_t total, uint32_t* queue, const uint32_t* __restrict__ list, uint32_t* ctr,
+                                 unsigned* err)
+{
+    extern __shared__ __align__(128) unsigned char fwd_dyn[];
+    if (*(volatile uint32_t*)ctr) {
+        unit_loop(fwd_dyn, views, begin, nviews, list, ctr, total);
+        __syncthreads();
+    }
+    FwdSmem<kRuleBatch>& sm = *reinterpret_cast<FwdSmem<kRuleBatch>*>(fwd_dyn);
+    __shared__ uint32_t s_item;
+    fwd_smem_init(sm, 256 / kRulePpt, false);
+    uint32_t gb = 0;
+    for (;;) {
+        if (threadIdx.x == 0) s_item = atomicAdd(queue, 1u);
+        __syncthreads();
+        const uint32_t item = s_item;
+        if (item >= total) break;
+        const int v = view_of(begin, nviews, item);
+        const TileArgs& a = views[v];  // fields read where used, not held in registers
+        const uint32_t split = auto_split_min(a.totals);
+        // (from the device descriptors: a captured graph follows fgs_batch_set_view_outputs)
+        if (a.out_point_weight || a.out_point_id || a.out_pw_pixel)
+            render_fwd_tile<kRulePpt, kRuleBatch, kWeights>(sm, a, (int)(item - begin[v]), gb, split, err);
+        else
+            render_fwd_tile<kRulePpt, kRuleBatch, kImage>(sm, a, (int)(item - begin[v]), gb, split, err);
         __syncthreads();
     }
 }
@@ -1306,8 +1544,9 @@ __global__ void __launch_bounds__(256 / PPT) render_bwd_kernel(TileArgs a, unsig
 template <int PPT, int kBatch, bool kConsistent>
 __global__ void __launch_bounds__(256 / PPT, bwd_multi_min_ctas<PPT>())
     render_bwd_multi_kernel(const TileArgs* __restrict__ views, const uint32_t* __restrict__ begin, int nviews,
-                            uint32_t total, uint32_t* queue, unsigned* err)
+                            uint32_t total, uint32_t* queue, uint32_t min_tiles, uint32_t max_tiles, unsigned* err)
 {
+    // the items are the tiles of the views of min_tiles .. max_tiles tiles (total of them)
     extern __shared__ __align__(128) unsigned char bwd_dyn[];
     BwdSmemT<PPT, kBatch>& sm = *reinterpret_cast<BwdSmemT<PPT, kBatch>*>(bwd_dyn);
     __shared__ uint32_t s_item;
@@ -1316,12 +1555,17 @@ __global__ void __launch_bounds__(256 / PPT, bwd_multi_min_ctas<PPT>())
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(queue, 1u);
         __syncthreads();
-        const uint32_t item = s_item;
+        uint32_t item = s_item;
         if (item >= total) break;
         int v = 0;
-        while (v + 1 < nviews && begin[v + 1] <= item) v++;
+        for (; v < nviews; v++) {
+            const uint32_t tiles = begin[v + 1] - begin[v];
+            if (tiles < min_tiles || tiles > max_tiles) continue;
+            if (item < tiles) break;
+            item -= tiles;
+        }
         const TileArgs& a = views[v];  // fields read where used, not held in registers
-        render_bwd_tile<PPT, kBatch, kConsistent>(sm, a, (int)(item - begin[v]), gb, err);
+        render_bwd_tile<PPT, kBatch, kConsistent>(sm, a, (int)item, gb, err);
         __syncthreads();
     }
 }
@@ -1329,7 +1573,7 @@ __global__ void __launch_bounds__(256 / PPT, bwd_multi_min_ctas<PPT>())
 }  // namespace
 
 namespace {
-RenderConfig g_cfg{2, 256, 2, 256, 0, 0};
+RenderConfig g_cfg{2, 256, 2, 256, 0, 0, false, false};
 
 // Dynamic shared memory of a forward launch: the whole FwdSmem with statistics,
 // up to its statistics sums without.
@@ -1479,15 +1723,36 @@ bool valid_render_config(const RenderConfig& c)
 void set_render_config(const RenderConfig& c) { g_cfg = c; }
 RenderConfig get_render_config() { return g_cfg; }
 
-void launch_render_fwd(int W, int H, const ImageState& im, const BinState& b, long long K, const float* bg,
-                       float* out_color, int* point_id, float* pw_pixel, float* point_weight, bool stats,
-                       unsigned* err, cudaStream_t s)
+namespace {
+template <int kOut>
+void fwd_rule_launch(int tiles, const TileArgs& a, const ImageState& im, unsigned* err, cudaStream_t s)
+{
+    const int long_ctas = (int)resident_ctas(render_fwd_rule_kernel<kOut>, 256 / kRulePpt);
+    render_fwd_rule_kernel<kOut><<<long_ctas + tiles, 256 / kRulePpt, fwd_smem_bytes<kRuleBatch>(kOut == kStats), s>>>(
+        a, long_ctas, im.long_list, im.long_ctr, (uint32_t)tiles, err);
+}
+}  // namespace
+
+void launch_render_fwd(const RenderConfig& c, int W, int H, const ImageState& im, const BinState& b, long long K,
+                       const unsigned long long* totals, const float* bg, float* out_color, int* point_id,
+                       float* pw_pixel, float* point_weight, bool stats, unsigned* err, cudaStream_t s)
 {
     const int gx = (W + kTileX - 1) / kTileX, gy = (H + kTileY - 1) / kTileY;
-    const RenderConfig c = g_cfg;
-    FGS_RENDER_DISPATCH(fwd_launch, c.fwd_ppt, c.fwd_batch, gx * gy, im, b, K, W, H, bg, out_color, point_id,
-                        pw_pixel, point_weight, stats, c.fwd_split, c.fwd_band, err, s);
     note_launches(1);
+    if (c.rule_long()) {
+        TileArgs a{};
+        a.ranges = im.ranges; a.recs = b.rec; a.W = W; a.H = H; a.bg = bg;
+        a.out_color = out_color; a.final_T = im.final_T; a.n_contrib = im.n_contrib; a.out_point_id = point_id;
+        a.out_pw_pixel = pw_pixel; a.out_point_weight = point_weight;
+        a.kv_sum = stats ? b.kv_sum : nullptr; a.kv_cnt = stats ? b.kv_cnt : nullptr;
+        a.totals = totals;
+        if (stats) fwd_rule_launch<kStats>(gx * gy, a, im, err, s);
+        else fwd_rule_launch<kWeights>(gx * gy, a, im, err, s);
+        return;
+    }
+    FGS_RENDER_DISPATCH(fwd_launch, c.own_shape ? c.fwd_ppt : kRulePpt, c.own_shape ? c.fwd_batch : kRuleBatch,
+                        gx * gy, im, b, K, W, H, bg, out_color, point_id, pw_pixel, point_weight, stats, c.fwd_split,
+                        c.fwd_band, err, s);
 }
 
 namespace {
@@ -1515,7 +1780,7 @@ void fwd_multi_launch(const TileArgs* views, const uint32_t* begin, int nviews, 
 
 template <int PPT, int B, bool kConsistent>
 void bwd_multi_launch_mode(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total, uint32_t* queue,
-                           unsigned* err, cudaStream_t s)
+                           uint32_t min_tiles, uint32_t max_tiles, unsigned* err, cudaStream_t s)
 {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
@@ -1525,43 +1790,86 @@ void bwd_multi_launch_mode(const TileArgs* views, const uint32_t* begin, int nvi
                                                   smem);
     const int grid = sms * (per_sm > 0 ? per_sm : 1);
     render_bwd_multi_kernel<PPT, B, kConsistent><<<grid, 256 / PPT, smem, s>>>(views, begin, nviews, total, queue,
-                                                                               err);
+                                                                               min_tiles, max_tiles, err);
 }
 
 template <int PPT, int B>
 void bwd_multi_launch(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total, uint32_t* queue,
-                      int consistent, unsigned* err, cudaStream_t s)
+                      uint32_t min_tiles, uint32_t max_tiles, int consistent, unsigned* err, cudaStream_t s)
 {
-    if (consistent) bwd_multi_launch_mode<PPT, B, true>(views, begin, nviews, total, queue, err, s);
-    else bwd_multi_launch_mode<PPT, B, false>(views, begin, nviews, total, queue, err, s);
+    if (consistent)
+        bwd_multi_launch_mode<PPT, B, true>(views, begin, nviews, total, queue, min_tiles, max_tiles, err, s);
+    else
+        bwd_multi_launch_mode<PPT, B, false>(views, begin, nviews, total, queue, min_tiles, max_tiles, err, s);
 }
 }  // namespace
 
-void launch_render_fwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
-                             uint32_t* queue, uint32_t* long_list, uint32_t* long_ctr, unsigned* err, cudaStream_t s)
+void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const uint32_t* begin, int nviews,
+                             uint32_t total_tiles, uint32_t* queue, uint32_t* long_list, uint32_t* long_ctr,
+                             unsigned* err, cudaStream_t s)
 {
     cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
-    const RenderConfig c = g_cfg;
-    FGS_RENDER_DISPATCH(fwd_multi_launch, c.fwd_ppt, c.fwd_batch, views, begin, nviews, total_tiles, queue, long_list,
-                        long_ctr, c.fwd_split, c.fwd_band, err, s);
     note_launches(1);
+    if (c.rule_long()) {
+        int dev = 0, sms = 148, per_sm = 1;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const size_t smem = fwd_smem_bytes<kRuleBatch>(false);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, render_fwd_multi_rule_kernel, 256 / kRulePpt, smem);
+        render_fwd_multi_rule_kernel<<<sms * (per_sm > 0 ? per_sm : 1), 256 / kRulePpt, smem, s>>>(
+            views, begin, nviews, total_tiles, queue, long_list, long_ctr, err);
+        return;
+    }
+    FGS_RENDER_DISPATCH(fwd_multi_launch, c.own_shape ? c.fwd_ppt : kRulePpt, c.own_shape ? c.fwd_batch : kRuleBatch,
+                        views, begin, nviews, total_tiles, queue, long_list, long_ctr, c.fwd_split, c.fwd_band, err,
+                        s);
 }
 
-void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
+namespace {
+// The backward's shape until a caller sets one: 4 pixels per lane and 64-record batches (two
+// warps per tile) for views whose tiles fill the GPU; for smaller ones, whose time is that of
+// their longest tiles, more and shorter warps: 2 pixels per lane and 128-record batches.
+// Measured, at 2 / at 4: 144 tiles 451 / 496 us, 920 tiles 164 / 205, 2304 tiles 184 / 201, 3600
+// tiles 234 / 235, 8160 tiles 395 / 372; but in a batch, where the other views' tiles fill the
+// GPU, 4 is 11% faster at any size, so the line lies where one view alone still gains 10%.  It
+// is drawn by the view's own tiles, alone and in a batch: a lane adds its pixels' terms in an
+// order that depends on the shape, and a batch's gradients equal the per-view ones bit for bit.
+constexpr uint32_t kSmallViewTiles = 2048;
+void bwd_rule(RenderConfig& c, bool small)
+{
+    if (c.own_shape) return;
+    c.bwd_ppt = small ? 2 : 4;
+    c.bwd_batch = small ? 128 : 64;
+}
+}  // namespace
+
+void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, const uint32_t* host_begin, int nviews,
                              uint32_t* queue, int consistent, unsigned* err, cudaStream_t s)
 {
-    cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
-    const RenderConfig c = g_cfg;
-    FGS_RENDER_DISPATCH(bwd_multi_launch, c.bwd_ppt, c.bwd_batch, views, begin, nviews, total_tiles, queue,
-                        consistent, err, s);
-    note_launches(1);
+    cudaMemsetAsync(queue, 0, 2 * sizeof(uint32_t), s);
+    RenderConfig c = g_cfg;
+    // the views of either kind: one launch each (one for all when the caller set the shape)
+    uint32_t items[2] = {0, 0};
+    for (int v = 0; v < nviews; v++) {
+        const uint32_t tiles = host_begin[v + 1] - host_begin[v];
+        items[!c.own_shape && tiles <= kSmallViewTiles] += tiles;
+    }
+    for (int small = 0; small < 2; small++) {
+        if (!items[small]) continue;
+        bwd_rule(c, small != 0);
+        const uint32_t lo = small || c.own_shape ? 0u : kSmallViewTiles + 1, hi = small ? kSmallViewTiles : 0xffffffffu;
+        FGS_RENDER_DISPATCH(bwd_multi_launch, c.bwd_ppt, c.bwd_batch, views, begin, nviews, items[small],
+                            queue + small, lo, hi, consistent, err, s);
+        note_launches(1);
+    }
 }
 
 void launch_render_bwd(int W, int H, const ImageState& im, const BinState& b, const float* bg,
                        const float* dL_dpix, int consistent, unsigned* err, cudaStream_t s)
 {
     const int gx = (W + kTileX - 1) / kTileX, gy = (H + kTileY - 1) / kTileY;
-    const RenderConfig c = g_cfg;
+    RenderConfig c = g_cfg;
+    bwd_rule(c, (uint32_t)(gx * gy) <= kSmallViewTiles);
     FGS_RENDER_DISPATCH(bwd_launch, c.bwd_ppt, c.bwd_batch, gx * gy, im, b, W, H, bg, dL_dpix, consistent, err, s);
     note_launches(1);
 }

@@ -347,13 +347,15 @@ int fgs_profile_enable(int on);
 /* Render kernel shape used by forward/backward in this process (no reference
  * counterpart; the reference hard-codes one pixel per thread and 256-record
  * batches): pixels per thread 1|2|4 and shared-memory batch 64|128|256 for
- * each of the forward and backward compositing kernels.  Chosen by the
- * autotuner (filtergs_b200/autotune.py).  cfg: int[4] out.             */
+ * each of the forward and backward compositing kernels.  Until this is
+ * called the library chooses them per launch from the view's tiles and pairs
+ * (the get call then reads 2, 256, 2, 256); the autotuner
+ * (filtergs_b200/autotune.py) sets them from measurements.  cfg: int[4] out. */
 int fgs_set_render_config(int fwd_ppt, int fwd_batch, int bwd_ppt, int bwd_batch);
 int fgs_get_render_config(int *cfg);
 /* Forward: tiles with at least min_records tile/Gaussian pairs are rendered in bands of pixels, one
- * warp per band and four bands per CTA, longest tiles first, before the other tiles (min_records 0,
- * the default: never).
+ * warp per band and four bands per CTA, longest tiles first, before the other tiles (min_records 0:
+ * never).  Until this or fgs_set_render_config is called, the library chooses the tiles per view.
  * band_shape: 0 = 16x2, 1 = 8x4, 2 = 4x4, 3 = 4x2 pixels per band.  The outputs do not change; long
  * tiles stop being the critical path of the forward.  Process-wide, like the above.
  * fgs_get_render_split: cfg int[2] out (min_records, band_shape).                                   */

@@ -122,3 +122,72 @@ def test_values_too_large_for_the_packed_form(cuda, shapes, which):
             keep = fine & (y.abs() < 1e12)
             if keep.any():
                 assert norm_rel(torch.where(keep, x, 0), torch.where(keep, y, 0)) <= 2e-5
+
+
+_RULE = """
+import sys
+import numpy as np, torch
+sys.path[:0] = {path!r}
+from _helpers import Case, S, ours, run_forward
+from filtergs_b200 import _lib
+from filtergs_b200.batched import BatchedRasterizer, Camera
+
+def case(P, scale, squeeze, W, H):
+    sc, cam = S.small_scene(P=P, seed=77, W=W, H=H)
+    sc["scales"] = (sc["scales"] * scale).astype(np.float32)
+    sc["means3D"][: P // 2, :2] *= squeeze
+    return Case(sc, cam)
+
+small = case(30000, 0.05, 0.05, 250, 190)   # K <= 2 V: bands from 256 records on
+large = case(9000, 1.0, 0.1, 333, 140)      # K > 2 V, one tile past 1024 records
+plain = case(3000, 1.0, 1.0, 147, 133)      # no long tile
+runs = [(c, st) for c in (small, large, plain) for st in (False, True)]
+rule = [run_forward(ours, c, stats=st) for c, st in runs]
+
+def batch(c):
+    a = c.torch_inputs()
+    cams = [Camera(c.cam.W, c.cam.H, c.cam.tanfovx, c.cam.tanfovy, a["viewmatrix"], a["projmatrix"], a["campos"])] * 3
+    br = BatchedRasterizer(a["means3D"], a["opacity"], a["scales"], a["rotations"], cams, shs=a["sh"],
+                           sh_degree=a["degree"], full_outputs=True)
+    br.step()
+    br.check()
+    return [(br.images[v].clone(), br.point_id[v], br.point_weight_pixel[v], br.point_weight[v]) for v in (0, 2)]
+
+batches = [batch(c) for c in (small, large)]
+lengths = []
+_lib.set_render_config(1, 64, 1, 64)
+_lib.set_render_split(0, 0)
+for (c, st), got in zip(runs, rule):
+    want = run_forward(ours, c, stats=st)
+    rg = ours.image_outputs(want[8], c.cam.W, c.cam.H)["ranges"]
+    lengths.append((int((rg[:, 1] - rg[:, 0]).max()), int(want[0]), int((want[5] > 0).sum())))
+    assert torch.equal(ours.image_outputs(got[8], c.cam.W, c.cam.H)["ranges"], rg)
+    for i in (1, 2, 3, 4, 5):
+        assert torch.equal(got[i], want[i]), i
+    if st:
+        assert np.allclose(got[9].numpy(), want[9].numpy(), rtol=1e-4, atol=1e-6)
+for c, views in zip((small, large), batches):
+    want = run_forward(ours, c)
+    for view in views:
+        for x, i in zip(view, (1, 2, 3, 4)):
+            assert torch.equal(x, want[i]), i
+n, K, V = lengths[0]
+assert K <= 2 * V and n >= 256, lengths
+n, K, V = lengths[2]
+assert K > 2 * V and n >= max(1024, K // 592), lengths
+assert lengths[4][0] < 1024, lengths
+print("rule ok", lengths)
+"""
+
+
+def test_launch_rule_gives_the_same_bits(cuda):
+    """The shapes and the long tiles the launch rule picks (before any set_render_* call, so in a process
+    of its own) against one pixel per lane without bands: one view and batched, with and without
+    statistics, with long tiles of small splats, of large ones, and without any."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = _RULE.format(path=[here, os.path.dirname(here)])
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "rule ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
