@@ -16,6 +16,7 @@
 //              training step keeps): sum of |dL/dmean2D[:, :2]| and the visibility
 //              count per Gaussian, plus this step's visible flag.
 #include <cmath>
+#include <initializer_list>
 
 #include "fgs_common.cuh"
 #include "fgs_internal.h"
@@ -296,12 +297,6 @@ __global__ void densify_dense_kernel(int P, const int* __restrict__ radii, const
     }
 }
 
-struct AdamRow {
-    float* p;
-    float* m;
-    float* v;
-};
-
 // sparse_optimizer.py:54-76 with torch's float32 arithmetic: the Python-float
 // coefficients beta and 1 - beta (formed in double) are rounded to float.
 __device__ __forceinline__ void adam_update(float& p, float& m, float& v, float g, float b1, float omb1, float b2,
@@ -322,104 +317,182 @@ struct AdamCoef {
     float bc2s, b1, b2, omb1, omb2, eps;
 };
 
-__device__ __forceinline__ AdamCoef adam_coef(const fgs_adam_args& a, int t)
+__device__ __noinline__ AdamCoef adam_coef(double beta1, double beta2, float eps, int t)
 {
     AdamCoef c;
-    c.bc1 = 1.0 - pow(a.beta1, (double)t);
-    c.bc2s = (float)sqrt(1.0 - pow(a.beta2, (double)t));
-    c.b1 = (float)a.beta1;
-    c.b2 = (float)a.beta2;
-    c.omb1 = (float)(1.0 - a.beta1);
-    c.omb2 = (float)(1.0 - a.beta2);
-    c.eps = a.eps;
+    c.bc1 = 1.0 - pow(beta1, (double)t);
+    c.bc2s = (float)sqrt(1.0 - pow(beta2, (double)t));
+    c.b1 = (float)beta1;
+    c.b2 = (float)beta2;
+    c.omb1 = (float)(1.0 - beta1);
+    c.omb2 = (float)(1.0 - beta2);
+    c.eps = eps;
     return c;
 }
 
-// The SH coefficients (as given) of the visible rows: one warp per row, lane k
-// updating coefficients k, k + 32, ... (coalesced), the visible test uniform over
-// the warp.
-__global__ void adam_sh_kernel(fgs_adam_args a, const uint8_t* __restrict__ flag, const int* __restrict__ step)
+// One Adam step of the visible rows, every parameter in one launch: a block takes 256
+// consecutive rows and lists the visible ones; blocks of blockIdx.y 0 update their SH
+// coefficients, of 1 the rest.  Bound by HBM traffic (per visible row 59 floats of value,
+// moments and gradient read and the first three written, 16 SH coefficients), so every
+// thread holds one item (16 bytes of an SH row, a float of a mean or a scale, a
+// quaternion) of the four arrays in flight, and a block issues its first loads before the
+// barrier behind which one thread forms the bias corrections: as double powers formed by
+// every thread they cost more than the traffic.  1M rows, 30% of them visible (506 MB):
+// 281 -> 114 us, at 40 to 64 resident warps per SM alike; a warp per row and a thread per row, as before, keep too little in
+// flight, and so did a warp per 32 rows with two items per lane (64 registers: 302 us).
+struct AdamShared {
+    AdamCoef c;
+    float ss[5];  // step sizes: means, SH, opacity, scale, rotation
+    uint32_t count[8];
+    uint8_t row[256];
+};
+
+__device__ __forceinline__ void adam_one(const AdamShared& sh, int which, float& p, float& m, float& v, float g)
 {
-    const AdamCoef c = adam_coef(a, *step);
-    const float ss = (float)(a.lr[1] / c.bc1);
-    const int F = 3 * a.M, lane = threadIdx.x & 31;
-    const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-    for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < a.P; i += nwarps) {
-        if (!flag[i]) continue;
-        for (int k = lane; k < F; k += 32) {
-            const size_t j = (size_t)F * i + k;
-            adam_update(a.shs[j], a.m_shs[j], a.v_shs[j], a.g_shs[j], c.b1, c.omb1, c.b2, c.omb2, ss, c.bc2s,
-                        c.eps);
-        }
+    adam_update(p, m, v, g, sh.c.b1, sh.c.omb1, sh.c.b2, sh.c.omb2, sh.ss[which], sh.c.bc2s, sh.c.eps);
+}
+
+// kW floats, in one access when the array is aligned for it.
+template <int kW>
+__device__ __forceinline__ void load_w(const float* __restrict__ p, bool vec, float (&o)[kW])
+{
+    if (kW == 4 && vec) {
+        const float4 q = *reinterpret_cast<const float4*>(p);
+        o[0] = q.x; o[kW > 1 ? 1 : 0] = q.y; o[kW > 2 ? 2 : 0] = q.z; o[kW > 3 ? 3 : 0] = q.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < kW; k++) o[k] = p[k];
+    }
+}
+template <int kW>
+__device__ __forceinline__ void store_w(float* __restrict__ p, bool vec, const float (&o)[kW])
+{
+    if (kW == 4 && vec) {
+        *reinterpret_cast<float4*>(p) = make_float4(o[0], o[kW > 1 ? 1 : 0], o[kW > 2 ? 2 : 0], o[kW > 3 ? 3 : 0]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kW; k++) p[k] = o[k];
     }
 }
 
-// Everything but the SH coefficients, one thread per row.
-__global__ void adam_kernel(fgs_adam_args a, const uint8_t* __restrict__ flag, const int* __restrict__ step)
+// The SH rows, in items of kW floats; per: items per row, per_inv = ceil(2^32 / per).
+template <int kW>
+__device__ __forceinline__ void adam_sh_rows(const fgs_adam_args& a, AdamShared& sh, size_t i0, uint32_t visible,
+                                             uint32_t per, uint32_t per_inv)
 {
-    const AdamCoef c = adam_coef(a, *step);
-    const double bc1 = c.bc1;
-    const float bc2s = c.bc2s, b1 = c.b1, b2 = c.b2, omb1 = c.omb1, omb2 = c.omb2, eps = c.eps;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.P; i += gridDim.x * blockDim.x) {
-        if (!flag[i]) continue;
-        // means (as given)
-        {
-            const float ss = (float)(a.lr[0] / bc1);
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const size_t j = 3 * (size_t)i + k;
-                adam_update(a.xyz[j], a.m_xyz[j], a.v_xyz[j], a.g_xyz[j], b1, omb1, b2, omb2, ss, bc2s, eps);
-            }
+    const uint32_t n = visible * per;
+    float p[kW], m[kW], v[kW], g[kW];
+    bool ready = false;
+    for (uint32_t it0 = 0; it0 < n; it0 += 256) {
+        const uint32_t it = it0 + threadIdx.x;
+        const uint32_t r = __umulhi(it, per_inv), q = it - r * per;  // it / per
+        const size_t j = it < n ? ((i0 + sh.row[r]) * per + q) * kW : 0;
+        if (it < n) {
+            load_w<kW>(a.shs + j, true, p);
+            load_w<kW>(a.m_shs + j, true, m);
+            load_w<kW>(a.v_shs + j, true, v);
+            load_w<kW>(a.g_shs + j, true, g);
         }
-        // opacity: d/dlogit = d/dopacity * s (1 - s)
-        {
-            const float ss = (float)(a.lr[2] / bc1);
-            const float s = a.opac[i];
-            const float g = a.g_opac[i] * (s * (1.f - s));
-            adam_update(a.opac_logit[i], a.m_opac[i], a.v_opac[i], g, b1, omb1, b2, omb2, ss, bc2s, eps);
-            a.opac[i] = sigmoidf(a.opac_logit[i]);
-        }
-        // scale: d/dlog = d/dscale * scale
-        {
-            const float ss = (float)(a.lr[3] / bc1);
+        if (!ready) __syncthreads();  // the coefficients, while the first loads are in flight
+        ready = true;
+        if (it >= n) continue;
 #pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const size_t j = 3 * (size_t)i + k;
-                const float g = a.g_scale[j] * a.scale[j];
-                adam_update(a.log_scale[j], a.m_scale[j], a.v_scale[j], g, b1, omb1, b2, omb2, ss, bc2s, eps);
-                a.scale[j] = expf(a.log_scale[j]);
-            }
-        }
-        // rotation: d/dq = (d/dq_hat - q_hat (q_hat . d/dq_hat)) / |q|
-        {
-            const float ss = (float)(a.lr[4] / bc1);
-            float q[4], qh[4], gq[4];
-            float n2 = 0.f, dot = 0.f;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                q[k] = a.rot_raw[4 * (size_t)i + k];
-                n2 += q[k] * q[k];
-            }
-            const float n = fmaxf(sqrtf(n2), 1e-12f);
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                qh[k] = a.rot[4 * (size_t)i + k];
-                dot += qh[k] * a.g_rot[4 * (size_t)i + k];
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) gq[k] = (a.g_rot[4 * (size_t)i + k] - qh[k] * dot) / n;
-            float m2 = 0.f;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const size_t j = 4 * (size_t)i + k;
-                adam_update(a.rot_raw[j], a.m_rot[j], a.v_rot[j], gq[k], b1, omb1, b2, omb2, ss, bc2s, eps);
-                m2 += a.rot_raw[j] * a.rot_raw[j];
-            }
-            const float nn = fmaxf(sqrtf(m2), 1e-12f);
-#pragma unroll
-            for (int k = 0; k < 4; k++) a.rot[4 * (size_t)i + k] = a.rot_raw[4 * (size_t)i + k] / nn;
-        }
+        for (int k = 0; k < kW; k++) adam_one(sh, 1, p[k], m[k], v[k], g[k]);
+        store_w<kW>(a.shs + j, true, p);
+        store_w<kW>(a.m_shs + j, true, m);
+        store_w<kW>(a.v_shs + j, true, v);
     }
+}
+
+// Means and scales as single floats, opacities and quaternions by row.
+__device__ __forceinline__ void adam_small_rows(const fgs_adam_args& a, AdamShared& sh, size_t i0, uint32_t visible,
+                                                bool vec)
+{
+    const uint32_t n = 3 * visible;
+    bool ready = false;
+    for (uint32_t it0 = 0; it0 < n; it0 += 256) {
+        const uint32_t it = it0 + threadIdx.x, r = it / 3;
+        const size_t j = it < n ? 3 * (i0 + sh.row[r]) + (it - 3 * r) : 0;
+        float px, mx, vx, gx, ps, ms, vs, gs, sc;
+        if (it < n) {
+            px = a.xyz[j]; mx = a.m_xyz[j]; vx = a.v_xyz[j]; gx = a.g_xyz[j];
+            ps = a.log_scale[j]; ms = a.m_scale[j]; vs = a.v_scale[j]; gs = a.g_scale[j]; sc = a.scale[j];
+        }
+        if (!ready) __syncthreads();
+        ready = true;
+        if (it >= n) continue;
+        adam_one(sh, 0, px, mx, vx, gx);
+        a.xyz[j] = px; a.m_xyz[j] = mx; a.v_xyz[j] = vx;
+        // scale: d/dlog = d/dscale * scale
+        adam_one(sh, 3, ps, ms, vs, gs * sc);
+        a.log_scale[j] = ps; a.m_scale[j] = ms; a.v_scale[j] = vs;
+        a.scale[j] = expf(ps);
+    }
+    if (threadIdx.x >= visible) return;
+    const size_t i = i0 + sh.row[threadIdx.x];
+    float po = a.opac_logit[i], mo = a.m_opac[i], vo = a.v_opac[i];
+    const float go = a.g_opac[i], so = a.opac[i];
+    float q[4], qh[4], gh[4], mq[4], vq[4];
+    load_w<4>(a.rot_raw + 4 * i, vec, q);
+    load_w<4>(a.rot + 4 * i, vec, qh);
+    load_w<4>(a.g_rot + 4 * i, vec, gh);
+    load_w<4>(a.m_rot + 4 * i, vec, mq);
+    load_w<4>(a.v_rot + 4 * i, vec, vq);
+    // opacity: d/dlogit = d/dopacity * s (1 - s)
+    adam_one(sh, 2, po, mo, vo, go * (so * (1.f - so)));
+    a.opac_logit[i] = po; a.m_opac[i] = mo; a.v_opac[i] = vo;
+    a.opac[i] = sigmoidf(po);
+    // rotation: d/dq = (d/dq_hat - q_hat (q_hat . d/dq_hat)) / |q|
+    float n2 = 0.f, dot = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) n2 += q[k] * q[k];
+    const float norm = fmaxf(sqrtf(n2), 1e-12f);
+#pragma unroll
+    for (int k = 0; k < 4; k++) dot += qh[k] * gh[k];
+    float m2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        adam_one(sh, 4, q[k], mq[k], vq[k], (gh[k] - qh[k] * dot) / norm);
+        m2 += q[k] * q[k];
+    }
+    const float nn = fmaxf(sqrtf(m2), 1e-12f);
+#pragma unroll
+    for (int k = 0; k < 4; k++) qh[k] = q[k] / nn;
+    store_w<4>(a.rot_raw + 4 * i, vec, q);
+    store_w<4>(a.m_rot + 4 * i, vec, mq);
+    store_w<4>(a.v_rot + 4 * i, vec, vq);
+    store_w<4>(a.rot + 4 * i, vec, qh);
+}
+
+// vec_rot / vec_sh: the quaternions / SH rows of every array start on 16-byte boundaries
+// (vec_sh: an item is four floats, else one).
+__global__ void __launch_bounds__(256)
+    adam_kernel(fgs_adam_args a, const uint8_t* __restrict__ flag, const int* __restrict__ step, bool vec_rot,
+                bool vec_sh, uint32_t per, uint32_t per_inv)
+{
+    __shared__ AdamShared sh;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t i0 = (size_t)blockIdx.x * 256, i = i0 + threadIdx.x;
+    const bool on = i < (size_t)a.P && flag[i] != 0;
+    const uint32_t mask = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) sh.count[warp] = __popc(mask);
+    __syncthreads();
+    uint32_t before = 0, visible = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        if (w < warp) before += sh.count[w];
+        visible += sh.count[w];
+    }
+    if (visible == 0) return;
+    if (on) sh.row[before + __popc(mask & ((1u << lane) - 1u))] = (uint8_t)threadIdx.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sh.c = adam_coef(a.beta1, a.beta2, a.eps, *step);
+        for (int k = 0; k < 5; k++) sh.ss[k] = (float)(a.lr[k] / sh.c.bc1);
+    }
+    if (blockIdx.y == 1) adam_small_rows(a, sh, i0, visible, vec_rot);
+    else if (vec_sh) adam_sh_rows<4>(a, sh, i0, visible, per, per_inv);
+    else adam_sh_rows<1>(a, sh, i0, visible, per, per_inv);
 }
 
 __global__ void step_tick_kernel(int* step) { *step += 1; }
@@ -504,12 +577,20 @@ int fgs_adam_step(const fgs_adam_args* a, const unsigned char* flag, int* step, 
     step_tick_kernel<<<1, 1, 0, s>>>(step);
     int n = 1;
     if (a->P > 0) {
-        adam_kernel<<<(a->P + 255) / 256 < 4096 ? (a->P + 255) / 256 : 4096, 256, 0, s>>>(*a, flag, step);
+        auto al = [](std::initializer_list<const void*> ps) {
+            for (const void* p : ps)
+                if (reinterpret_cast<uintptr_t>(p) & 15u) return false;
+            return true;
+        };
+        const bool vec_rot = al({a->rot_raw, a->rot, a->g_rot, a->m_rot, a->v_rot});
+        const uint32_t floats = a->shs ? 3u * (uint32_t)a->M : 0u;
+        const bool vec_sh = floats % 4 == 0 && al({a->shs, a->m_shs, a->v_shs, a->g_shs});
+        const uint32_t per = vec_sh ? floats / 4 : floats;
+        const uint32_t per_inv = per ? (uint32_t)((0x100000000ull + per - 1) / per) : 0u;  // per is 0 or at least 3
+        // (without SH rows the blocks of y = 0 would have nothing to do: y = 1 alone cannot be
+        // launched, so they leave after the list)
+        adam_kernel<<<dim3(((uint32_t)a->P + 255) / 256, 2), 256, 0, s>>>(*a, flag, step, vec_rot, vec_sh, per, per_inv);
         n++;
-        if (a->shs && a->M > 0) {
-            adam_sh_kernel<<<(a->P + 7) / 8 < 4096 ? (a->P + 7) / 8 : 4096, 256, 0, s>>>(*a, flag, step);
-            n++;
-        }
     }
     note_launches(n);
     return cudaGetLastError() == cudaSuccess ? FGS_OK : FGS_ERR_CUDA;
