@@ -472,6 +472,49 @@ __device__ __forceinline__ uint32_t auto_split_min(const unsigned long long* tot
     return K <= 2 * V ? 256u : max(1024u, (uint32_t)(min(K, 1ull << 30) / 592));
 }
 
+// ---------------------------------------------------------------- two floats per instruction
+// A pair of float32 in one 64-bit register; each half of an operation is rounded to
+// nearest as the scalar operation is.
+typedef unsigned long long F2;
+
+__device__ __forceinline__ F2 f2(float lo, float hi)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float v) { return f2(v, v); }
+__device__ __forceinline__ float f2_lo(F2 v)
+{
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return a;
+}
+__device__ __forceinline__ float f2_hi(F2 v)
+{
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return b;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 // ---------------------------------------------------------------- warp helpers
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31; }
 
