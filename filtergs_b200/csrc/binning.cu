@@ -171,8 +171,8 @@ __global__ void __launch_bounds__(kSortThreads, 4)
             if (rec_out) {
                 // The record also carries the pair's emission index: the Gaussian's first
                 // pair plus this tile's row-major place in its tile rectangle (the order in
-                // which duplicate_kernel emitted them), from the row base and width that
-                // duplicate_kernel left per Gaussian.  The backward writes the pair's
+                // which emit_pairs_kernel emitted them), from the row base and width that
+                // pair_offsets_kernel left per Gaussian.  The backward writes the pair's
                 // gradients there, so each Gaussian's pairs are contiguous and are summed
                 // in a fixed order.
                 PairRecord r = grec[v];
@@ -207,99 +207,157 @@ __global__ void depth_hist_kernel(const uint32_t* __restrict__ keys, uint32_t n,
     }
 }
 
-// duplicateWithKeys over the depth-ordered Gaussians, with the prefix sum of
-// tiles_touched fused in (decoupled look-back over 256-Gaussian chunks, taken
-// by persistent CTAs; the tile histograms leave each CTA once) and
-// warp-aggregated pair emission: the pairs of a warp's 32 Gaussians are
-// spread evenly over its lanes, so a large splat does not serialise on one
-// thread.  Also builds the per-pass tile digit histograms for the tile sort.
+// duplicateWithKeys over the depth-ordered Gaussians, in two kernels.
+//
+// pair_offsets_kernel: the prefix sum of tiles_touched in depth order (decoupled look-back
+// over chunks of 2048 Gaussians, eight per thread), and per depth rank j the tile rectangle
+// its pairs walk: off[j] the first pair, corner[j] the rectangle's first tile, w[j] its
+// width; per Gaussian the emission row for the sort's gather.
+//
+// emit_pairs_kernel: the pairs themselves, kEmitPairs consecutive ones per block whatever
+// Gaussians they belong to.  A block finds its first and last Gaussian by a 32-way search of
+// off[], holds their offsets in shared memory and every pair finds its Gaussian there by
+// bisection.  In depth order the near Gaussians come first and cover hundreds of tiles
+// each, so blocks that took a fixed number of Gaussians (one kernel with the prefix sum)
+// left the SMs idle three quarters of the time behind the first few: 2.09M pairs of 130K
+// Gaussians 128 us -> 16 + 19.  Also builds the tile digit histograms of the tile sort.
+constexpr int kOffItems = 8;
+constexpr uint32_t kOffChunk = 256u * kOffItems;
+constexpr uint32_t kEmitPairs = 2048;
+
 __global__ void __launch_bounds__(256)
-    duplicate_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ tiles,
-                     const PairRecord* __restrict__ grec, const int* __restrict__ radii, uint32_t V, int gx,
-                     int gy, uint32_t* __restrict__ tile_out, uint32_t* __restrict__ val_out, uint32_t K,
-                     uint32_t* status, uint32_t* chunk_counter, uint32_t* __restrict__ tile_hist, int tile_passes,
-                     const unsigned long long* __restrict__ V_dev, uint32_t* __restrict__ pair_off,
-                     int2* __restrict__ erow, unsigned* err)
+    pair_offsets_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ tiles,
+                        const PairRecord* __restrict__ grec, const int* __restrict__ radii, uint32_t V, int gx,
+                        int gy, uint32_t* status, uint32_t* chunk_counter,
+                        const unsigned long long* __restrict__ V_dev, uint32_t* __restrict__ off,
+                        uint32_t* __restrict__ corner, uint32_t* __restrict__ w, int2* __restrict__ erow, unsigned* err)
 {
-    __shared__ uint32_t s_hist[4][kRadix];
+    __shared__ uint32_t s_cnt[kOffChunk];  // counts, then exclusive prefixes within the chunk
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_chunk, s_prefix;
-    const int tid = threadIdx.x, lane = tid & 31;
-    // persistent over chunks of 256 Gaussians (the grid covers a bound on V)
+    const int tid = threadIdx.x;
     V = (uint32_t)min((unsigned long long)V, *V_dev);
-    const uint32_t live = (V + 255) / 256;
+    const uint32_t live = (V + kOffChunk - 1) / kOffChunk;
     if (blockIdx.x >= live) return;
-    for (int i = tid; i < 4 * kRadix; i += 256) (&s_hist[0][0])[i] = 0;
     for (;;) {
         if (tid == 0) s_chunk = atomicAdd(chunk_counter, 1u);
         __syncthreads();
         const uint32_t chunk = s_chunk;
         if (chunk >= live) break;
-        const uint32_t j = chunk * 256 + tid;
-        uint32_t id = 0, cnt = 0;
-        int x0 = 0, y0 = 0, w = 1;
-        if (j < V) {
-            id = __ldg(sorted_ids + j);
-            cnt = __ldg(tiles + id);
-            const float4 a = grec[id].a;
-            int x1, y1;
-            tile_rect(a.x, a.y, __ldg(radii + id), gx, gy, kTileX, kTileY, x0, y0, x1, y1);
-            w = max(1, x1 - x0);
+        const uint32_t base = chunk * kOffChunk;
+        uint32_t id[kOffItems];
+#pragma unroll
+        for (int i = 0; i < kOffItems; i++) {
+            const uint32_t j = base + i * 256 + tid;
+            id[i] = j < V ? __ldg(sorted_ids + j) : 0xffffffffu;
         }
-        uint32_t block_total;
-        const uint32_t local = block_excl_scan(cnt, s_warp, &block_total);
+#pragma unroll
+        for (int i = 0; i < kOffItems; i++) s_cnt[i * 256 + tid] = id[i] != 0xffffffffu ? __ldg(tiles + id[i]) : 0u;
+        __syncthreads();
+        uint32_t c[kOffItems], sum = 0;
+#pragma unroll
+        for (int i = 0; i < kOffItems; i++) {
+            c[i] = s_cnt[tid * kOffItems + i];
+            sum += c[i];
+        }
+        uint32_t total;
+        uint32_t at = block_excl_scan(sum, s_warp, &total);
+#pragma unroll
+        for (int i = 0; i < kOffItems; i++) {
+            s_cnt[tid * kOffItems + i] = at;
+            at += c[i];
+        }
         if (tid < 32) {
-            const uint32_t e = warp_lookback(status, chunk, 1, block_total, err);
+            const uint32_t e = warp_lookback(status, chunk, 1, total, err);
             if (tid == 0) s_prefix = e;
         }
         __syncthreads();
-        const uint32_t off = s_prefix + local;
-        if (cnt) {
-            // first emitted pair (by depth rank j: Gaussian j's pairs are
-            // [pair_off[j], pair_off[j + 1])), and the emission index of tile
-            // (tx, ty) as erow.x + ty * erow.y + tx (unsigned wrap-around)
-            pair_off[j] = off;
-            erow[id] = make_int2((int)(off - (uint32_t)y0 * (uint32_t)w - (uint32_t)x0), w);
-        }
-        // warp-local exclusive prefix of cnt
-        uint32_t wx = cnt;
+        const uint32_t prefix = s_prefix;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, wx, o);
-            if (lane >= o) wx += y;
+        for (int i = 0; i < kOffItems; i++) {
+            if (id[i] == 0xffffffffu) continue;
+            const uint32_t j = base + i * 256 + tid;
+            const float2 m = *reinterpret_cast<const float2*>(&grec[id[i]].a);
+            int x0, y0, x1, y1;
+            tile_rect(m.x, m.y, __ldg(radii + id[i]), gx, gy, kTileX, kTileY, x0, y0, x1, y1);
+            const uint32_t o = prefix + s_cnt[i * 256 + tid], wd = (uint32_t)max(1, x1 - x0);
+            // Gaussian j's pairs are [off[j], off[j + 1]); the emission index of tile (tx, ty) is
+            // erow.x + ty * erow.y + tx (unsigned wrap-around)
+            off[j] = o;
+            corner[j] = (uint32_t)y0 * (uint32_t)gx + (uint32_t)x0;
+            w[j] = wd;
+            erow[id[i]] = make_int2((int)(o - (uint32_t)y0 * wd - (uint32_t)x0), (int)wd);
         }
-        const uint32_t wtotal = __shfl_sync(0xffffffffu, wx, 31);
-        wx -= cnt;  // exclusive
-        for (uint32_t pb = 0; pb < wtotal; pb += 32) {
-            const uint32_t p = pb + lane;
-            // owner lane: last lane g with wx[g] <= p (lanes with no pairs never win)
-            int lo = 0;
+        __syncthreads();  // the shared arrays are reused by the next chunk
+    }
+}
+
+// Last rank j < V with off[j] <= p (off[0] = 0), by one warp: 32 probes per step.
+__device__ __forceinline__ uint32_t rank_of_pair(const uint32_t* __restrict__ off, uint32_t V, uint32_t p)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, n = V;  // the answer lies in [lo, lo + n)
+    while (n > 1) {
+        const uint32_t step = (n + 31) / 32, at = lane * step;
+        const bool le = at < n && __ldg(off + lo + at) <= p;  // monotone over the lanes; lane 0 holds
+        const uint32_t k = (uint32_t)(31 - __clz(__ballot_sync(0xffffffffu, le)));
+        lo += k * step;
+        n = min(step, n - k * step);
+    }
+    return lo;
+}
+
+// (Offsets that a look-back which ran out of time left inconsistent keep every index inside
+// its array: ranks below V, at most kEmitPairs of them, tiles below num_tiles.)
+__global__ void __launch_bounds__(256)
+    emit_pairs_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ off,
+                      const uint32_t* __restrict__ corner, const uint32_t* __restrict__ w, uint32_t V, uint32_t K, int gx,
+                      uint32_t num_tiles, const unsigned long long* __restrict__ totals, uint32_t* __restrict__ tile_out,
+                      uint32_t* __restrict__ val_out, uint32_t* __restrict__ tile_hist, int tile_passes, unsigned* err)
+{
+    __shared__ uint32_t s_hist[4][kRadix];
+    __shared__ uint32_t s_off[kEmitPairs];
+    __shared__ uint32_t s_j[2];
+    const int tid = threadIdx.x;
+    V = (uint32_t)min((unsigned long long)V, totals[1]);
+    if (totals[0] > K && blockIdx.x == 0 && tid == 0) set_error(err, FGS_ERR_OVERFLOW);  // truncated at the capacity
+    K = (uint32_t)min((unsigned long long)K, totals[0]);
+    const uint32_t chunks = (K + kEmitPairs - 1) / kEmitPairs;
+    if (V == 0 || blockIdx.x >= chunks) return;
+    for (int i = tid; i < tile_passes * kRadix; i += 256) (&s_hist[0][0])[i] = 0;
+    for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
+        const uint32_t p0 = chunk * kEmitPairs, p1 = min(K, p0 + kEmitPairs);
+        if (tid < 64) {
+            const uint32_t j = rank_of_pair(off, V, tid < 32 ? p0 : p1 - 1);
+            if ((tid & 31) == 0) s_j[tid >> 5] = j;
+        }
+        __syncthreads();
+        const uint32_t j0 = s_j[0];
+        const uint32_t nj = s_j[1] < j0 ? 1u : min(s_j[1] - j0 + 1, kEmitPairs);  // at most one Gaussian per pair
+        for (uint32_t i = tid; i < nj; i += 256) s_off[i] = __ldg(off + j0 + i);
+        __syncthreads();
 #pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-                const int probe = lo + step;
-                const uint32_t e = __shfl_sync(0xffffffffu, wx, probe);
-                if (e <= p) lo = probe;
+        for (uint32_t i = 0; i < kEmitPairs / 256; i++) {
+            const uint32_t p = p0 + i * 256 + tid;
+            if (p >= p1) break;
+            uint32_t lo = 0, hi = nj;  // last entry with s_off <= p lies in [lo, hi)
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (s_off[mid] <= p) lo = mid;
+                else hi = mid;
             }
-            const uint32_t owx = __shfl_sync(0xffffffffu, wx, lo);
-            const uint32_t ooff = __shfl_sync(0xffffffffu, off, lo);
-            const uint32_t oid = __shfl_sync(0xffffffffu, id, lo);
-            const int ox0 = __shfl_sync(0xffffffffu, x0, lo);
-            const int oy0 = __shfl_sync(0xffffffffu, y0, lo);
-            const int ow = __shfl_sync(0xffffffffu, w, lo);
-            if (p < wtotal) {
-                const uint32_t t = p - owx;
-                if (ooff + t >= K) {  // K and tiles_touched come from the same kernel; guard anyway
-                    set_error(err, FGS_ERR_OVERFLOW);
-                    continue;
-                }
-                const uint32_t ty = t / (uint32_t)ow, tx = t - ty * (uint32_t)ow;
-                const uint32_t tile = (uint32_t)(oy0 + ty) * (uint32_t)gx + (uint32_t)(ox0 + tx);
-                tile_out[ooff + t] = tile;
-                val_out[ooff + t] = oid;
-                for (int b = 0; b < tile_passes; b++) atomicAdd(&s_hist[b][(tile >> (8 * b)) & 255u], 1u);
+            const uint32_t j = j0 + lo, t = p - s_off[lo], wd = __ldg(w + j), c = __ldg(corner + j);
+            const uint32_t ty = t / wd, tx = t - ty * wd;
+            uint32_t tile = c + ty * (uint32_t)gx + tx;
+            if (tile >= num_tiles) {
+                set_error(err, FGS_ERR_OVERFLOW);
+                tile = num_tiles - 1;
             }
+            tile_out[p] = tile;
+            val_out[p] = __ldg(sorted_ids + j);
+            for (int b = 0; b < tile_passes; b++) atomicAdd(&s_hist[b][(tile >> (8 * b)) & 255u], 1u);
         }
-        __syncthreads();  // s_chunk / s_prefix / s_warp are reused by the next chunk
+        __syncthreads();  // s_j and s_off are rewritten for the next chunk
     }
     for (int i = tid; i < tile_passes * kRadix; i += 256) {
         const uint32_t c = (&s_hist[0][0])[i];
@@ -417,11 +475,15 @@ void launch_duplicate(const GeomState& g, const BinState& b, uint32_t V, uint32_
     // with an odd number of passes it starts from a, with an even one from b.
     uint32_t* tout = (passes & 1) ? b.tile_a : b.tile_b;
     uint32_t* vout = (passes & 1) ? b.val_a : b.val_b;
-    const uint32_t grid = min(chunks_of(V, 256), resident_ctas(duplicate_kernel, 256));
-    duplicate_kernel<<<grid, 256, 0, s>>>(g.sort_ids_b, g.tiles, g.grec, g.radii, V, gx, gy, tout,
-                                                       vout, K, b.scan_status, g.counters + 8, g.hist + 4 * kRadix,
-                                                       passes, g.total + 1, g.pair_off, g.erow, g.err);
-    note_launches(1);
+    // the depth keys and the other id buffer are free once the Gaussians are sorted
+    uint32_t *corner = g.depth_key, *w = g.sort_ids_a;
+    const uint32_t grid = min(chunks_of(V, kOffChunk), resident_ctas(pair_offsets_kernel, 256));
+    pair_offsets_kernel<<<grid, 256, 0, s>>>(g.sort_ids_b, g.tiles, g.grec, g.radii, V, gx, gy, b.scan_status,
+                                             g.counters + 8, g.total + 1, g.pair_off, corner, w, g.erow, g.err);
+    const uint32_t egrid = min(chunks_of(K, kEmitPairs), resident_ctas(emit_pairs_kernel, 256));
+    emit_pairs_kernel<<<egrid, 256, 0, s>>>(g.sort_ids_b, g.pair_off, corner, w, V, K, gx, (uint32_t)(gx * gy), g.total,
+                                            tout, vout, g.hist + 4 * kRadix, passes, g.err);
+    note_launches(2);
 }
 
 void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int tile_bits, int W, int H, cudaStream_t s,
