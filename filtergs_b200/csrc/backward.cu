@@ -652,7 +652,20 @@ void fold_launch(const FoldView* views, const FoldView& single, int nviews, int 
     note_launches(sh ? 3 : 1);
 }
 
+// One launch instead of a memset per buffer: a launch costs about 2 us of a small view's chain
+// each, and a large buffer is written at the memory's rate either way.
+__global__ void __launch_bounds__(256) zero_kernel(ZeroList z) { zero_share(z, blockIdx.x, gridDim.x); }
+
 }  // namespace
+
+void launch_zero(const ZeroList& z, cudaStream_t s)
+{
+    size_t words = 0;
+    for (int b = 0; b < z.n; b++) words += z.words[b];
+    if (!words) return;
+    zero_kernel<<<grid_for(words / 4 + 1, 8), 256, 0, s>>>(z);
+    note_launches(1);
+}
 
 void launch_preprocess_bwd(const PreParams& p, const GeomState& g, const float* pgrad, float* dmean2D,
                            float* dconic, float* dcolor, float* dopac, float* dmean3D, float* dcov3D, float* dsh,
@@ -666,16 +679,9 @@ void launch_preprocess_bwd(const PreParams& p, const GeomState& g, const float* 
     note_launches(1);
     // the list: the view's visible Gaussians (depth order); the view's geometric
     // dL/dmean3D waits in the dL/dmean3D rows for the SH pass.  dL/dopacity is the
-    // gather's output, read and rewritten in place (rows outside the list were
-    // zeroed by the caller).
-    const size_t P = (size_t)p.P;
-    cudaMemsetAsync(dmean3D, 0, sizeof(float) * 3 * P, s);
-    cudaMemsetAsync(dcov3D, 0, sizeof(float) * 6 * P, s);
-    if (sh) cudaMemsetAsync(dsh, 0, sizeof(float) * 3 * (size_t)p.M * P, s);
-    if (dscale) cudaMemsetAsync(dscale, 0, sizeof(float) * 3 * P, s);
-    if (drot) cudaMemsetAsync(drot, 0, sizeof(float) * 4 * P, s);
+    // gather's output, read and rewritten in place (the caller zeroed all output rows).
     const FoldView one{p, dmean3D, dmean2D, dconic, dopac, dcolor, g.clamped};
-    fold_launch(nullptr, one, 1, p.P, g.sort_ids_b, g.total + 1, P, nullptr, consistent, sh, dmean3D, dopac, dcov3D,
+    fold_launch(nullptr, one, 1, p.P, g.sort_ids_b, g.total + 1, (size_t)p.P, nullptr, consistent, sh, dmean3D, dopac, dcov3D,
                 dsh, dscale, drot, nullptr, s);
 }
 

@@ -345,7 +345,7 @@ int fgs_batch_forward(void* handle, void* stream)
     }
     const RenderConfig rc = get_render_config();
     uint32_t* long_ctr = B->d_long + 32 * (size_t)B->total_tiles;
-    if (rc.rule_long()) cudaMemsetAsync(long_ctr, 0, 34 * sizeof(uint32_t), s);  // the views' ranges add to it
+    if (rc.rule_long()) cudaMemsetAsync(long_ctr, 0, kLongCtrBytes, s);  // the views' ranges add to it
     if (cudaEventRecord(B->forked, s) != cudaSuccess) return FGS_ERR_CUDA;
     for (int i = 0; i < ns; i++) cudaStreamWaitEvent(B->aux[i], B->forked, 0);
     for (int vi = 0; vi < B->V; vi++) {
@@ -412,11 +412,13 @@ int fgs_batch_backward(void* handle, void* stream)
     // the shared outputs are zeroed while the gathers run (the fold writes the rows of
     // the Gaussians some view saw)
     const bool sh = B->views[0].pre.shs && B->g_sh;
-    cudaMemsetAsync(B->g_means3D, 0, sizeof(float) * 3 * P, s);
-    cudaMemsetAsync(B->g_opacity, 0, sizeof(float) * P, s);
-    if (sh) cudaMemsetAsync(B->g_sh, 0, sizeof(float) * 3 * (size_t)B->M * P, s);
-    if (B->has_sr && B->g_scales) cudaMemsetAsync(B->g_scales, 0, sizeof(float) * 3 * P, s);
-    if (B->has_sr && B->g_rot) cudaMemsetAsync(B->g_rot, 0, sizeof(float) * 4 * P, s);
+    ZeroList zero;
+    zero.add(B->g_means3D, sizeof(float) * 3 * P);
+    zero.add(B->g_opacity, sizeof(float) * P);
+    if (sh) zero.add(B->g_sh, sizeof(float) * 3 * (size_t)B->M * P);
+    if (B->has_sr) zero.add(B->g_scales, sizeof(float) * 3 * P);
+    if (B->has_sr) zero.add(B->g_rot, sizeof(float) * 4 * P);
+    launch_zero(zero, s);
     for (int vi = 0; vi < B->V; vi++) {
         ViewState& v = B->views[vi];
         launch_pair_grad_gather(v.g, v.b.pgrad, v.cap, v.dmean2D, v.dconic, v.dcolor, v.dopac,

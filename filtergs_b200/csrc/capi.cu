@@ -1,5 +1,6 @@
 // extern "C" entry points (include/filtergs_b200.h): argument checks,
 // workspace carving, kernel sequencing on the caller's stream.
+#include <algorithm>
 #include <atomic>
 #include <cerrno>
 #include <cstdlib>
@@ -95,12 +96,13 @@ BinCarve carve_bin(void* base, long long K, int P, bool with_grad = true)
 
 // Device errors recorded after a launch are read back lazily through this
 // pinned word (checked at the next synchronisation point on the host).
+constexpr size_t kPinnedTotals = 64, kPinnedBytes = 64 + 2 * kAlign;  // error words; totals .. error word of a view
 unsigned int* pinned_words()
 {
     static unsigned int* w = nullptr;
     if (!w) {
-        if (cudaHostAlloc(reinterpret_cast<void**>(&w), 64, cudaHostAllocDefault) != cudaSuccess) w = nullptr;
-        if (w) memset(w, 0, 64);
+        if (cudaHostAlloc(reinterpret_cast<void**>(&w), kPinnedBytes, cudaHostAllocDefault) != cudaSuccess) w = nullptr;
+        if (w) memset(w, 0, kPinnedBytes);
     }
     return w;
 }
@@ -178,13 +180,12 @@ int make_params(const fgs_raster_args* a, PreParams& p, bool backward)
     return FGS_OK;
 }
 
-// The launch rule's long-tile list of one view (counters zeroed here), or none when the caller set
-// a shape or a split.
+// The launch rule's long-tile list of one view (the caller zeroes the counters), or none when the
+// user set a shape or a split.
 LongList long_list_of(const RenderConfig& c, const ImageState& im, int num_tiles, const unsigned long long* totals,
-                      const BinState* stats, cudaStream_t s)
+                      const BinState* stats)
 {
     if (!c.rule_long()) return LongList{};
-    cudaMemsetAsync(im.long_ctr, 0, 34 * sizeof(uint32_t), s);
     return LongList{im.long_list, im.long_ctr, (uint32_t)num_tiles, 0u, totals, stats ? stats->kv_sum : nullptr,
                     stats ? stats->kv_cnt : nullptr};
 }
@@ -376,14 +377,6 @@ int fgs_forward_preprocess(const fgs_raster_args* a, void* geom, void* image, in
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     unsigned int* pin = pinned_words();
     if (!pin) return FGS_ERR_CUDA;
-    // an error recorded by an earlier call on this stream surfaces now
-    st = cuda_status(cudaStreamSynchronize(s));
-    if (st) return st;
-    if (pin[4]) {
-        const int prev = err_code_from_bits(pin[4]);
-        pin[4] = 0;
-        return prev;
-    }
     GeomCarve gc = carve_geom(geom, p.P);
     cudaMemsetAsync(gc.zero_begin, 0, gc.zero_bytes, s);
     {
@@ -395,12 +388,23 @@ int fgs_forward_preprocess(const fgs_raster_args* a, void* geom, void* image, in
         launch_depth_sort(gc.g, p.P, s);
     }
     if ((st = check_launch())) return st;
-    unsigned long long* tot = reinterpret_cast<unsigned long long*>(pin + 8);
-    cudaMemcpyAsync(tot, gc.g.total, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(pin, gc.g.err, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+    // totals and error word in one copy (one follows the other in the workspace)
+    char* back = reinterpret_cast<char*>(pin) + kPinnedTotals;
+    const size_t err_off = (size_t)(reinterpret_cast<char*>(gc.g.err) - reinterpret_cast<char*>(gc.g.total));
+    cudaMemcpyAsync(back, gc.g.total, err_off + sizeof(unsigned), cudaMemcpyDeviceToHost, s);
     st = cuda_status(cudaStreamSynchronize(s));
     if (st) return st;
-    if (pin[0]) return err_code_from_bits(pin[0]);
+    // an error recorded by an earlier call on this stream surfaces now (its copy precedes this
+    // call's work on the stream: waiting for it first kept this call's kernels from being queued
+    // behind the earlier call's)
+    if (pin[4]) {
+        const int prev = err_code_from_bits(pin[4]);
+        pin[4] = 0;
+        return prev;
+    }
+    const unsigned long long* tot = reinterpret_cast<const unsigned long long*>(back);
+    const unsigned err_bits = *reinterpret_cast<const unsigned*>(back + err_off);
+    if (err_bits) return err_code_from_bits(err_bits);
     if (tot[0] >= (1ull << 30)) return FGS_ERR_OVERFLOW;
     *num_rendered = (long long)tot[0];
     return FGS_OK;
@@ -429,9 +433,12 @@ int fgs_forward_render(const fgs_raster_args* a, void* geom, void* image, void* 
     const RenderConfig rc = get_render_config();
     const bool stats = a->ogfs_enable_stats != 0;
     if (stats && stats_host && stats_len < 9 + 2 * FGS_STATS_SLOTS) return FGS_ERR_ARG;
-    if (p.P > 0) cudaMemsetAsync(out_point_weight, 0, sizeof(float) * (size_t)p.P, s);
+    ZeroList zero;
+    zero.add(out_point_weight, sizeof(float) * (size_t)p.P);
+    if (K > 0) zero.add(bc.b.status, sizeof(uint32_t) * (bc.b.status_words + bc.b.scan_words));
+    if (rc.rule_long()) zero.add(im.long_ctr, kLongCtrBytes);
+    launch_zero(zero, s);
     if (K > 0) {
-        cudaMemsetAsync(bc.b.status, 0, sizeof(uint32_t) * (bc.b.status_words + bc.b.scan_words), s);
         // V lives on the device (g.total[1]); every Gaussian beyond it has no pairs.
         {
             StageTimer t(FGS_STAGE_DUPLICATE, s);
@@ -442,7 +449,7 @@ int fgs_forward_render(const fgs_raster_args* a, void* geom, void* image, void* 
     }
     {
         StageTimer t(FGS_STAGE_RANGES, s);
-        launch_ranges(bc.b, im, K, num_tiles, s, nullptr, long_list_of(rc, im, num_tiles, g.total, stats ? &bc.b : nullptr, s));
+        launch_ranges(bc.b, im, K, num_tiles, s, nullptr, long_list_of(rc, im, num_tiles, g.total, stats ? &bc.b : nullptr));
     }
     {
         StageTimer t_render(FGS_STAGE_RENDER_FWD, s);
@@ -454,50 +461,38 @@ int fgs_forward_render(const fgs_raster_args* a, void* geom, void* image, void* 
     if (stats && stats_host) {
         // rasterize_points.cu:138-177
         const int slots = FGS_STATS_SLOTS;
-        const bool tiles_out = K > 0;
-        const int need = 9 + 2 * slots + (tiles_out ? 2 * num_tiles : 0);
+        const int need = 9 + 2 * slots + (K > 0 ? 2 * num_tiles : 0);
         if (stats_len < need) return FGS_ERR_ARG;
-        double* dev = nullptr;
-        const size_t nd = 3 + 11 + 2 * (size_t)num_tiles;
+        for (int i = 0; i < stats_len; i++) stats_host[i] = 0.0;
         if (K > 0) {
-            // device scratch for the statistics: the tail of the pair-record buffer is free
-            // only when it is large enough; otherwise use a temporary allocation.
-            if (cudaMallocAsync(reinterpret_cast<void**>(&dev), nd * sizeof(double), s) != cudaSuccess) return FGS_ERR_CUDA;
-            StageTimer t(FGS_STAGE_STATS, s);
-            launch_kpc_stats(bc.b, im, num_tiles, kpc_used_thresh(), dev, s);
-        }
-        double* host = static_cast<double*>(std::malloc(nd * sizeof(double)));
-        if (!host) return FGS_ERR_CUDA;
-        memset(host, 0, nd * sizeof(double));
-        if (K > 0) {
-            cudaMemcpyAsync(host, dev, nd * sizeof(double), cudaMemcpyDeviceToHost, s);
-            cudaFreeAsync(dev, s);
+            // in the long-tile bins, dead once the tiles are rendered (128 bytes per tile; the statistics
+            // take 16 per tile and 1096): an allocation here was given back to the driver at every
+            // synchronisation and cost more than the rest of a small view
+            double* dev = reinterpret_cast<double*>(im.long_list);
+            if (sizeof(double) * (size_t)need > 32 * sizeof(uint32_t) * (size_t)num_tiles) {
+                // fewer than ten tiles: the sort's status words (a chunk's worth at least: 4 KB)
+                dev = reinterpret_cast<double*>(bc.b.status);
+            }
+            {
+                StageTimer t(FGS_STAGE_STATS, s);
+                launch_kpc_stats(bc.b, im, num_tiles, kpc_used_thresh(), dev, need, s);
+            }
+            cudaMemcpyAsync(stats_host, dev, sizeof(double) * (size_t)need, cudaMemcpyDeviceToHost, s);
         }
         cudaMemcpyAsync(pin, g.err, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
         st = cuda_status(cudaStreamSynchronize(s));
-        if (st) { std::free(host); return st; }
-        for (int i = 0; i < stats_len; i++) stats_host[i] = 0.0;
-        stats_host[0] = K > 0 ? host[0] / (double)num_tiles : 0.0;
+        if (st) return st;
+        if (K > 0) stats_host[0] /= (double)num_tiles;
         stats_host[1] = p.P > 0 ? (double)K / (double)p.P : 0.0;
         stats_host[2] = num_tiles > 0 ? (double)K / (double)num_tiles : 0.0;
         stats_host[3] = (double)K;
         stats_host[4] = (double)num_tiles;
         stats_host[5] = (double)p.P;
-        stats_host[6] = K > 0 ? host[1] : 0.0;
-        stats_host[7] = K > 0 ? host[2] : 0.0;
         stats_host[8] = K > 0 ? 11.0 : 0.0;
         if (K > 0) {
             const double edges[11] = {0.01f, 0.05f, 0.10f, 0.15f, 0.20f, 0.25f, 0.30f, 0.35f, 0.40f, 0.45f, 0.50f};
-            for (int b = 0; b < 11; b++) {
-                stats_host[9 + b] = edges[b];
-                stats_host[9 + slots + b] = host[3 + b];
-            }
-            for (int t = 0; t < num_tiles; t++) {
-                stats_host[9 + 2 * slots + t] = host[14 + t];
-                stats_host[9 + 2 * slots + num_tiles + t] = host[14 + num_tiles + t];
-            }
+            for (int b = 0; b < 11; b++) stats_host[9 + b] = edges[b];
         }
-        std::free(host);
         if (pin[0]) return err_code_from_bits(pin[0]);
     } else if (stats_host) {
         for (int i = 0; i < stats_len; i++) stats_host[i] = 0.0;
@@ -533,19 +528,23 @@ int fgs_backward(const fgs_raster_args* a, const void* geom, const void* image, 
     ImageState im = image_views(const_cast<void*>(image), p.W, p.H);
     BinState b = bin_views(const_cast<void*>(binning), num_rendered, p.P);
     (void)radii;  // the forward's visible list (radii > 0) is in geom
-    cudaMemsetAsync(dL_dmeans2D, 0, sizeof(float) * 3 * (size_t)p.P, s);
-    cudaMemsetAsync(dL_dconic, 0, sizeof(float) * 4 * (size_t)p.P, s);
-    cudaMemsetAsync(dL_dopacity, 0, sizeof(float) * (size_t)p.P, s);
-    cudaMemsetAsync(dL_dcolors, 0, sizeof(float) * 3 * (size_t)p.P, s);
-    if (!p.scales) {
-        if (dL_dscales) cudaMemsetAsync(dL_dscales, 0, sizeof(float) * 3 * (size_t)p.P, s);
-        if (dL_drotations) cudaMemsetAsync(dL_drotations, 0, sizeof(float) * 4 * (size_t)p.P, s);
-    }
-    if (!p.shs && dL_dsh && a->M > 0) cudaMemsetAsync(dL_dsh, 0, sizeof(float) * 3 * (size_t)a->M * p.P, s);
+    // every gradient row starts at zero (the kernels write the visible Gaussians' rows only)
+    const size_t fP = sizeof(float) * (size_t)p.P;
+    ZeroList zero;
+    zero.add(dL_dmeans2D, 3 * fP);
+    zero.add(dL_dconic, 4 * fP);
+    zero.add(dL_dopacity, fP);
+    zero.add(dL_dcolors, 3 * fP);
+    zero.add(dL_dmeans3D, 3 * fP);
+    zero.add(dL_dcov3D, 6 * fP);
+    zero.add(dL_dsh, 3 * (size_t)std::max(a->M, 0) * fP);
+    zero.add(dL_dscales, 3 * fP);
+    zero.add(dL_drotations, 4 * fP);
+    if (num_rendered <= 0) launch_zero(zero, s);
     const int consistent = backward_mode == FGS_BACKWARD_CONSISTENT;
     if (num_rendered > 0) {
         StageTimer t(FGS_STAGE_RENDER_BWD, s);
-        launch_render_bwd(p.W, p.H, im, b, a->background, dL_dout_color, consistent, g.err, s);
+        launch_render_bwd(p.W, p.H, im, b, a->background, dL_dout_color, consistent, zero, g.err, s);
     }
     {
         StageTimer t_pb(FGS_STAGE_PREPROCESS_BWD, s);

@@ -114,6 +114,42 @@ int sort_chunk_size();
 // K is the pair count, or the capacity when n_dev (device-side count) is given.
 void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int tile_bits, int W, int H, cudaStream_t s,
                       const unsigned long long* n_dev = nullptr);
+// Buffers zeroed by one launch (whole 4-byte words from 4-byte boundaries).
+struct ZeroList {
+    static constexpr int kMax = 10;
+    void* p[kMax];
+    size_t words[kMax];
+    int n = 0;
+    void add(void* ptr, size_t bytes)
+    {
+        if (!ptr || bytes == 0) return;
+        p[n] = ptr;
+        words[n++] = bytes / 4;
+    }
+};
+void launch_zero(const ZeroList& z, cudaStream_t s);
+#ifdef __CUDACC__
+// Block `part` of `parts` zeroes its share of every buffer: a run of whole 16-byte items, and the first
+// and last blocks the words before the first 16-byte boundary and after the last.
+__device__ __forceinline__ void zero_share(const ZeroList& z, uint32_t part, uint32_t parts)
+{
+    for (int b = 0; b < z.n; b++) {
+        uint32_t* p = static_cast<uint32_t*>(z.p[b]);
+        const size_t n = z.words[b];
+        size_t head = ((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / 4;
+        if (head > n) head = n;
+        const size_t items = (n - head) / 4;
+        const size_t i1 = items * (part + 1) / parts;
+        uint4* q = reinterpret_cast<uint4*>(p + head);
+        for (size_t i = items * part / parts + threadIdx.x; i < i1; i += blockDim.x) q[i] = make_uint4(0, 0, 0, 0);
+        if (part == 0 && threadIdx.x < head) p[threadIdx.x] = 0;
+        const size_t tail = head + 4 * items;
+        if (part == parts - 1 && threadIdx.x < n - tail) p[tail + threadIdx.x] = 0;
+    }
+}
+#endif
+
+constexpr size_t kLongCtrBytes = 34 * sizeof(uint32_t);  // ImageState::long_ctr
 struct RenderConfig;
 // Where the tiles that the launch rule renders in bands are listed (render.cu): list [32][cap]
 // binned by log2(records), ctr [34] (zeroed by the caller) and the first id of this view's tiles.
@@ -134,8 +170,10 @@ void launch_ranges(const BinState& b, const ImageState& im, long long K, int num
 void launch_render_fwd(const RenderConfig& c, int W, int H, const ImageState& im, const BinState& b, long long K,
                        const unsigned long long* totals, const float* bg, float* out_color, int* point_id,
                        float* pw_pixel, float* point_weight, bool stats, unsigned* err, cudaStream_t s);
+// zero: buffers the launch also zeroes (the gradient outputs: 568 MB at 2M Gaussians with SH 3, whose
+// writing then costs next to nothing beside compositing that is bound by instruction issue).
 void launch_render_bwd(int W, int H, const ImageState& im, const BinState& b, const float* bg,
-                       const float* dL_dpix, int consistent, unsigned* err, cudaStream_t s);
+                       const float* dL_dpix, int consistent, const ZeroList& zero, unsigned* err, cudaStream_t s);
 // Densification statistics a training step keeps per Gaussian (null pointers: off).
 struct DensifyStats {
     float* grad_sum;   // += |dL/dmean2D[:2]| per view that sees the Gaussian
@@ -172,8 +210,10 @@ void launch_pair_grad_gather(const GeomState& g, const float* pgrad, long long r
 void launch_fold_bwd(const FoldView* views, int nviews, int P, const uint32_t* vis, uint32_t* list,
                      unsigned long long* count, int consistent, bool sh, float* dmean3D, float* dopac, float* dsh,
                      float* dscale, float* drot, const DensifyStats* dens, const FoldView& shared, cudaStream_t s);
+// dev_out: the statistics array of fgs_forward_render (`need` doubles, zeroed here): the sum over tiles in [0],
+// used and unused pairs in [6] and [7], the KPC histogram, the tiles' used ratios and pair counts.
 void launch_kpc_stats(const BinState& b, const ImageState& im, int num_tiles, float used_thresh, double* dev_out,
-                      cudaStream_t s);
+                      int need, cudaStream_t s);
 
 // radius / visibility helpers
 void launch_compute_radius(int variant, int P, const float* means, const float* scales, const float* rots,
@@ -236,7 +276,7 @@ struct RenderConfig {
     bool rule_long() const { return !own_shape && !own_split; }  // long tiles by the launch rule
 };
 LongList long_list_of(const RenderConfig& c, const ImageState& im, int num_tiles, const unsigned long long* totals,
-                      const BinState* stats, cudaStream_t s);
+                      const BinState* stats);
 bool valid_render_config(const RenderConfig& c);
 void set_render_config(const RenderConfig& c);
 RenderConfig get_render_config();

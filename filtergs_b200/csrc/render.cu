@@ -1489,13 +1489,15 @@ template <int PPT>
 constexpr int bwd_multi_min_ctas() { return PPT == 2 ? 8 : (PPT == 4 ? 12 : 1); }
 
 template <int PPT, int kBatch, bool kConsistent>
-__global__ void __launch_bounds__(256 / PPT) render_bwd_kernel(TileArgs a, unsigned* err)
+__global__ void __launch_bounds__(256 / PPT) render_bwd_kernel(TileArgs a, ZeroList zero, unsigned* err)
 {
     extern __shared__ __align__(128) unsigned char bwd_dyn[];
     BwdSmemT<PPT, kBatch>& sm = *reinterpret_cast<BwdSmemT<PPT, kBatch>*>(bwd_dyn);
     bwd_smem_init(sm, 256 / PPT);
     uint32_t gb = 0;
     render_bwd_tile<PPT, kBatch, kConsistent>(sm, a, blockIdx.x, gb, err);
+    // last, so that the first blocks composite while later ones have not yet anything to store
+    zero_share(zero, blockIdx.x, gridDim.x);
 }
 
 template <int PPT, int kBatch, bool kConsistent>
@@ -1640,7 +1642,7 @@ size_t bwd_smem_bytes(Kern k)
 
 template <int PPT, int B>
 void bwd_launch(int grid, const ImageState& im, const BinState& b, int W, int H, const float* bg, const float* dL,
-                int consistent, unsigned* err, cudaStream_t s)
+                int consistent, const ZeroList& zero, unsigned* err, cudaStream_t s)
 {
     TileArgs a{};
     a.ranges = im.ranges; a.recs = b.rec; a.W = W; a.H = H; a.bg = bg;
@@ -1648,10 +1650,10 @@ void bwd_launch(int grid, const ImageState& im, const BinState& b, int W, int H,
     a.dL_dpix = dL; a.pgrad = b.pgrad;
     if (consistent) {
         const size_t smem = bwd_smem_bytes<PPT, B, 2>(render_bwd_kernel<PPT, B, true>);
-        render_bwd_kernel<PPT, B, true><<<grid, 256 / PPT, smem, s>>>(a, err);
+        render_bwd_kernel<PPT, B, true><<<grid, 256 / PPT, smem, s>>>(a, zero, err);
     } else {
         const size_t smem = bwd_smem_bytes<PPT, B, 0>(render_bwd_kernel<PPT, B, false>);
-        render_bwd_kernel<PPT, B, false><<<grid, 256 / PPT, smem, s>>>(a, err);
+        render_bwd_kernel<PPT, B, false><<<grid, 256 / PPT, smem, s>>>(a, zero, err);
     }
 }
 
@@ -1822,12 +1824,13 @@ void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, const
 }
 
 void launch_render_bwd(int W, int H, const ImageState& im, const BinState& b, const float* bg,
-                       const float* dL_dpix, int consistent, unsigned* err, cudaStream_t s)
+                       const float* dL_dpix, int consistent, const ZeroList& zero, unsigned* err, cudaStream_t s)
 {
     const int gx = (W + kTileX - 1) / kTileX, gy = (H + kTileY - 1) / kTileY;
     RenderConfig c = g_cfg;
     bwd_rule(c, (uint32_t)(gx * gy) <= kSmallViewTiles);
-    FGS_RENDER_DISPATCH(bwd_launch, c.bwd_ppt, c.bwd_batch, gx * gy, im, b, W, H, bg, dL_dpix, consistent, err, s);
+    FGS_RENDER_DISPATCH(bwd_launch, c.bwd_ppt, c.bwd_batch, gx * gy, im, b, W, H, bg, dL_dpix, consistent, zero, err,
+                        s);
     note_launches(1);
 }
 

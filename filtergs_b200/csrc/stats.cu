@@ -16,9 +16,8 @@ constexpr int kBins = 11;
 
 __global__ void __launch_bounds__(128) kpc_kernel(const uint2* __restrict__ ranges, const float* __restrict__ kv_sum,
                                                   const uint32_t* __restrict__ kv_cnt, float used_thresh,
-                                                  double* __restrict__ out /* gtc, used, unused, bins[11] */,
-                                                  double* __restrict__ tile_ratio, double* __restrict__ tile_total,
-                                                  int num_tiles)
+                                                  double* __restrict__ out, double* __restrict__ tile_ratio,
+                                                  double* __restrict__ tile_total, int num_tiles)
 {
     const float edges[kBins] = {0.01f, 0.05f, 0.10f, 0.15f, 0.20f, 0.25f, 0.30f, 0.35f, 0.40f, 0.45f, 0.50f};
     __shared__ unsigned long long s_cnt[kBins + 3];  // bins, used, unused, used_in_tile
@@ -58,23 +57,23 @@ __global__ void __launch_bounds__(128) kpc_kernel(const uint2* __restrict__ rang
         tile_total[t] = (double)n;
         tile_ratio[t] = n ? (double)s_cnt[kBins + 2] / (double)n : 0.0;
         if (n) atomicAdd(&out[0], s_sum / (double)n);
-        if (s_cnt[kBins]) atomicAdd(&out[1], (double)s_cnt[kBins]);
-        if (s_cnt[kBins + 1]) atomicAdd(&out[2], (double)s_cnt[kBins + 1]);
+        if (s_cnt[kBins]) atomicAdd(&out[6], (double)s_cnt[kBins]);
+        if (s_cnt[kBins + 1]) atomicAdd(&out[7], (double)s_cnt[kBins + 1]);
         for (int b = 0; b < kBins; b++)
-            if (s_cnt[b]) atomicAdd(&out[3 + b], (double)s_cnt[b]);
+            if (s_cnt[b]) atomicAdd(&out[9 + FGS_STATS_SLOTS + b], (double)s_cnt[b]);
     }
 }
 
 }  // namespace
 
-// dev_out: [3 + 11 + 2 * num_tiles] doubles, zeroed here.
 void launch_kpc_stats(const BinState& b, const ImageState& im, int num_tiles, float used_thresh, double* dev_out,
-                      cudaStream_t s)
+                      int need, cudaStream_t s)
 {
-    cudaMemsetAsync(dev_out, 0, sizeof(double) * (3 + kBins + 2 * (size_t)num_tiles), s);
+    cudaMemsetAsync(dev_out, 0, sizeof(double) * (size_t)need, s);
     if (num_tiles <= 0) return;
-    kpc_kernel<<<num_tiles, 128, 0, s>>>(im.ranges, b.kv_sum, b.kv_cnt, used_thresh, dev_out, dev_out + 3 + kBins,
-                                         dev_out + 3 + kBins + num_tiles, num_tiles);
+    double* tiles = dev_out + 9 + 2 * FGS_STATS_SLOTS;
+    kpc_kernel<<<num_tiles, 128, 0, s>>>(im.ranges, b.kv_sum, b.kv_cnt, used_thresh, dev_out, tiles,
+                                         tiles + num_tiles, num_tiles);
     note_launches(1);
 }
 

@@ -64,6 +64,8 @@ class _RasterizeGaussians(torch.autograd.Function):
         ctx.raster_settings = raster_settings
         ctx.num_rendered = num_rendered
         ctx.use_filter = bool(use_filter)
+        # the other outputs' gradients are not used: no zero tensors for them
+        ctx.set_materialize_grads(False)
         ctx.save_for_backward(colors_precomp, means3D, scales, rotations, cov3Ds_precomp, radii, sh, geomBuffer,
                               binningBuffer, imgBuffer)
         return color, radii, point_id, point_weight_pixel, point_weight
@@ -72,6 +74,8 @@ class _RasterizeGaussians(torch.autograd.Function):
     def backward(ctx, grad_out_color, radii, point_id, point_weight_pixel, point_weight):
         num_rendered = ctx.num_rendered
         rs = ctx.raster_settings
+        if grad_out_color is None:  # the image is not part of the loss
+            grad_out_color = torch.zeros(3, int(rs.image_height), int(rs.image_width), device=ctx.saved_tensors[1].device)
         colors_precomp, means3D, scales, rotations, cov3Ds_precomp, radii, sh, geomBuffer, binningBuffer, \
             imgBuffer = ctx.saved_tensors
         args = (rs.bg, means3D, radii, colors_precomp, scales, rotations, rs.scale_modifier, cov3Ds_precomp,
@@ -124,7 +128,7 @@ def parse_stats(stats_tensor):
     """The `latest_stats` dictionary of wodilate/__init__.py:306-344."""
     if stats_tensor is None or not torch.is_tensor(stats_tensor):
         return None
-    s = stats_tensor.detach().cpu().tolist()
+    s = stats_tensor.detach().cpu().numpy().tolist()
     if len(s) < 16:
         return None
     d = {'bar_g': float(s[0]), 'avg_kv_per_gaussian': float(s[1]), 'avg_kv_per_tile': float(s[2]),
