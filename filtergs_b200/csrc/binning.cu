@@ -23,15 +23,13 @@ namespace fgs {
 
 namespace {
 
-constexpr int kSortThreads = 256;
-constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 16;                        // keys per thread, at most
-constexpr int kSortItemsMin = 8;                      // keys per thread, at least
-constexpr int kSortTile = kSortThreads * kSortItems;  // largest chunk
-constexpr int kSortTileMin = kSortThreads * kSortItemsMin;
+constexpr int kSortTileMin = 2048;  // smallest chunk (sizes the status words)
+constexpr int kSortItems = 16;      // keys per thread, at most
 constexpr int kRadix = 256;
-// Exclusive scan of one value per thread over a 256-thread block.
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp /*[8]*/, uint32_t* total)
+
+// Exclusive scan of one value per thread over the first 256 threads of a block (all
+// threads call it; s_warp: 8 words).
+__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp, uint32_t* total)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t x = v;
@@ -40,11 +38,11 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
-    if (lane == 31) s_warp[warp] = x;
+    if (lane == 31 && warp < 8) s_warp[warp] = x;
     __syncthreads();
     uint32_t wpre = 0, tot = 0;
 #pragma unroll
-    for (int w = 0; w < kSortWarps; w++) {
+    for (int w = 0; w < 8; w++) {
         const uint32_t c = s_warp[w];
         if (w < warp) wpre += c;
         tot += c;
@@ -54,6 +52,17 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp
     return wpre + x - v;
 }
 
+template <int kThreads>
+struct SortSmem {
+    uint16_t hist[kThreads / 32][kRadix];  // per warp; a chunk holds at most 16384 keys
+    uint32_t keys[kThreads * kSortItems];
+    uint32_t vals[kThreads * kSortItems];
+    uint32_t start[kRadix];
+    uint32_t gbase[kRadix];
+    uint32_t warp[8];
+    uint32_t chunk;
+};
+
 // One onesweep pass over `n` 32-bit keys with 32-bit values.
 //   vals_in == nullptr: values are the element indices.
 //   rec_out != nullptr (last tile pass): also gathers the per-Gaussian render
@@ -61,12 +70,22 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp
 //   n_dev != nullptr: the live count is min(n, *n_dev) (the grid covers n).
 // Persistent: each CTA takes chunks from the counter until none is left, so a
 // grid sized for a bound costs nothing for the chunks that are not live.  Per
-// chunk: rank the keys (warp match), publish the digit counts at once, sort the
+// chunk: rank the keys (a ballot per digit bit), publish the digit counts at once, sort the
 // chunk locally in shared memory (which needs no global offsets), and only
 // then walk back for the global offsets -- the registers that held the keys
-// are free by then, so the walk keeps 32 status loads in flight per digit
-// (64 registers, 4 CTAs per SM).
-__global__ void __launch_bounds__(kSortThreads, 4)
+// are free by then, so the walk keeps 32 status loads in flight per digit.
+//
+// With all chunks of a pass resident at once a walk sums half of the chunks before it,
+// some six instructions each on every digit's thread: in blocks of 256 threads that
+// was more than half of all instructions of the tile passes (570 chunks, 211 thread
+// instructions per pair), so their blocks have 1024 threads and chunks of up to 16384
+// pairs (128 chunks).  The depth sort, which runs over the ~120K visible Gaussians of a
+// view and beside seven other views in a batch, takes 512: at least 2048 keys per chunk
+// are then four per thread instead of eight, a shorter chain of ranks.
+// A 1080p view of 2M Gaussians with 2.1M pairs: the four depth passes 84 -> 70 us, the two
+// tile passes 126 -> 110; a 256x256 view of 10K Gaussians, all six passes: 59 -> 51 us.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads)
     onesweep_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
                     const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ vals_out, uint32_t n, int shift,
                     int nbits, const uint32_t* __restrict__ pass_hist, uint32_t* status, uint32_t* chunk_counter,
@@ -74,37 +93,32 @@ __global__ void __launch_bounds__(kSortThreads, 4)
                     const unsigned long long* __restrict__ n_dev, const int2* __restrict__ erow, int gx,
                     unsigned long long wait_ns = kWaitLimitNs, uint32_t skip_chunk = 0xffffffffu)
 {
-    __shared__ uint32_t s_hist[kSortWarps][kRadix];
-    __shared__ uint32_t s_keys[kSortTile];
-    __shared__ uint32_t s_vals[kSortTile];
-    __shared__ uint32_t s_start[kRadix];
-    __shared__ uint32_t s_gbase[kRadix];
-    __shared__ uint32_t s_warp[kSortWarps];
-    __shared__ uint32_t s_chunk;
+    constexpr int kWarps = kThreads / 32, kItemsMin = kSortTileMin / kThreads;
+    extern __shared__ __align__(16) unsigned char sort_dyn[];
+    SortSmem<kThreads>& sm = *reinterpret_cast<SortSmem<kThreads>*>(sort_dyn);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (n_dev) n = (uint32_t)min((unsigned long long)n, *n_dev);
     // Keys per thread from the live count: about one chunk per resident CTA, between
-    // kSortItemsMin and kSortItems (a small sort gets more, shorter chunks; a large one
+    // kItemsMin and kSortItems (a small sort gets more, shorter chunks; a large one
     // fewer chunks and a shorter look-back chain).  The same on every CTA.
     const uint32_t per_cta = (n + gridDim.x - 1) / gridDim.x;
     const int items = (int)min((uint32_t)kSortItems,
-                               max((uint32_t)kSortItemsMin, (per_cta + kSortThreads - 1) / kSortThreads));
-    const uint32_t tile = (uint32_t)items * kSortThreads;
+                               max((uint32_t)kItemsMin, (per_cta + kThreads - 1) / kThreads));
+    const uint32_t tile = (uint32_t)items * kThreads;
     const uint32_t live = (n + tile - 1) / tile;
     if (blockIdx.x >= live) return;
     const uint32_t dmask = (1u << nbits) - 1u;
     // global start of every digit in this pass (the same for all chunks)
     const uint32_t gh = (uint32_t)tid <= dmask ? __ldg(pass_hist + tid) : 0u;
-    const uint32_t gofs = block_excl_scan(gh, s_warp, nullptr);
+    const uint32_t gofs = block_excl_scan(gh, sm.warp, nullptr);
     const unsigned lt = (1u << lane) - 1u;
 
     for (;;) {
-        if (tid == 0) s_chunk = atomicAdd(chunk_counter, 1u);
-#pragma unroll
-        for (int w = 0; w < kSortWarps; w++) s_hist[w][tid] = 0;
+        if (tid == 0) sm.chunk = atomicAdd(chunk_counter, 1u);
+        for (int i = tid; i < kWarps * kRadix / 2; i += kThreads) reinterpret_cast<uint32_t*>(sm.hist)[i] = 0;
         __syncthreads();
-        const uint32_t chunk = s_chunk;
+        const uint32_t chunk = sm.chunk;
         if (chunk >= live) break;
         const uint32_t base = chunk * tile;
         const uint32_t count = min(tile, n - base);
@@ -114,33 +128,47 @@ __global__ void __launch_bounds__(kSortThreads, 4)
         for (int i = 0; i < kSortItems; i++) {
             if (i >= items) break;
             const uint32_t pos = warp * (items * 32) + i * 32 + lane;
+            key[i] = pos < count ? __ldg(keys_in + base + pos) : 0xffffffffu;
+        }
+#pragma unroll
+        for (int i = 0; i < kSortItems; i++) {
+            if (i >= items) break;
+            const uint32_t pos = warp * (items * 32) + i * 32 + lane;
             const bool valid = pos < count;
-            key[i] = valid ? __ldg(keys_in + base + pos) : 0xffffffffu;
-            const uint32_t dg = valid ? ((key[i] >> shift) & dmask) : kRadix;
-            const unsigned peers = __match_any_sync(0xffffffffu, dg);
-            const int leader = __ffs(peers) - 1;
-            uint32_t old = 0;
-            if (lane == leader && dg < kRadix) {
-                old = s_hist[warp][dg];
-                s_hist[warp][dg] = old + __popc(peers);
+            const uint32_t dg = (key[i] >> shift) & dmask;
+            // lanes with this lane's digit: one vote per digit bit (a match instruction takes longer)
+            unsigned peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+                if (b >= nbits) break;
+                const bool one = (dg >> b) & 1u;
+                const unsigned m = __ballot_sync(0xffffffffu, one);
+                peers &= one ? m : ~m;
             }
-            old = __shfl_sync(0xffffffffu, old, leader);
+            // every lane of a digit reads its count before the last of them adds to it
+            uint32_t old = 0;
+            if (valid) old = sm.hist[warp][dg];
+            __syncwarp();
+            if (valid && (peers >> lane) == 1u) sm.hist[warp][dg] = (uint16_t)(old + __popc(peers));
             rank[i] = old + __popc(peers & lt);
             __syncwarp();
         }
         __syncthreads();
         // per digit (thread d): exclusive prefix over warps, chunk total, published at once
         uint32_t tot = 0;
-#pragma unroll
-        for (int w = 0; w < kSortWarps; w++) {
-            const uint32_t c = s_hist[w][tid];
-            s_hist[w][tid] = tot;
-            tot += c;
-        }
         // skip_chunk (a test hook) never publishes: its successors wait until wait_ns runs out
         const bool publish = chunk != skip_chunk;
-        if (publish) lookback_publish(status + tid, chunk, kRadix, tot);
-        s_start[tid] = block_excl_scan(tot, s_warp, nullptr);
+        if ((uint32_t)tid <= dmask) {
+#pragma unroll 8
+            for (int w = 0; w < kWarps; w++) {
+                const uint32_t c = sm.hist[w][tid];
+                sm.hist[w][tid] = (uint16_t)tot;
+                tot += c;
+            }
+            if (publish) lookback_publish(status + tid, chunk, kRadix, tot);
+        }
+        const uint32_t start = block_excl_scan(tot, sm.warp, nullptr);
+        if (tid < kRadix) sm.start[tid] = start;
         __syncthreads();
         // local sort of the chunk by digit
 #pragma unroll
@@ -149,19 +177,20 @@ __global__ void __launch_bounds__(kSortThreads, 4)
             const uint32_t pos = warp * (items * 32) + i * 32 + lane;
             if (pos < count) {
                 const uint32_t dg = (key[i] >> shift) & dmask;
-                const uint32_t lp = s_start[dg] + s_hist[warp][dg] + rank[i];
-                s_keys[lp] = key[i];
-                s_vals[lp] = vals_in ? __ldg(vals_in + base + pos) : base + pos;
+                const uint32_t lp = sm.start[dg] + sm.hist[warp][dg] + rank[i];
+                sm.keys[lp] = key[i];
+                sm.vals[lp] = vals_in ? __ldg(vals_in + base + pos) : base + pos;
             }
         }
         // global offset of this chunk's digit run
-        s_gbase[tid] = gofs + thread_lookback_walk<32>(status + tid, chunk, kRadix, tot, err, wait_ns, publish);
+        if ((uint32_t)tid <= dmask)
+            sm.gbase[tid] = gofs + thread_lookback_walk<32>(status + tid, chunk, kRadix, tot, err, wait_ns, publish);
         __syncthreads();
-        for (uint32_t p = tid; p < count; p += kSortThreads) {
-            const uint32_t k = s_keys[p];
+        for (uint32_t p = tid; p < count; p += kThreads) {
+            const uint32_t k = sm.keys[p];
             const uint32_t dg = (k >> shift) & dmask;
-            const uint32_t gp = s_gbase[dg] + (p - s_start[dg]);
-            const uint32_t v = s_vals[p];
+            const uint32_t gp = sm.gbase[dg] + (p - sm.start[dg]);
+            const uint32_t v = sm.vals[p];
             if (gp >= n) {  // cannot happen with consistent histograms; never write out of bounds
                 set_error(err, FGS_ERR_OVERFLOW);
                 continue;
@@ -186,6 +215,8 @@ __global__ void __launch_bounds__(kSortThreads, 4)
         __syncthreads();  // shared buffers are reused by the next chunk
     }
 }
+
+constexpr int kDepthThreads = 512, kTileThreads = 1024;
 
 // Histograms of the 4 depth-key bytes (one read of the keys).
 __global__ void depth_hist_kernel(const uint32_t* __restrict__ keys, uint32_t n,
@@ -449,7 +480,8 @@ void launch_depth_sort(const GeomState& g, int P, cudaStream_t s)
     const uint32_t hb0 = (n + 1023) / 1024;
     const int hb = (int)(hb0 < 1184u ? hb0 : 1184u);
     depth_hist_kernel<<<hb, 256, 0, s>>>(g.depth_key, n, V, g.hist);
-    const uint32_t grid = min(nch, resident_ctas(onesweep_kernel, kSortThreads));
+    const size_t smem = sizeof(SortSmem<kDepthThreads>);
+    const uint32_t grid = min(nch, resident_ctas(onesweep_kernel<kDepthThreads>, kDepthThreads, smem));
     note_launches(5);
     // ping-pong: depth_key -> sort_keys_b -> depth_key -> sort_keys_b ; ids b -> a -> b -> a -> b
     const uint32_t* kin[4] = {g.depth_key, g.sort_keys_b, g.depth_key, g.sort_keys_b};
@@ -457,11 +489,10 @@ void launch_depth_sort(const GeomState& g, int P, cudaStream_t s)
     const uint32_t* vin[4] = {g.sort_ids_b, g.sort_ids_a, g.sort_ids_b, g.sort_ids_a};
     uint32_t* vout[4] = {g.sort_ids_a, g.sort_ids_b, g.sort_ids_a, g.sort_ids_b};
     for (int pass = 0; pass < 4; pass++) {
-        onesweep_kernel<<<grid, kSortThreads, 0, s>>>(kin[pass], kout[pass], vin[pass], vout[pass], n, 8 * pass, 8,
-                                                     g.hist + pass * kRadix, g.status + (size_t)pass * nch * kRadix,
-                                                     g.counters + pass, g.err, nullptr, nullptr, V, nullptr, 1,
-                                                     pass ? kWaitLimitNs : g_fault_wait_ns,
-                                                     pass ? 0xffffffffu : g_fault_skip_chunk);
+        onesweep_kernel<kDepthThreads><<<grid, kDepthThreads, smem, s>>>(
+            kin[pass], kout[pass], vin[pass], vout[pass], n, 8 * pass, 8, g.hist + pass * kRadix,
+            g.status + (size_t)pass * nch * kRadix, g.counters + pass, g.err, nullptr, nullptr, V, nullptr, 1,
+            pass ? kWaitLimitNs : g_fault_wait_ns, pass ? 0xffffffffu : g_fault_skip_chunk);
     }
 }
 
@@ -494,7 +525,8 @@ void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int ti
     (void)H;
     const uint32_t n = (uint32_t)K;
     const uint32_t nch = chunks_of(n, kSortTileMin);
-    const uint32_t grid = min(nch, resident_ctas(onesweep_kernel, kSortThreads));
+    const size_t smem = sizeof(SortSmem<kTileThreads>);
+    const uint32_t grid = min(nch, resident_ctas(onesweep_kernel<kTileThreads>, kTileThreads, smem));
     const int passes = (tile_bits + 7) / 8;
     const uint32_t* ki = (passes & 1) ? b.tile_a : b.tile_b;
     const uint32_t* vi = (passes & 1) ? b.val_a : b.val_b;
@@ -503,10 +535,10 @@ void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int ti
         const int nbits = min(8, tile_bits - 8 * pass);
         uint32_t* ko = (ki == b.tile_a) ? b.tile_b : b.tile_a;
         uint32_t* vo = (vi == b.val_a) ? b.val_b : b.val_a;
-        onesweep_kernel<<<grid, kSortThreads, 0, s>>>(ki, ko, vi, vo, n, 8 * pass, nbits, g.hist + (4 + pass) * kRadix,
-                                                     b.status + (size_t)pass * nch * kRadix, g.counters + 4 + pass,
-                                                     g.err, last ? g.grec : nullptr, last ? b.rec : nullptr, n_dev,
-                                                     g.erow, gx);
+        onesweep_kernel<kTileThreads><<<grid, kTileThreads, smem, s>>>(
+            ki, ko, vi, vo, n, 8 * pass, nbits, g.hist + (4 + pass) * kRadix,
+            b.status + (size_t)pass * nch * kRadix, g.counters + 4 + pass, g.err, last ? g.grec : nullptr,
+            last ? b.rec : nullptr, n_dev, g.erow, gx);
         ki = ko;
         vi = vo;
     }

@@ -259,11 +259,12 @@ cudaEvent_t pool_event()
 
 void note_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-uint32_t resident_ctas_query(const void* kernel, int threads)
+uint32_t resident_ctas_query(const void* kernel, int threads, size_t smem)
 {
     struct Entry {
         const void* k;
         int threads, dev;
+        size_t smem;
         uint32_t ctas;
     };
     static std::mutex mu;
@@ -272,12 +273,14 @@ uint32_t resident_ctas_query(const void* kernel, int threads)
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lock(mu);
     for (const Entry& e : cache)
-        if (e.k == kernel && e.threads == threads && e.dev == dev) return e.ctas;
+        if (e.k == kernel && e.threads == threads && e.dev == dev && e.smem == smem) return e.ctas;
     int sms = 148, per = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, 0);
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
     const uint32_t r = (uint32_t)(sms * (per > 0 ? per : 1));
-    cache.push_back(Entry{kernel, threads, dev, r});
+    cache.push_back(Entry{kernel, threads, dev, smem, r});
     return r;
 }
 

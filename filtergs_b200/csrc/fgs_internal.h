@@ -93,14 +93,15 @@ size_t bin_bytes_forward(long long K, int P);  // without the per-pair gradients
 int tile_bits_for(int num_tiles);
 
 // ---------------------------------------------------------------- launchers
-// Resident CTAs of a kernel on this device (persistent grids never exceed it).
-// Cached per (kernel, block size, device): kernels of the same signature have
+// Resident CTAs of a kernel on this device (persistent grids never exceed it), with `smem` bytes
+// of dynamic shared memory, which the first query on a device opts the kernel in to.
+// Cached per (kernel, block size, shared memory, device): kernels of the same signature have
 // their own entries.
-uint32_t resident_ctas_query(const void* kernel, int threads);
+uint32_t resident_ctas_query(const void* kernel, int threads, size_t smem);
 template <typename Kern>
-inline uint32_t resident_ctas(Kern k, int threads)
+inline uint32_t resident_ctas(Kern k, int threads, size_t smem = 0)
 {
-    return resident_ctas_query(reinterpret_cast<const void*>(k), threads);
+    return resident_ctas_query(reinterpret_cast<const void*>(k), threads, smem);
 }
 
 void launch_preprocess(const PreParams& p, const GeomState& g, int* radii, cudaStream_t s);
