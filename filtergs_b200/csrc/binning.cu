@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
                 const int2 er = __ldg(erow + v);
                 const uint32_t ty = k / (uint32_t)gx, tx = k - ty * (uint32_t)gx;
                 r.c.w = __uint_as_float((uint32_t)er.x + ty * (uint32_t)er.y + tx);
-                r.c.z = __uint_as_float(quad_mask(r, (float)(tx * kTileX), (float)(ty * kTileY)));
+                r.c.z = __uint_as_float(block_mask(r, (float)(tx * kTileX), (float)(ty * kTileY)));
                 rec_out[gp] = r;
             }
         }

@@ -398,7 +398,7 @@ __device__ __forceinline__ float3 sh_to_rgb(int deg, const float* __restrict__ s
 struct __align__(16) PairRecord {
     float4 a;  // x, y, conic.x, conic.y
     float4 b;  // conic.z, opacity, r, g
-    float4 c;  // b, gaussian id (bits); per Gaussian: view depth, 0; per sorted pair: quad_mask, emission index (bits)
+    float4 c;  // b, gaussian id (bits); per Gaussian: view depth, 0; per sorted pair: block_mask, emission index (bits)
 };
 static_assert(sizeof(PairRecord) == 48, "record size");
 
@@ -409,12 +409,12 @@ __device__ __forceinline__ float sqrt_approx(float v)
     return r;
 }
 
-// The 8x8 quads of the tile at (tx0, ty0) in which a Gaussian can reach alpha >= 1/255
-// at a pixel centre: bit 2 r + c for the quad of columns tx0 + 8 c .. + 7 and rows
-// ty0 + 8 r .. + 7; and kWild when its colour or position is not finite or too large for
-// arithmetic that multiplies unreached pixels by zero.  A quad outside the mask has no
+// The 8x4 blocks of the tile at (tx0, ty0) in which a Gaussian can reach alpha >= 1/255
+// at a pixel centre: bit 2 r + c for the block of columns tx0 + 8 c .. + 7 and rows
+// ty0 + 4 r .. + 3; and kWild when its colour or position is not finite or too large for
+// arithmetic that multiplies unreached pixels by zero.  A block outside the mask has no
 // pixel that the per-pixel tests of the compositing accept, so skipping it changes no
-// output.
+// output.  (mask >> 2 r) & 3: the 16x4 strip r; (mask >> (4 q + c)) & 5: the 8x8 quad (c, q).
 //
 // alpha >= 1/255 needs Q(d) = a dx^2 + 2 b dx dy + c dy^2 <= t0 = 2 ln(255 o).  The test
 // uses the ellipse Q <= t, t = 1.02 t0 + 0.1.  Within a strip of rows its right edge
@@ -423,10 +423,10 @@ __device__ __forceinline__ float sqrt_approx(float v)
 // clamped to the strip and to |dy| <= sqrt(t a / det); the left edge is its mirror image.
 // With det >= 2.5e-4 a c (kappa = a c / det <= 4000) the rounding of the per-pixel Q
 // (under 12 eps kappa t < 0.3%), of det (eps kappa) and of the square roots stays far
-// inside the 2% + 0.1; every quad for a conic beyond that, and for one that is not
+// inside the 2% + 0.1; every block for a conic beyond that, and for one that is not
 // positive definite.
-constexpr uint32_t kWild = 16u;
-__device__ __forceinline__ uint32_t quad_mask(const PairRecord& g, float tx0, float ty0)
+constexpr uint32_t kWild = 256u;
+__device__ __forceinline__ uint32_t block_mask(const PairRecord& g, float tx0, float ty0)
 {
     const float mx = g.a.x, my = g.a.y, a = g.a.z, b = g.a.w, c = g.b.x, o = g.b.y;
     const bool tame = fabsf(mx) < 1e7f && fabsf(my) < 1e7f && fabsf(g.b.z) < 1e15f && fabsf(g.b.w) < 1e15f &&
@@ -439,13 +439,13 @@ __device__ __forceinline__ uint32_t quad_mask(const PairRecord& g, float tx0, fl
     const float xmax = sqrt_approx(s * c), ymax = sqrt_approx(s * a);
     if (!(tame && a > 0.f && c > 0.f && det >= 2.5e-4f * ac && xmax < 1e7f && ymax < 1e7f && ra < 1e30f &&
           a * t < 1e30f))
-        return wild | 15u;
+        return wild | 255u;
     const float ytop = -__fdividef(b * xmax, c);  // where the right edge is furthest; -ytop for the left one
     const float X = tx0 - mx, at = a * t;
     uint32_t m = 0;
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-        const float lo = fmaxf(ty0 + 8 * r - my, -ymax), hi = fminf(ty0 + 8 * r + 7 - my, ymax);
+    for (int r = 0; r < 4; r++) {
+        const float lo = fmaxf(ty0 + 4 * r - my, -ymax), hi = fminf(ty0 + 4 * r + 3 - my, ymax);
         const float yr = fminf(fmaxf(ytop, lo), hi), yl = fminf(fmaxf(-ytop, lo), hi);
         const float xr = (sqrt_approx(fmaxf(at - det * yr * yr, 0.f)) - b * yr) * ra + 0.01f;
         const float xl = -(sqrt_approx(fmaxf(at - det * yl * yl, 0.f)) + b * yl) * ra - 0.01f;

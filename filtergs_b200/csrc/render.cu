@@ -5,10 +5,9 @@
 // records (written by the last sort pass), so each record batch is ONE bulk copy
 // (cp.async.bulk, the TMA engine's 1-D form) into shared memory, completed on an
 // mbarrier.  Three record buffers keep two batches in flight while the current
-// one is composited.  A warp owns a block of 8 columns x 4 PPT rows (PPT pixels of
-// one column per lane, 4 rows apart), and a record carries the mask of the tile's
-// four 8x8 quads it can reach (quad_mask, written by the sort): one ballot per 32
-// records tells a warp which of them to composite.
+// one is composited.  A warp owns a block of pixels (PPT of one column per lane), and a
+// record carries the mask of the tile's eight 8x4 blocks it can reach (block_mask,
+// written by the sort): one ballot per 32 records tells a warp which to composite.
 //
 // Both directions are bound by instruction issue (86% and 73% of the issue slots of
 // 1080p views), so two pixels of a lane are composited per instruction with packed
@@ -98,24 +97,26 @@ __device__ __forceinline__ float warp_sum(float v)
     return v;
 }
 
-// The block of pixels of this thread's warp: 8 columns x 4 PPT rows of the tile, lane
-// (x, y) = (lane & 7, lane >> 3), its pixel k at row y + 4 k.
+// The forward's block of pixels of this thread's warp: 8 columns x 4 PPT rows of the tile,
+// lane (x, y) = (lane & 7, lane >> 3), its pixel k at row y + 4 k.
 template <int PPT>
 struct WarpBlock {
-    int px, py0, col, quad_row;  // first pixel; the block's column of quads and its first row of quads
+    int px, py0, bit;  // first pixel; the block's first bit in a record's block_mask
     __device__ __forceinline__ WarpBlock(int bx, int by)
     {
         const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        col = w & 1;
-        const int row = (w >> 1) * 4 * PPT;
-        quad_row = row >> 3;
+        const int col = w & 1, row = (w >> 1) * 4 * PPT;
+        bit = 2 * (row >> 2) + col;
         px = bx * kTileX + 8 * col + (lane & 7);
         py0 = by * kTileY + row + (lane >> 3);
     }
 };
-// Quads of 8x8 pixels one warp's block covers (a block of PPT = 1 is half a quad).
+// Quads of 8x8 pixels one warp's block covers (a block of PPT = 1 is half a quad), and the
+// block_mask bits of one of them above the block's first bit.
 template <int PPT>
 constexpr int warp_quads() { return PPT == 4 ? 2 : 1; }
+template <int PPT>
+constexpr uint32_t quad_bits() { return PPT == 1 ? 1u : 5u; }
 
 // ---------------------------------------------------------------- per-view render descriptors
 // Everything one tile needs, for the plain launch (one view, one tile per CTA)
@@ -133,14 +134,13 @@ struct FwdSmem {
     uint32_t kcnt[2][kBatch];
 };
 
-// Per-record gradient sums of a batch, [record][component] so that the nine lanes
-// that store a record's totals hit nine banks.  With two warps per tile (PPT = 4)
-// each has a slot of its own, stores its totals (no read-modify-write; a record the
-// warp did not touch is told by `live`), and the slots are added in warp order.  With
-// more warps, warps 2s and 2s+1 add into slot s: a slot starts at zero and takes at
-// most two additions, and float addition is commutative, so its value does not depend
-// on which warp came first.  Either way the result is the same on every run (no
-// order-dependent float atomics anywhere in the backward).
+// Per-record gradient sums of a batch, [record][component] so that the lanes that store a
+// record's totals hit different banks.  With two warps per tile (PPT = 4) each has a slot
+// of its own and stores its totals (no read-modify-write; a record the warp did not touch
+// is told by `live`).  With more, warps 2s and 2s+1 add into slot s: a slot starts at zero
+// and takes at most two additions, and float addition is commutative, so its value does not
+// depend on which warp came first.  Slots are added in order.  Either way the result is the
+// same on every run (no order-dependent float atomics anywhere in the backward).
 template <int PPT>
 constexpr int bwd_slots() { return PPT == 4 ? 2 : (256 / PPT / 32) / 2; }
 
@@ -152,6 +152,8 @@ struct BwdSmem {
     uint32_t live[2][kBatch / 32];
     uint32_t max_last;
 };
+template <int PPT, int kBatch>
+using BwdSmemT = BwdSmem<kBatch, bwd_slots<PPT>()>;
 
 // ---------------------------------------------------------------- forward
 // One (pixel, record) step of the compositing loop (forward.cu:466-544), in two
@@ -207,10 +209,9 @@ __device__ __forceinline__ float fwd_accumulate(float alpha, const float4 rb, co
 // outputs), point_id / point_weight_pixel / point_weight, or those and the statistics.
 enum { kImage = 0, kWeights = 1, kStats = 2 };
 
-// One pixel's state between records: T, colour and the strongest contributor as in
-// fwd_accumulate; amin is the smallest alpha that still counts: 1/255, or 2 (no alpha
-// reaches it) once the pixel is done or when it lies outside the image.
-constexpr float kAlphaMin = 1.0f / 255.0f, kDone = 2.0f;
+// One pixel's state between records: colour and the strongest contributor as in
+// fwd_accumulate; T is the transmittance, negative once the pixel takes no record any more
+// (it lies outside the image, or the next record would have brought T below 1e-4).
 
 // One record on one pixel, with branches: the form for one pixel per lane, and for a
 // record whose colour or position is too large for the packed form (kWild), where a
@@ -218,13 +219,14 @@ constexpr float kAlphaMin = 1.0f / 255.0f, kDone = 2.0f;
 // the record took, 0 when it did not contribute.
 __device__ __forceinline__ float fwd_pixel_step(const float4 ra, const float4 rb, float c2, int id, float pxf,
                                                 float pyf, uint32_t position, float& T, float& C0, float& C1,
-                                                float& C2, float& wmax, int& maxid, uint32_t& last, float& amin)
+                                                float& C2, float& wmax, int& maxid, uint32_t& last)
 {
+    if (T < 0.f) return 0.f;
     const float alpha = fwd_alpha(ra, rb, pxf, pyf);
-    if (!(alpha >= amin)) return 0.f;
+    if (alpha == 0.f) return 0.f;
     const float test_T = __fmul_rn(T, 1.0f - alpha);
     if (test_T < 0.0001f) {
-        amin = kDone;
+        T = -T;
         return 0.f;
     }
     C0 = __fmaf_rn(__fmul_rn(rb.z, alpha), T, C0);
@@ -244,16 +246,16 @@ __device__ __forceinline__ float fwd_pixel_step(const float4 ra, const float4 rb
 template <int NP>
 struct FwdPixels {
     F2 T[NP], C[NP][3], wmax[NP], npy[NP];  // npy: -row
-    float amin[2 * NP];
     int maxid[2 * NP];
     uint32_t last[2 * NP];
 };
 
-// One record on one pair of pixels, without branches: a pixel the record does not
-// reach takes alpha 0, which leaves T, the colours and the weight as they are (T * 1,
-// C + 0 * T).  The same operations, in the same order and rounding, as fwd_alpha and
-// fwd_accumulate.  Returns the larger of the two weights (kImage: alphas): > 0 when
-// either pixel took something.
+// One record on one pair of pixels, without branches: a pixel that does not take the
+// record gets alpha 0, which leaves the colours and the weight as they are (C + 0 * T).
+// The same operations, in the same order and rounding, as fwd_alpha and fwd_accumulate.
+// A pixel that is done has T < 0, so its product with 1 - alpha is below 1e-4 for every
+// record: one comparison tells both.  Returns the larger of the two weights (kImage:
+// alphas): > 0 when either pixel took something.
 template <int kOut, int NP>
 __device__ __forceinline__ float fwd_pair_step(FwdPixels<NP>& s, int q, const float4 ra, const float4 rb, float c2,
                                                int id, float dx, float sx, float nbx, uint32_t position, F2& wsum,
@@ -263,25 +265,18 @@ __device__ __forceinline__ float fwd_pair_step(FwdPixels<NP>& s, int q, const fl
     const F2 qf = f2_fma(f2(sx), f2(dx), f2_mul(f2_mul(f2(rb.x), dy), dy));
     const F2 power = f2_fma(f2(-0.5f), qf, f2_mul(f2(nbx), dy));
     const F2 oG = f2_mul(f2(rb.y), f2(expf(f2_lo(power)), expf(f2_hi(power))));
-    const float a0 = fminf(0.99f, f2_lo(oG)), a1 = fminf(0.99f, f2_hi(oG));
-    float& m0 = s.amin[2 * q];
-    float& m1 = s.amin[2 * q + 1];
-    const bool ok0 = !(f2_lo(power) > 0.f) && a0 >= m0, ok1 = !(f2_hi(power) > 0.f) && a1 >= m1;
-    F2 alpha = f2(ok0 ? a0 : 0.f, ok1 ? a1 : 0.f);
-    const F2 keep = f2_fma(alpha, f2(-1.f), f2(1.f));  // 1 - alpha
-    const F2 test_T = f2_mul(s.T[q], keep);
-    // (a pixel that takes nothing keeps T >= 1e-4 and cannot end here)
-    const bool end0 = ok0 && f2_lo(test_T) < 0.0001f, end1 = ok1 && f2_hi(test_T) < 0.0001f;
-    m0 = end0 ? kDone : m0;
-    m1 = end1 ? kDone : m1;
-    const float e0 = end0 ? 0.f : f2_lo(alpha), e1 = end1 ? 0.f : f2_hi(alpha);
-    alpha = f2(e0, e1);
+    const F2 a = f2(fminf(0.99f, f2_lo(oG)), fminf(0.99f, f2_hi(oG)));
+    const F2 test_T = f2_mul(s.T[q], f2_fma(a, f2(-1.f), f2(1.f)));  // T (1 - alpha)
+    const bool ok0 = !(f2_lo(power) > 0.f) && f2_lo(a) >= 1.0f / 255.0f;
+    const bool ok1 = !(f2_hi(power) > 0.f) && f2_hi(a) >= 1.0f / 255.0f;
+    const bool take0 = ok0 && !(f2_lo(test_T) < 0.0001f), take1 = ok1 && !(f2_hi(test_T) < 0.0001f);
+    const F2 alpha = f2(take0 ? f2_lo(a) : 0.f, take1 ? f2_hi(a) : 0.f);
     s.C[q][0] = f2_fma(f2_mul(f2(rb.z), alpha), s.T[q], s.C[q][0]);
     s.C[q][1] = f2_fma(f2_mul(f2(rb.w), alpha), s.T[q], s.C[q][1]);
     s.C[q][2] = f2_fma(f2_mul(f2(c2), alpha), s.T[q], s.C[q][2]);
-    s.last[2 * q] = e0 > 0.f ? position : s.last[2 * q];
-    s.last[2 * q + 1] = e1 > 0.f ? position : s.last[2 * q + 1];
-    float took = fmaxf(e0, e1);
+    s.last[2 * q] = take0 ? position : s.last[2 * q];
+    s.last[2 * q + 1] = take1 ? position : s.last[2 * q + 1];
+    float took = fmaxf(f2_lo(alpha), f2_hi(alpha));
     if constexpr (kOut != kImage) {
         const F2 w = f2_mul(s.T[q], alpha);
         const float w0 = f2_lo(w), w1 = f2_hi(w);
@@ -291,11 +286,13 @@ __device__ __forceinline__ float fwd_pair_step(FwdPixels<NP>& s, int q, const fl
         s.maxid[2 * q + 1] = g1 ? id : s.maxid[2 * q + 1];
         took = fmaxf(w0, w1);
         if constexpr (kOut == kStats) {
-            wsum = f2_add(wsum, w);
-            wcount += (e0 > 0.f) + (e1 > 0.f);
+            wsum = f2_add(wsum, f2(fmaxf(w0, 0.f), fmaxf(w1, 0.f)));
+            wcount += (int)take0 + (int)take1;
         }
     }
-    s.T[q] = f2(end0 ? f2_lo(s.T[q]) : f2_lo(test_T), end1 ? f2_hi(s.T[q]) : f2_hi(test_T));
+    // taken: T (1 - alpha); reached but not taken: done; else unchanged
+    const float T0 = f2_lo(s.T[q]), T1 = f2_hi(s.T[q]);
+    s.T[q] = f2(take0 ? f2_lo(test_T) : (ok0 ? -fabsf(T0) : T0), take1 ? f2_hi(test_T) : (ok1 ? -fabsf(T1) : T1));
     return took;
 }
 
@@ -334,27 +331,26 @@ __device__ __forceinline__ void render_fwd_tile(FwdSmem<kBatch>& sm, const TileA
     FwdPixels<NP> s;
 #pragma unroll
     for (int q = 0; q < NP; q++) {
-        s.T[q] = f2(1.f);
         s.C[q][0] = s.C[q][1] = s.C[q][2] = f2(0.f);
         s.wmax[q] = f2(0.f);
         s.npy[q] = f2(-(float)(blk.py0 + 8 * q), -(float)(blk.py0 + 8 * q + 4));
+        float T[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const bool inside = px < W && blk.py0 + 8 * q + 4 * h < H && 2 * q + h < PPT;
-            s.amin[2 * q + h] = inside ? kAlphaMin : kDone;
+            T[h] = inside ? 1.f : -1.f;  // negative: takes no record any more
             s.last[2 * q + h] = 0;
             s.maxid[2 * q + h] = -1;
         }
+        s.T[q] = f2(T[0], T[1]);
     }
     const float pxf = (float)px;
     auto all_done = [&] {
         bool d = true;
 #pragma unroll
-        for (int k = 0; k < PPT; k++) d = d && s.amin[k] > 1.f;
+        for (int k = 0; k < PPT; k++) d = d && ((k & 1) ? f2_hi(s.T[k >> 1]) : f2_lo(s.T[k >> 1])) < 0.f;
         return d;
     };
-    const int qbit0 = 2 * blk.quad_row + blk.col;
-
     int issued = nb < 2 ? nb : 2;
     uint32_t contributor = 0;
     bool stop = __all_sync(0xffffffffu, all_done());  // warp-uniform: no pixel of the warp takes any more
@@ -369,11 +365,11 @@ __device__ __forceinline__ void render_fwd_tile(FwdSmem<kBatch>& sm, const TileA
         for (uint32_t k0 = 0; k0 < cnt && !stop; k0 += 32) {
             // which of these 32 records reach this warp's quads
             const uint32_t e = k0 + (tid & 31);
-            const uint32_t mask = e < cnt ? __float_as_uint(R[e].c.z) >> qbit0 : 0u;
+            const uint32_t mask = e < cnt ? __float_as_uint(R[e].c.z) >> blk.bit : 0u;
             uint32_t quad[kQuads], live = 0;
 #pragma unroll
             for (int q = 0; q < kQuads; q++) {
-                quad[q] = __ballot_sync(0xffffffffu, (mask >> (2 * q)) & 1u);
+                quad[q] = __ballot_sync(0xffffffffu, ((mask >> (4 * q)) & quad_bits<PPT>()) != 0);
                 live |= quad[q];
             }
             while (live) {
@@ -397,7 +393,7 @@ __device__ __forceinline__ void render_fwd_tile(FwdSmem<kBatch>& sm, const TileA
                         for (int c = 0; c < 3; c++) C[c] = (k & 1) ? f2_hi(s.C[q][c]) : f2_lo(s.C[q][c]);
                         const float pyf = -((k & 1) ? f2_hi(s.npy[q]) : f2_lo(s.npy[q]));
                         const float w = fwd_pixel_step(ra, rb, rc.x, __float_as_int(rc.y), pxf, pyf, position, T, C[0],
-                                                       C[1], C[2], wm, s.maxid[k], s.last[k], s.amin[k]);
+                                                       C[1], C[2], wm, s.maxid[k], s.last[k]);
                         wj = fmaxf(wj, w);
                         wsum = f2_add(wsum, f2(w, 0.f));
                         kc += w > 0.f;
@@ -489,7 +485,7 @@ __device__ __forceinline__ void render_fwd_tile(FwdSmem<kBatch>& sm, const TileA
         auto half = [&](F2 v) { return (k & 1) ? f2_hi(v) : f2_lo(v); };
         if (px < W && py < H) {
             const int pix = W * py + px;
-            const float T = half(s.T[q]);
+            const float T = fabsf(half(s.T[q]));
             a.final_T[pix] = T;
             a.n_contrib[pix] = s.last[k];
             a.out_color[pix] = __fmaf_rn(T, a.bg[0], half(s.C[q][0]));
@@ -903,11 +899,11 @@ __global__ void __launch_bounds__(LongTile<BW, BH>::kThreads)
 
 // ---------------------------------------------------------------- long tiles by quads
 // The launch rule's form of a long tile: a CTA renders a unit of 8x4 pixels, four warps
-// with a 4x2 band each, and stages only the records whose quad_mask has the unit's quad.
+// with a 4x2 band each, and stages only the records whose block_mask has the unit's block.
 // What bounds a tile of thousands of small splats is staging, not compositing: with
 // every record staged and tested by each of the tile's eight CTAs, two thirds of the
 // time went there.  Here a CTA reads the 4-byte masks of kUnitIn records (the next ones
-// in flight meanwhile), compacts the survivors (about a quarter) in order, loads only
+// in flight meanwhile), compacts the survivors (about a seventh) in order, loads only
 // those records and tests only those against the bands.  Per pixel the same records in
 // the same order with the same arithmetic as on the tile path.  8M-node LoD views at
 // 1080p with 2.7M / 6.4M / 8.5M pairs: 0.60 / 1.08 / 1.06 ms; in bands that stage every
@@ -933,7 +929,7 @@ __device__ __forceinline__ void render_unit(UnitSmem& sm, const TileArgs& a, int
     const int bx = tile % gx, by = tile / gx, ux = unit & 1, uy = unit >> 1;
     const float tx0 = (float)(bx * kTileX), ty0 = (float)(by * kTileY);
     const int band0 = 8 * uy + 2 * ux;  // the unit's bands in band_mask<4, 2>: band0 + {0, 1, 4, 5}
-    const int qbit = 2 * (uy >> 1) + ux;
+    const int mbit = 2 * uy + ux;  // the unit's bit in a record's block_mask
     const int pix_lane = lane % kPix, slot = lane / kPix;
     const int px = bx * kTileX + 8 * ux + 4 * (warp & 1) + pix_lane % 4;
     const int py = by * kTileY + 4 * uy + 2 * (warp >> 1) + pix_lane / 4;
@@ -960,7 +956,7 @@ __device__ __forceinline__ void render_unit(UnitSmem& sm, const TileArgs& a, int
         uint32_t b[kPer];
 #pragma unroll
         for (int i = 0; i < kPer; i++) {
-            b[i] = __ballot_sync(0xffffffffu, (m[i] >> qbit) & 1u);
+            b[i] = __ballot_sync(0xffffffffu, (m[i] >> mbit) & 1u);
             if (lane == 0) sm.cnt[i * (kUnitThreads / 32) + warp] = __popc(b[i]);
         }
 #pragma unroll
@@ -1146,30 +1142,30 @@ __global__ void __launch_bounds__(256 / kRulePpt, fwd_min_ctas<kRulePpt>())
 }
 
 // ---------------------------------------------------------------- backward
-// The pixels of one lane in the backward, in pairs (k = 2q, 2q + 1).  The reference's
-// accum_rec recurrence (the colour composited behind the current Gaussian,
-// backward.cu:513-520) enters dL/dalpha only through its dot product with dL/dpixel,
-// so a pixel carries that dot product (acc): one value instead of six.  bgT: the
-// numerator -T_final (bg . dL/dpixel) of the background term of dL/dalpha.
+// The backward's pixels: a warp owns PPT / 2 strips of 16x4 (half a strip at one pixel per
+// lane), lane (x, y) = (lane & 15, lane >> 4) with the rows 2 y and 2 y + 1 of each strip, so
+// that all of a lane's pixels share a column.  In pairs (k = 2q, 2q + 1: a strip's).
+// The reference's accum_rec recurrence (the colour composited behind the current Gaussian,
+// backward.cu:513-520) enters dL/dalpha only through its dot product with dL/dpixel, so a
+// pixel carries that dot product (acc): one value instead of six.  bgT: the numerator
+// -T_final (bg . dL/dpixel) of the background term of dL/dalpha.
 template <int NP>
 struct BwdPixels {
     F2 T[NP], acc[NP], d[NP][3], bgT[NP], npy[NP];
     uint32_t last[2 * NP];
 };
 
-// A record's sums over a lane's pixels: alpha T dL/dpixel (c) and w, w dy, w dy dy (s)
-// with w = G dL/dalpha.  All of a lane's pixels share a column, so the products with dx
-// are formed from these once per column (warp_column_sum9) instead of once per pixel.
-struct BwdSums {
-    F2 c[3], s[3];
-};
+// A record's nine sums over a lane's pixels of one strip, with w = G dL/dalpha:
+// alpha T dL/dpixel (three channels), w dx, w dy, w dx dx, w dx dy, w dy dy, w.  Pixels are
+// added one after the other, lanes by warp_transpose_sum9 and strips as (0 + 1) + (2 + 3),
+// whatever the block's shape: a training step carries the last bits of these sums on to the
+// next one, where they decide comparisons.
 
-// One record on one pixel, with branches (see fwd_pixel_step for when).  The values of
-// the pixel are passed one by one; sums go into the low halves.
+// One record on one pixel, with branches (see fwd_pixel_step for when).
 template <bool kConsistent>
 __device__ __forceinline__ bool bwd_pixel_step(const float4 ra, const float4 rb, float c2, float pxf, float pyf,
                                                bool before_last, float& T, float& acc, float d0, float d1, float d2,
-                                               float bgT, BwdSums& g)
+                                               float bgT, float (&g)[9])
 {
     if (!before_last) return false;
     const float dx = ra.x - pxf, dy = ra.y - pyf;
@@ -1181,21 +1177,24 @@ __device__ __forceinline__ bool bwd_pixel_step(const float4 ra, const float4 rb,
     const float alpha = fminf(0.99f, oG);
     if (alpha < 1.0f / 255.0f) return false;
     const float inv = __fdividef(1.f, 1.f - alpha);
-    T = T * inv;
-    const float wc = alpha * T;
-    g.c[0] = f2_add(g.c[0], f2(wc * d0, 0.f));
-    g.c[1] = f2_add(g.c[1], f2(wc * d1, 0.f));
-    g.c[2] = f2_add(g.c[2], f2(wc * d2, 0.f));
-    const float cdot = rb.z * d0 + rb.w * d1 + c2 * d2;
+    T = __fmul_rn(T, inv);
+    const float wc = __fmul_rn(alpha, T);
+    g[0] = __fmaf_rn(wc, d0, g[0]);
+    g[1] = __fmaf_rn(wc, d1, g[1]);
+    g[2] = __fmaf_rn(wc, d2, g[2]);
+    const float cdot = __fmaf_rn(c2, d2, __fmaf_rn(rb.z, d0, __fmul_rn(rb.w, d1)));
     const float diff = cdot - acc;
-    float dL_dalpha = diff * T;
-    if (bgT != 0.f) dL_dalpha += bgT * inv;
+    float dL_dalpha = __fmul_rn(diff, T);
+    if (bgT != 0.f) dL_dalpha = __fmaf_rn(bgT, inv, dL_dalpha);
     if (kConsistent && oG > 0.99f) dL_dalpha = 0.f;
-    acc += alpha * diff;
-    const float w = G * dL_dalpha, v = w * dy;
-    g.s[0] = f2_add(g.s[0], f2(w, 0.f));
-    g.s[1] = f2_add(g.s[1], f2(v, 0.f));
-    g.s[2] = f2_add(g.s[2], f2(v * dy, 0.f));
+    acc = __fmaf_rn(alpha, diff, acc);
+    const float w = __fmul_rn(G, dL_dalpha), u = __fmul_rn(w, dx), v = __fmul_rn(w, dy);
+    g[3] = __fadd_rn(g[3], u);
+    g[4] = __fadd_rn(g[4], v);
+    g[5] = __fmaf_rn(u, dx, g[5]);
+    g[6] = __fmaf_rn(u, dy, g[6]);
+    g[7] = __fmaf_rn(v, dy, g[7]);
+    g[8] = __fadd_rn(g[8], w);
     return true;
 }
 
@@ -1206,7 +1205,7 @@ __device__ __forceinline__ bool bwd_pixel_step(const float4 ra, const float4 rb,
 // below 1e15 here (kWild records and warps take bwd_pixel_step), so no 0 * inf arises.
 template <bool kConsistent, int NP>
 __device__ __forceinline__ bool bwd_pair_step(BwdPixels<NP>& s, int q, const float4 ra, const float4 rb, float c2,
-                                              float dx, float sx, float nbx, uint32_t contributor, BwdSums& g)
+                                              float dx, float sx, float nbx, uint32_t contributor, float (&g)[9])
 {
     const F2 dy = f2_add(f2(ra.y), s.npy[q]);
     const F2 qf = f2_fma(f2(sx), f2(dx), f2_mul(f2_mul(f2(rb.x), dy), dy));
@@ -1223,80 +1222,60 @@ __device__ __forceinline__ bool bwd_pair_step(BwdPixels<NP>& s, int q, const flo
     s.T[q] = f2_mul(s.T[q], inv);  // transmittance before this Gaussian
     const F2 wc = f2_mul(alpha, s.T[q]);
 #pragma unroll
-    for (int c = 0; c < 3; c++) g.c[c] = f2_fma(wc, s.d[q][c], g.c[c]);
-    const F2 cdot = f2_fma(f2(c2), s.d[q][2], f2_fma(f2(rb.w), s.d[q][1], f2_mul(f2(rb.z), s.d[q][0])));
+    for (int i = 0; i < 3; i++)
+        g[i] = __fmaf_rn(f2_hi(wc), f2_hi(s.d[q][i]), __fmul_rn(f2_lo(wc), f2_lo(s.d[q][i])));
+    const F2 cdot = f2_fma(f2(c2), s.d[q][2], f2_fma(f2(rb.z), s.d[q][0], f2_mul(f2(rb.w), s.d[q][1])));
     const F2 diff = f2_fma(s.acc[q], f2(-1.f), cdot);
     s.acc[q] = f2_fma(alpha, diff, s.acc[q]);
     const F2 dL_dalpha = f2_fma(s.bgT[q], inv, f2_mul(diff, s.T[q]));
     F2 w = f2_mul(G, dL_dalpha);
     const bool w0 = ok0 && !(kConsistent && f2_lo(oG) > 0.99f), w1 = ok1 && !(kConsistent && f2_hi(oG) > 0.99f);
     w = f2(w0 ? f2_lo(w) : 0.f, w1 ? f2_hi(w) : 0.f);
-    const F2 v = f2_mul(w, dy);
-    g.s[0] = f2_add(g.s[0], w);
-    g.s[1] = f2_add(g.s[1], v);
-    g.s[2] = f2_fma(v, dy, g.s[2]);
+    const F2 u = f2_mul(w, f2(dx)), v = f2_mul(w, dy);
+    g[3] = __fadd_rn(f2_lo(u), f2_hi(u));
+    g[4] = __fadd_rn(f2_lo(v), f2_hi(v));
+    g[5] = __fmaf_rn(f2_hi(u), dx, __fmul_rn(f2_lo(u), dx));
+    g[6] = __fmaf_rn(f2_hi(u), f2_hi(dy), __fmul_rn(f2_lo(u), f2_lo(dy)));
+    g[7] = __fmaf_rn(f2_hi(v), f2_hi(dy), __fmul_rn(f2_lo(v), f2_lo(dy)));
+    g[8] = __fadd_rn(f2_lo(w), f2_hi(w));
     return ok0 || ok1;
 }
 
-// The nine sums of a record over a warp's block (8 columns x 4 rows of lanes) from each
-// lane's BwdSums.  The lanes of a column (lane distances 16 and 8) are added first: at
-// distance 16 the upper lanes keep s and the lower ones c; after distance 8 every lane
-// has its column's three totals, and the lanes with bit 3 of the upper half turn theirs
-// into the dx products (w dx, w dx dx, w dy dx).  Then the eight columns: 3 -> 2 -> 1
-// values over distances 4 and 2, and a plain step over distance 1.  10 shuffles.
-// Lane l ends with the total of component column_sum9_component(l) of
-// c0 c1 c2 | w dx, w dy | w dx dx, w dx dy, w dy dy | w.
-__device__ __forceinline__ float warp_column_sum9(const BwdSums& g, float dx)
+// Nine sums of a warp's two strips, added: the first level of the butterfly gives each half
+// of the warp one strip, which halves what the next levels exchange (21 shuffles; one strip
+// after the other takes 24).  Lane l ends with the total of value sum9_component(2 l) for l < 16.
+__device__ __forceinline__ float strip_pair_sum9(const float (&a)[9], const float (&b)[9])
 {
     const unsigned lane = threadIdx.x & 31;
-    const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4, b2 = lane & 2;
-    float v[3];
+    const bool hi = lane & 16;
+    float v9[9], v5[5], v3[3], v2[2], v1[1];
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const float c = f2_lo(g.c[i]) + f2_hi(g.c[i]), s = f2_lo(g.s[i]) + f2_hi(g.s[i]);
-        v[i] = (b16 ? s : c) + __shfl_xor_sync(0xffffffffu, b16 ? c : s, 16);
-    }
-#pragma unroll
-    for (int i = 0; i < 3; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 8);
-    const bool expand = b16 && b8;
-    const float x0 = v[0] * dx, x1 = x0 * dx, x2 = v[1] * dx;
-    v[0] = expand ? x0 : v[0];
-    v[1] = expand ? x1 : v[1];
-    v[2] = expand ? x2 : v[2];
-    const float r0 = (b4 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, b4 ? v[0] : v[2], 4);
-    const float r1 = v[1] + __shfl_xor_sync(0xffffffffu, v[1], 4);
-    const float t = (b2 ? r1 : r0) + __shfl_xor_sync(0xffffffffu, b2 ? r0 : r1, 2);
-    return t + __shfl_xor_sync(0xffffffffu, t, 1);
-}
-
-// Which component warp_column_sum9 leaves on `lane`; 15 for the lanes whose copy is not
-// stored (odd lanes, the second copies).
-__device__ __forceinline__ int column_sum9_component(unsigned lane)
-{
-    const int part = (lane >> 3) & 3, pick = (lane & 2) ? 1 : ((lane & 4) ? 2 : 0);
-    if ((lane & 1) || part == 1 || ((lane & 2) && (lane & 4))) return 15;
-    // parts (three nibbles each): 0 colours, 2 (w, w dy, w dy dy), 3 (w dx, w dx dx, w dx dy)
-    return (int)((0x653748fff210ull >> (4 * (3 * part + pick))) & 15u);
+    for (int i = 0; i < 9; i++) v9[i] = (hi ? b[i] : a[i]) + __shfl_xor_sync(0xffffffffu, hi ? a[i] : b[i], 16);
+    sum9_level<5, 9>(v9, v5, lane, 8);
+    sum9_level<3, 5>(v5, v3, lane, 4);
+    sum9_level<2, 3>(v3, v2, lane, 2);
+    sum9_level<1, 2>(v2, v1, lane, 1);
+    return v1[0] + __shfl_xor_sync(0xffffffffu, v1[0], 16);
 }
 
 // kConsistent: the exact-gradient backward mode (FGS_BACKWARD_CONSISTENT), a
 // compile-time switch so that the reference mode pays nothing for it per pixel.
 template <int PPT, int kBatch, bool kConsistent>
-__device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()>& sm, const TileArgs& a, int tile,
-                                                uint32_t& gb, unsigned* err)
+__device__ __forceinline__ void render_bwd_tile(BwdSmemT<PPT, kBatch>& sm, const TileArgs& a, int tile, uint32_t& gb,
+                                                unsigned* err)
 {
     constexpr int kSlots = bwd_slots<PPT>();
     constexpr bool kOwnSlot = PPT == 4;
     constexpr int NT = 256 / PPT;
     constexpr int NP = PPT > 1 ? PPT / 2 : 1;
-    constexpr int kQuads = warp_quads<PPT>();
     constexpr int NG = 9;  // dcolor r,g,b ; dmean2D x,y ; dconic x,y,w ; dopacity
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int W = a.W, H = a.H;
     const int gx = (W + kTileX - 1) / kTileX;
     const int bx = tile % gx, by = tile / gx;
-    const WarpBlock<PPT> blk(bx, by);
-    const int px = blk.px;
+    const int px = bx * kTileX + (lane & 15);
+    // first row of the lane's pair in the warp's first strip (its row at one pixel per lane)
+    const int py0 = by * kTileY + 2 * PPT * warp + (PPT > 1 ? 2 : 1) * (lane >> 4);
     const uint2 range = a.ranges[tile];
     const PairRecord* recs = a.recs;
 
@@ -1309,7 +1288,7 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()
         float T[2], d[2][3], bgT[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int py = blk.py0 + 8 * q + 4 * h;
+            const int py = py0 + 4 * q + h;
             const bool inside = px < W && py < H && 2 * q + h < PPT;
             const int pix = W * py + px;
             T[h] = inside ? a.final_T[pix] : 0.f;
@@ -1326,22 +1305,24 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()
         s.T[q] = f2(T[0], T[1]);
         s.bgT[q] = f2(bgT[0], bgT[1]);
         s.acc[q] = f2(0.f);
-        s.npy[q] = f2(-(float)(blk.py0 + 8 * q), -(float)(blk.py0 + 8 * q + 4));
+        s.npy[q] = f2(-(float)(py0 + 4 * q), -(float)(py0 + 4 * q + 1));
 #pragma unroll
         for (int c = 0; c < 3; c++) s.d[q][c] = f2(d[0][c], d[1][c]);
     }
     // a gradient too large for the packed form (or not finite) sends the warp the other way
     const uint32_t wild_warp = __all_sync(0xffffffffu, tame) ? 0u : kWild;
     const float pxf = (float)px;
-    const int qbit0 = 2 * blk.quad_row + blk.col;
+    const int mbit = PPT == 4 ? 4 * warp : 2 * (warp * PPT / 2);  // the first strip's bits in a block_mask
     const float ddelx_dx = 0.5 * W;
     const float ddely_dy = 0.5 * H;
-    const int q_lane = column_sum9_component((unsigned)tid & 31u);
+    // the component whose total each lane holds after warp_transpose_sum9, strip_pair_sum9
+    const int q_lane = (lane & 1) ? 15 : sum9_component((unsigned)lane);
+    const int q_pair = lane < 16 ? sum9_component(2u * lane) : 15;
 
     if (tid == 0) sm.max_last = 0;
     __syncthreads();
     const uint32_t warp_last = __reduce_max_sync(0xffffffffu, my_max);
-    if ((tid & 31) == 0) atomicMax(&sm.max_last, warp_last);
+    if (lane == 0) atomicMax(&sm.max_last, warp_last);
     __syncthreads();
     // Entries at or beyond the largest n_contrib of the tile touch no pixel.
     const uint32_t n = min(range.y - range.x, sm.max_last);
@@ -1364,14 +1345,14 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()
         const PairRecord* R = sm.rec[buf];
         for (int k0 = (int)((cnt - 1) & ~31u); k0 >= 0; k0 -= 32) {
             // records of this chunk that sit before some pixel's last contributor and reach
-            // this warp's quads, walked back to front
-            const uint32_t e = (uint32_t)k0 + (tid & 31);
-            const uint32_t mask = e < cnt && lo + e < warp_last ? __float_as_uint(R[e].c.z) >> qbit0 : 0u;
-            uint32_t quad[kQuads], live = 0, touched = 0;
+            // this warp's strips, walked back to front
+            const uint32_t e = (uint32_t)k0 + lane;
+            const uint32_t mask = e < cnt && lo + e < warp_last ? __float_as_uint(R[e].c.z) >> mbit : 0u;
+            uint32_t strip[NP], live = 0, touched = 0;
 #pragma unroll
-            for (int q = 0; q < kQuads; q++) {
-                quad[q] = __ballot_sync(0xffffffffu, (mask >> (2 * q)) & 1u);
-                live |= quad[q];
+            for (int q = 0; q < NP; q++) {
+                strip[q] = __ballot_sync(0xffffffffu, ((mask >> (2 * q)) & 3u) != 0);
+                live |= strip[q];
             }
             while (live) {
                 const int bit = 31 - __clz(live);
@@ -1381,42 +1362,55 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()
                 const float4 ra = R[j].a;
                 const float4 rb = R[j].b;
                 const float2 rc = make_float2(R[j].c.x, R[j].c.z);
-                BwdSums sums;
-#pragma unroll
-                for (int i = 0; i < 3; i++) sums.c[i] = sums.s[i] = f2(0.f);
                 const float dx = ra.x - pxf;
-                bool any = false;
-                if (PPT == 1 || ((__float_as_uint(rc.y) | wild_warp) & kWild)) {
+                float g[NP][NG];
+                bool any[NP];
+                const bool branchy = PPT == 1 || ((__float_as_uint(rc.y) | wild_warp) & kWild);
+                const float sx = __fmul_rn(ra.z, dx), nbx = -__fmul_rn(ra.w, dx);
 #pragma unroll
-                    for (int k = 0; k < PPT; k++) {
-                        const int q = k >> 1;
-                        auto half = [&](F2 v) { return (k & 1) ? f2_hi(v) : f2_lo(v); };
-                        float T = half(s.T[q]), acc = half(s.acc[q]);
-                        any |= bwd_pixel_step<kConsistent>(ra, rb, rc.x, pxf, -half(s.npy[q]), contributor < s.last[k],
-                                                           T, acc, half(s.d[q][0]), half(s.d[q][1]), half(s.d[q][2]),
-                                                           half(s.bgT[q]), sums);
-                        s.T[q] = (k & 1) ? f2(f2_lo(s.T[q]), T) : f2(T, f2_hi(s.T[q]));
-                        s.acc[q] = (k & 1) ? f2(f2_lo(s.acc[q]), acc) : f2(acc, f2_hi(s.acc[q]));
-                    }
-                } else {
-                    const float sx = __fmul_rn(ra.z, dx), nbx = -__fmul_rn(ra.w, dx);
+                for (int q = 0; q < NP; q++) {
+                    any[q] = false;
 #pragma unroll
-                    for (int q = 0; q < NP; q++)
-                        if (kQuads == 1 || ((quad[q] >> bit) & 1u))
-                            any |= bwd_pair_step<kConsistent, NP>(s, q, ra, rb, rc.x, dx, sx, nbx, contributor, sums);
-                }
-                if (__any_sync(0xffffffffu, any)) {
-                    const float tot = warp_column_sum9(sums, dx);
-                    if constexpr (kOwnSlot) {
-                        touched |= 1u << bit;
-                        if (q_lane < NG) sm.acc[warp][j][q_lane] = tot;
+                    for (int i = 0; i < NG; i++) g[q][i] = 0.f;
+                    if (NP > 1 && !((strip[q] >> bit) & 1u)) continue;
+                    if (branchy) {
+#pragma unroll
+                        for (int h = 0; h < 2 && 2 * q + h < PPT; h++) {
+                            auto half = [&](F2 x) { return h ? f2_hi(x) : f2_lo(x); };
+                            float T = half(s.T[q]), acc = half(s.acc[q]);
+                            any[q] |= bwd_pixel_step<kConsistent>(
+                                ra, rb, rc.x, pxf, -half(s.npy[q]), contributor < s.last[2 * q + h], T, acc,
+                                half(s.d[q][0]), half(s.d[q][1]), half(s.d[q][2]), half(s.bgT[q]), g[q]);
+                            s.T[q] = h ? f2(f2_lo(s.T[q]), T) : f2(T, f2_hi(s.T[q]));
+                            s.acc[q] = h ? f2(f2_lo(s.acc[q]), acc) : f2(acc, f2_hi(s.acc[q]));
+                        }
                     } else {
-                        if (q_lane < NG) atomicAdd(&sm.acc[warp >> 1][j][q_lane], tot);
+                        any[q] = bwd_pair_step<kConsistent, NP>(s, q, ra, rb, rc.x, dx, sx, nbx, contributor, g[q]);
                     }
+                }
+                if constexpr (kOwnSlot) {
+                    const bool first = __any_sync(0xffffffffu, any[0]), second = __any_sync(0xffffffffu, any[1]);
+                    if (first || second) {
+                        float tot;
+                        int at = q_lane;
+                        if (first && second) {
+                            tot = strip_pair_sum9(g[0], g[1]);
+                            at = q_pair;
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < NG; i++) g[0][i] = first ? g[0][i] : g[1][i];
+                            tot = warp_transpose_sum9(g[0]);
+                        }
+                        touched |= 1u << bit;
+                        if (at < NG) sm.acc[warp][j][at] = tot;
+                    }
+                } else if (__any_sync(0xffffffffu, any[0])) {
+                    const float tot = warp_transpose_sum9(g[0]);
+                    if (q_lane < NG) atomicAdd(&sm.acc[warp >> 1][j][q_lane], tot);
                 }
             }
             if constexpr (kOwnSlot)
-                if ((tid & 31) == 0) sm.live[warp][k0 >> 5] = touched;
+                if (lane == 0) sm.live[warp][k0 >> 5] = touched;
         }
         __syncthreads();
         // this batch's per-pair gradients, at each pair's emission index: the slot sums times
@@ -1428,11 +1422,12 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()
             for (int q = 0; q < NG; q++) sum[q] = 0.f;
 #pragma unroll
             for (int sl = 0; sl < kSlots; sl++) {
+                float* acc = sm.acc[sl][e];
                 if (kOwnSlot && !((sm.live[sl][e >> 5] >> (e & 31)) & 1u)) continue;
 #pragma unroll
                 for (int q = 0; q < NG; q++) {
-                    sum[q] += sm.acc[sl][e][q];
-                    if (!kOwnSlot) sm.acc[sl][e][q] = 0.f;
+                    sum[q] += acc[q];
+                    if (!kOwnSlot) acc[q] = 0.f;
                 }
             }
             const float4 ea = R[e].a, eb = R[e].b;  // conic (ea.z, ea.w, eb.x), opacity eb.y
@@ -1463,21 +1458,17 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmem<kBatch, bwd_slots<PPT>()
     }
 }
 
-template <int kBatch, int kSlots>
-__device__ __forceinline__ void bwd_smem_init(BwdSmem<kBatch, kSlots>& sm, int NT)
+template <typename Smem>
+__device__ __forceinline__ void bwd_smem_init(Smem& sm, int NT)
 {
-    for (int e = threadIdx.x; e < kSlots * 9 * kBatch; e += NT) (&sm.acc[0][0][0])[e] = 0.f;
+    float* acc = &sm.acc[0][0][0];
+    for (int e = threadIdx.x; e < (int)(sizeof(sm.acc) / sizeof(float)); e += NT) acc[e] = 0.f;
     if (threadIdx.x == 0) {
         for (int i = 0; i < kBufs; i++) mbar_init(&sm.bar[i], 1);
         mbar_fence_init();
     }
     __syncthreads();
 }
-
-// The backward's shared state can pass the 48 KB static limit (8 warps, 256-record
-// batches): it lives in dynamic shared memory.
-template <int PPT, int kBatch>
-using BwdSmemT = BwdSmem<kBatch, bwd_slots<PPT>()>;
 
 // Resident CTAs per SM the multi-view backward is compiled for: 32 warps at 2 pixels
 // per thread (64 registers, a few spilled bytes) and 24 at 4 (80 registers and a few

@@ -400,14 +400,16 @@ __global__ void densify_dense_kernel(int P, const int* __restrict__ radii, const
 }
 
 // sparse_optimizer.py:54-76 with torch's float32 arithmetic: the Python-float
-// coefficients beta and 1 - beta (formed in double) are rounded to float.
+// coefficients beta and 1 - beta (formed in double) are rounded to float.  The fused
+// products are spelled out, so that no parameter's last bits hang on how a caller's loop
+// is compiled.
 __device__ __forceinline__ void adam_update(float& p, float& m, float& v, float g, float b1, float omb1, float b2,
                                             float omb2, float step_size, float bc2_sqrt, float eps)
 {
-    m = m * b1 + g * omb1;
-    v = v * b2 + omb2 * g * g;
+    m = __fmaf_rn(g, omb1, __fmul_rn(m, b1));
+    v = __fmaf_rn(__fmul_rn(omb2, g), g, __fmul_rn(v, b2));
     const float denom = sqrtf(v) / bc2_sqrt + eps;
-    p = p + (-step_size) * (m / denom);
+    p = __fmaf_rn(-step_size, m / denom, p);
 }
 
 }  // namespace
