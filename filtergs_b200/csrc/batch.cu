@@ -398,7 +398,7 @@ int fgs_batch_backward(void* handle, void* stream)
     if (!B->g_means3D || !B->g_opacity) return FGS_ERR_ARG;
     {
         StageTimer t(FGS_STAGE_RENDER_BWD, s);
-        launch_render_bwd_multi(B->d_args_bwd, B->d_begin, B->h_begin.data(), B->V, B->d_queue + 1, B->consistent,
+        launch_render_bwd_multi(B->d_args_bwd, B->d_begin, B->V, B->total_tiles, B->d_queue + 1, B->consistent,
                                 B->d_err, s);
     }
     StageTimer t(FGS_STAGE_PREPROCESS_BWD, s);

@@ -262,8 +262,7 @@ struct TileArgs {
 void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const uint32_t* begin, int nviews,
                              uint32_t total_tiles, uint32_t* queue, uint32_t* long_list, uint32_t* long_ctr,
                              unsigned* err, cudaStream_t s);
-// host_begin: the values of begin; queue: two counters.
-void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, const uint32_t* host_begin, int nviews,
+void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
                              uint32_t* queue, int consistent, unsigned* err, cudaStream_t s);
 
 // Render kernel shape: pixels per thread {1,2,4} and records per shared-memory batch {64,128,256}.

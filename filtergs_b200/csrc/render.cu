@@ -134,26 +134,37 @@ struct FwdSmem {
     uint32_t kcnt[2][kBatch];
 };
 
-// Per-record gradient sums of a batch, [record][component] so that the lanes that store a
-// record's totals hit different banks.  With two warps per tile (PPT = 4) each has a slot
-// of its own and stores its totals (no read-modify-write; a record the warp did not touch
-// is told by `live`).  With more, warps 2s and 2s+1 add into slot s: a slot starts at zero
-// and takes at most two additions, and float addition is commutative, so its value does not
+constexpr int kPend = 4;  // steps that add_step_sums adds at once
+
+// The nine sums of up to kPend (record, strip) steps of a warp, every lane's, until
+// add_step_sums adds them over the lanes: a[half] holds four sums of each lane (lane l
+// of the second half at l ^ 4, so that the eight lanes that read a step meet no bank
+// twice), b the ninth.
+struct __align__(16) StepSums {
+    struct {
+        float4 a[2][32];
+        float b[40];
+    } step[kPend];
+    int rec[kPend];  // the record's index in the batch
+};
+
+// Per-record gradient sums of a batch.  With two warps per tile (PPT = 4) each has a slot of
+// its own.  With more, warps 2s and 2s+1 add into slot s: a slot starts at zero and takes at
+// most two additions per record, and float addition is commutative, so its value does not
 // depend on which warp came first.  Slots are added in order.  Either way the result is the
 // same on every run (no order-dependent float atomics anywhere in the backward).
 template <int PPT>
 constexpr int bwd_slots() { return PPT == 4 ? 2 : (256 / PPT / 32) / 2; }
 
-template <int kBatch, int kSlots>
+template <int PPT, int kBatch>
 struct BwdSmem {
     PairRecord rec[kBufs][kBatch];
+    StepSums step[PPT == 1 ? 1 : 8 / PPT];
     uint64_t bar[kBufs];
-    float acc[kSlots][kBatch][9];
-    uint32_t live[2][kBatch / 32];
+    float acc[kBufs][bwd_slots<PPT>()][kBatch][9];
+    uint32_t arrived[kBufs];  // warps that are through with a batch
     uint32_t max_last;
 };
-template <int PPT, int kBatch>
-using BwdSmemT = BwdSmem<kBatch, bwd_slots<PPT>()>;
 
 // ---------------------------------------------------------------- forward
 // One (pixel, record) step of the compositing loop (forward.cu:466-544), in two
@@ -1152,14 +1163,25 @@ __global__ void __launch_bounds__(256 / kRulePpt, fwd_min_ctas<kRulePpt>())
 template <int NP>
 struct BwdPixels {
     F2 T[NP], acc[NP], d[NP][3], bgT[NP], npy[NP];
+    F2 d01[NP][2];  // channels 0 and 1 of either pixel
     uint32_t last[2 * NP];
 };
 
 // A record's nine sums over a lane's pixels of one strip, with w = G dL/dalpha:
-// alpha T dL/dpixel (three channels), w dx, w dy, w dx dx, w dx dy, w dy dy, w.  Pixels are
+// alpha T dL/dpixel (channels 0, 1), w dx, w dy, w dx dx, w dx dy, w dy dy, w and
+// alpha T dL/dpixel (channel 2): neighbours come from one packed instruction.  Pixels are
 // added one after the other, lanes by warp_transpose_sum9 and strips as (0 + 1) + (2 + 3),
 // whatever the block's shape: a training step carries the last bits of these sums on to the
 // next one, where they decide comparisons.
+
+// 1 / x for x in [0.01, 1], with the bits of __fdividef(1, x) there, which spends its time on
+// guarding the ends of the range.
+__device__ __forceinline__ float rcp_unit(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 
 // One record on one pixel, with branches (see fwd_pixel_step for when).
 template <bool kConsistent>
@@ -1176,12 +1198,12 @@ __device__ __forceinline__ bool bwd_pixel_step(const float4 ra, const float4 rb,
     const float oG = __fmul_rn(rb.y, G);
     const float alpha = fminf(0.99f, oG);
     if (alpha < 1.0f / 255.0f) return false;
-    const float inv = __fdividef(1.f, 1.f - alpha);
+    const float inv = rcp_unit(1.f - alpha);
     T = __fmul_rn(T, inv);
     const float wc = __fmul_rn(alpha, T);
     g[0] = __fmaf_rn(wc, d0, g[0]);
     g[1] = __fmaf_rn(wc, d1, g[1]);
-    g[2] = __fmaf_rn(wc, d2, g[2]);
+    g[8] = __fmaf_rn(wc, d2, g[8]);
     const float cdot = __fmaf_rn(c2, d2, __fmaf_rn(rb.z, d0, __fmul_rn(rb.w, d1)));
     const float diff = cdot - acc;
     float dL_dalpha = __fmul_rn(diff, T);
@@ -1189,12 +1211,12 @@ __device__ __forceinline__ bool bwd_pixel_step(const float4 ra, const float4 rb,
     if (kConsistent && oG > 0.99f) dL_dalpha = 0.f;
     acc = __fmaf_rn(alpha, diff, acc);
     const float w = __fmul_rn(G, dL_dalpha), u = __fmul_rn(w, dx), v = __fmul_rn(w, dy);
-    g[3] = __fadd_rn(g[3], u);
-    g[4] = __fadd_rn(g[4], v);
-    g[5] = __fmaf_rn(u, dx, g[5]);
-    g[6] = __fmaf_rn(u, dy, g[6]);
-    g[7] = __fmaf_rn(v, dy, g[7]);
-    g[8] = __fadd_rn(g[8], w);
+    g[2] = __fadd_rn(g[2], u);
+    g[3] = __fadd_rn(g[3], v);
+    g[4] = __fmaf_rn(u, dx, g[4]);
+    g[5] = __fmaf_rn(u, dy, g[5]);
+    g[6] = __fmaf_rn(v, dy, g[6]);
+    g[7] = __fadd_rn(g[7], w);
     return true;
 }
 
@@ -1218,50 +1240,97 @@ __device__ __forceinline__ bool bwd_pair_step(BwdPixels<NP>& s, int q, const flo
     const F2 alpha = f2(ok0 ? a0 : 0.f, ok1 ? a1 : 0.f);
     const F2 rem = f2_fma(alpha, f2(-1.f), f2(1.f));
     // (fast reciprocal: 1 - alpha >= 0.01)
-    const F2 inv = f2(__fdividef(1.f, f2_lo(rem)), __fdividef(1.f, f2_hi(rem)));
+    const F2 inv = f2(rcp_unit(f2_lo(rem)), rcp_unit(f2_hi(rem)));
     s.T[q] = f2_mul(s.T[q], inv);  // transmittance before this Gaussian
     const F2 wc = f2_mul(alpha, s.T[q]);
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-        g[i] = __fmaf_rn(f2_hi(wc), f2_hi(s.d[q][i]), __fmul_rn(f2_lo(wc), f2_lo(s.d[q][i])));
+    const F2 c01 = f2_fma(f2(f2_hi(wc)), s.d01[q][1], f2_mul(f2(f2_lo(wc)), s.d01[q][0]));
+    g[0] = f2_lo(c01);
+    g[1] = f2_hi(c01);
+    g[8] = __fmaf_rn(f2_hi(wc), f2_hi(s.d[q][2]), __fmul_rn(f2_lo(wc), f2_lo(s.d[q][2])));
     const F2 cdot = f2_fma(f2(c2), s.d[q][2], f2_fma(f2(rb.z), s.d[q][0], f2_mul(f2(rb.w), s.d[q][1])));
     const F2 diff = f2_fma(s.acc[q], f2(-1.f), cdot);
     s.acc[q] = f2_fma(alpha, diff, s.acc[q]);
     const F2 dL_dalpha = f2_fma(s.bgT[q], inv, f2_mul(diff, s.T[q]));
-    F2 w = f2_mul(G, dL_dalpha);
-    const bool w0 = ok0 && !(kConsistent && f2_lo(oG) > 0.99f), w1 = ok1 && !(kConsistent && f2_hi(oG) > 0.99f);
-    w = f2(w0 ? f2_lo(w) : 0.f, w1 ? f2_hi(w) : 0.f);
-    const F2 u = f2_mul(w, f2(dx)), v = f2_mul(w, dy);
-    g[3] = __fadd_rn(f2_lo(u), f2_hi(u));
-    g[4] = __fadd_rn(f2_lo(v), f2_hi(v));
-    g[5] = __fmaf_rn(f2_hi(u), dx, __fmul_rn(f2_lo(u), dx));
-    g[6] = __fmaf_rn(f2_hi(u), f2_hi(dy), __fmul_rn(f2_lo(u), f2_lo(dy)));
-    g[7] = __fmaf_rn(f2_hi(v), f2_hi(dy), __fmul_rn(f2_lo(v), f2_lo(dy)));
-    g[8] = __fadd_rn(f2_lo(w), f2_hi(w));
+    const F2 Gd = f2_mul(G, dL_dalpha);
+    const float w0 = ok0 && !(kConsistent && f2_lo(oG) > 0.99f) ? f2_lo(Gd) : 0.f;
+    const float w1 = ok1 && !(kConsistent && f2_hi(oG) > 0.99f) ? f2_hi(Gd) : 0.f;
+    const F2 xy0 = f2(dx, f2_lo(dy)), xy1 = f2(dx, f2_hi(dy));
+    const F2 uv0 = f2_mul(f2(w0), xy0), uv1 = f2_mul(f2(w1), xy1);
+    const F2 uv = f2_add(uv0, uv1);
+    const F2 uxy = f2_fma(f2(f2_lo(uv1)), xy1, f2_mul(f2(f2_lo(uv0)), xy0));
+    g[2] = f2_lo(uv);
+    g[3] = f2_hi(uv);
+    g[4] = f2_lo(uxy);
+    g[5] = f2_hi(uxy);
+    g[6] = __fmaf_rn(f2_hi(uv1), f2_hi(dy), __fmul_rn(f2_hi(uv0), f2_lo(dy)));
+    g[7] = __fadd_rn(w0, w1);
     return ok0 || ok1;
 }
 
-// Nine sums of a warp's two strips, added: the first level of the butterfly gives each half
-// of the warp one strip, which halves what the next levels exchange (21 shuffles; one strip
-// after the other takes 24).  Lane l ends with the total of value sum9_component(2 l) for l < 16.
-__device__ __forceinline__ float strip_pair_sum9(const float (&a)[9], const float (&b)[9])
+// Adds the warp's `count` pending steps over the lanes and into `acc`, in the order of
+// warp_transpose_sum9 (lanes 16 apart first, then 8, 4, 2, 1): eight lanes per step, of which
+// each takes four sums of every fourth lane (128-bit loads, packed adds) through the first
+// three levels; two exchanges halve the four sums a lane still holds.  The two strips of one
+// record are added to each other first.  kAtomic: two warps share a slot.
+// What bounds the backward is instructions issued (78% of the slots; about 125 per step of 32
+// lanes x 2 pixels).  A butterfly over one step's nine sums takes 12 shuffles and 46
+// instructions, this about 20 with the stores: with it, and with warps that do not wait for
+// one another at each batch, the backward of a 1237x823 view of 300K Gaussians takes 263 us
+// (308 before), of 2M at 1080p 465 (476), of 16 such views 7.07 ms (7.25), of six smaller
+// views 1.70 ms (2.03), of 10K at 256x256 50 us (62).  Two steps at a time, in half the shared
+// memory and with one more CTA per SM: 491 us at 2M.
+template <bool kAtomic>
+__device__ __forceinline__ void add_step_sums(const StepSums& u, float (*acc)[9], int count)
 {
-    const unsigned lane = threadIdx.x & 31;
-    const bool hi = lane & 16;
-    float v9[9], v5[5], v3[3], v2[2], v1[1];
+    const int lane = threadIdx.x & 31, step = lane >> 3, r = lane & 3, x = lane & 4;
+    __syncwarp();
+    const ulonglong2* A = reinterpret_cast<const ulonglong2*>(u.step[step].a[x >> 2]);
+    F2 v[4][2];
 #pragma unroll
-    for (int i = 0; i < 9; i++) v9[i] = (hi ? b[i] : a[i]) + __shfl_xor_sync(0xffffffffu, hi ? a[i] : b[i], 16);
-    sum9_level<5, 9>(v9, v5, lane, 8);
-    sum9_level<3, 5>(v5, v3, lane, 4);
-    sum9_level<2, 3>(v3, v2, lane, 2);
-    sum9_level<1, 2>(v2, v1, lane, 1);
-    return v1[0] + __shfl_xor_sync(0xffffffffu, v1[0], 16);
+    for (int k = 0; k < 4; k++) {
+        const ulonglong2 p = A[(r + 4 * k) ^ x], q = A[(r + 4 * k + 16) ^ x];
+        v[k][0] = f2_add(p.x, q.x);
+        v[k][1] = f2_add(p.y, q.y);
+    }
+    const float* B = u.step[step].b + (lane & 7);
+    float z = (B[0] + B[16]) + (B[8] + B[24]);
+    const int rec = u.rec[step];
+#pragma unroll
+    for (int c = 0; c < 2; c++) v[0][c] = f2_add(f2_add(v[0][c], v[2][c]), f2_add(v[1][c], v[3][c]));
+    const float v0 = f2_lo(v[0][0]), v1 = f2_hi(v[0][0]), v2 = f2_lo(v[0][1]), v3 = f2_hi(v[0][1]);
+    const bool b2 = r & 2, b1 = r & 1;
+    const float s0 = (b2 ? v2 : v0) + __shfl_xor_sync(0xffffffffu, b2 ? v0 : v2, 2);
+    const float s1 = (b2 ? v3 : v1) + __shfl_xor_sync(0xffffffffu, b2 ? v1 : v3, 2);
+    float tot = (b1 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b1 ? s0 : s1, 1);  // sum number lane & 7
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+    bool on = step < count;
+    if constexpr (!kAtomic) {
+        const int after = __shfl_down_sync(0xffffffffu, rec, 8), before = __shfl_up_sync(0xffffffffu, rec, 8);
+        const float t2 = __shfl_down_sync(0xffffffffu, tot, 8), z2 = __shfl_down_sync(0xffffffffu, z, 8);
+        if (step + 1 < count && after == rec) {
+            tot += t2;
+            z += z2;
+        }
+        if (step > 0 && before == rec) on = false;
+    }
+    if (on) {
+        float* dst = acc[rec];
+        if constexpr (kAtomic) {
+            atomicAdd(dst + (lane & 7), tot);
+            if ((lane & 7) == 0) atomicAdd(dst + 8, z);
+        } else {
+            dst[lane & 7] += tot;
+            if ((lane & 7) == 0) dst[8] += z;
+        }
+    }
+    __syncwarp();
 }
 
 // kConsistent: the exact-gradient backward mode (FGS_BACKWARD_CONSISTENT), a
 // compile-time switch so that the reference mode pays nothing for it per pixel.
 template <int PPT, int kBatch, bool kConsistent>
-__device__ __forceinline__ void render_bwd_tile(BwdSmemT<PPT, kBatch>& sm, const TileArgs& a, int tile, uint32_t& gb,
+__device__ __forceinline__ void render_bwd_tile(BwdSmem<PPT, kBatch>& sm, const TileArgs& a, int tile, uint32_t& gb,
                                                 unsigned* err)
 {
     constexpr int kSlots = bwd_slots<PPT>();
@@ -1308,6 +1377,8 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmemT<PPT, kBatch>& sm, const
         s.npy[q] = f2(-(float)(py0 + 4 * q), -(float)(py0 + 4 * q + 1));
 #pragma unroll
         for (int c = 0; c < 3; c++) s.d[q][c] = f2(d[0][c], d[1][c]);
+        s.d01[q][0] = f2(d[0][0], d[0][1]);
+        s.d01[q][1] = f2(d[1][0], d[1][1]);
     }
     // a gradient too large for the packed form (or not finite) sends the warp the other way
     const uint32_t wild_warp = __all_sync(0xffffffffu, tame) ? 0u : kWild;
@@ -1315,9 +1386,9 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmemT<PPT, kBatch>& sm, const
     const int mbit = PPT == 4 ? 4 * warp : 2 * (warp * PPT / 2);  // the first strip's bits in a block_mask
     const float ddelx_dx = 0.5 * W;
     const float ddely_dy = 0.5 * H;
-    // the component whose total each lane holds after warp_transpose_sum9, strip_pair_sum9
     const int q_lane = (lane & 1) ? 15 : sum9_component((unsigned)lane);
-    const int q_pair = lane < 16 ? sum9_component(2u * lane) : 15;
+    StepSums& steps = sm.step[PPT == 1 ? 0 : warp];
+    int pending = 0;
 
     if (tid == 0) sm.max_last = 0;
     __syncthreads();
@@ -1328,14 +1399,19 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmemT<PPT, kBatch>& sm, const
     const uint32_t n = min(range.y - range.x, sm.max_last);
     const int nb = (int)((n + kBatch - 1) / kBatch);
     // batch b holds entries [lo_b, hi_b) with hi_b = n - b*kBatch (back to front)
-    if (tid == 0) {
-        for (int b = 0; b < 2 && b < nb; b++) {
-            const uint32_t hi = n - b * kBatch, lo = hi > (uint32_t)kBatch ? hi - kBatch : 0;
-            const int buf = (int)((gb + b) % kBufs);
-            issue_batch(sm.rec[buf], &sm.bar[buf], recs, range.x + lo, hi - lo);
-        }
-    }
+    auto issue = [&](int b) {
+        const uint32_t hi = n - b * kBatch, lo = hi > (uint32_t)kBatch ? hi - kBatch : 0;
+        const int buf = (int)((gb + b) % kBufs);
+        issue_batch(sm.rec[buf], &sm.bar[buf], recs, range.x + lo, hi - lo);
+    };
+    if (tid == 0)
+        for (int b = 0; b < kBufs && b < nb; b++) issue(b);
 
+    // Warps go through the batches on their own: a batch's sums are written out by the warp
+    // that is through with it last, which then has the batch three later copied into its
+    // buffer; a warp that waits for that copy also knows that the sums it will add to are
+    // zero again.  (With the block waiting twice per batch of 32 a fifth of the warps' time
+    // went there.)
     for (int b = 0; b < nb; b++) {
         const uint32_t g = gb + b;
         const int buf = (int)(g % kBufs);
@@ -1348,7 +1424,7 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmemT<PPT, kBatch>& sm, const
             // this warp's strips, walked back to front
             const uint32_t e = (uint32_t)k0 + lane;
             const uint32_t mask = e < cnt && lo + e < warp_last ? __float_as_uint(R[e].c.z) >> mbit : 0u;
-            uint32_t strip[NP], live = 0, touched = 0;
+            uint32_t strip[NP], live = 0;
 #pragma unroll
             for (int q = 0; q < NP; q++) {
                 strip[q] = __ballot_sync(0xffffffffu, ((mask >> (2 * q)) & 3u) != 0);
@@ -1363,92 +1439,95 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmemT<PPT, kBatch>& sm, const
                 const float4 rb = R[j].b;
                 const float2 rc = make_float2(R[j].c.x, R[j].c.z);
                 const float dx = ra.x - pxf;
-                float g[NP][NG];
-                bool any[NP];
                 const bool branchy = PPT == 1 || ((__float_as_uint(rc.y) | wild_warp) & kWild);
                 const float sx = __fmul_rn(ra.z, dx), nbx = -__fmul_rn(ra.w, dx);
 #pragma unroll
                 for (int q = 0; q < NP; q++) {
-                    any[q] = false;
-#pragma unroll
-                    for (int i = 0; i < NG; i++) g[q][i] = 0.f;
                     if (NP > 1 && !((strip[q] >> bit) & 1u)) continue;
+                    float g[NG];
+                    bool any = false;
                     if (branchy) {
+#pragma unroll
+                        for (int i = 0; i < NG; i++) g[i] = 0.f;
 #pragma unroll
                         for (int h = 0; h < 2 && 2 * q + h < PPT; h++) {
                             auto half = [&](F2 x) { return h ? f2_hi(x) : f2_lo(x); };
                             float T = half(s.T[q]), acc = half(s.acc[q]);
-                            any[q] |= bwd_pixel_step<kConsistent>(
+                            any |= bwd_pixel_step<kConsistent>(
                                 ra, rb, rc.x, pxf, -half(s.npy[q]), contributor < s.last[2 * q + h], T, acc,
-                                half(s.d[q][0]), half(s.d[q][1]), half(s.d[q][2]), half(s.bgT[q]), g[q]);
+                                half(s.d[q][0]), half(s.d[q][1]), half(s.d[q][2]), half(s.bgT[q]), g);
                             s.T[q] = h ? f2(f2_lo(s.T[q]), T) : f2(T, f2_hi(s.T[q]));
                             s.acc[q] = h ? f2(f2_lo(s.acc[q]), acc) : f2(acc, f2_hi(s.acc[q]));
                         }
                     } else {
-                        any[q] = bwd_pair_step<kConsistent, NP>(s, q, ra, rb, rc.x, dx, sx, nbx, contributor, g[q]);
+                        any = bwd_pair_step<kConsistent, NP>(s, q, ra, rb, rc.x, dx, sx, nbx, contributor, g);
                     }
-                }
-                if constexpr (kOwnSlot) {
-                    const bool first = __any_sync(0xffffffffu, any[0]), second = __any_sync(0xffffffffu, any[1]);
-                    if (first || second) {
-                        float tot;
-                        int at = q_lane;
-                        if (first && second) {
-                            tot = strip_pair_sum9(g[0], g[1]);
-                            at = q_pair;
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < NG; i++) g[0][i] = first ? g[0][i] : g[1][i];
-                            tot = warp_transpose_sum9(g[0]);
+                    if (!__any_sync(0xffffffffu, any)) continue;
+                    if constexpr (PPT == 1) {
+                        const float tot = warp_transpose_sum9(g);
+                        if (q_lane < NG) atomicAdd(&sm.acc[buf][warp >> 1][j][q_lane], tot);
+                    } else {
+                        auto& st = steps.step[pending];
+                        st.a[0][lane] = make_float4(g[0], g[1], g[2], g[3]);
+                        st.a[1][lane ^ 4] = make_float4(g[4], g[5], g[6], g[7]);
+                        st.b[lane] = g[8];
+                        if (lane == 0) steps.rec[pending] = j;
+                        if (++pending == kPend) {
+                            add_step_sums<!kOwnSlot>(steps, sm.acc[buf][kOwnSlot ? warp : warp >> 1], kPend);
+                            pending = 0;
                         }
-                        touched |= 1u << bit;
-                        if (at < NG) sm.acc[warp][j][at] = tot;
                     }
-                } else if (__any_sync(0xffffffffu, any[0])) {
-                    const float tot = warp_transpose_sum9(g[0]);
-                    if (q_lane < NG) atomicAdd(&sm.acc[warp >> 1][j][q_lane], tot);
                 }
             }
-            if constexpr (kOwnSlot)
-                if (lane == 0) sm.live[warp][k0 >> 5] = touched;
         }
-        __syncthreads();
+        if (PPT > 1 && pending) {
+            add_step_sums<!kOwnSlot>(steps, sm.acc[buf][kOwnSlot ? warp : warp >> 1], pending);
+            pending = 0;
+        }
+        uint32_t through = 0;
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence_block();
+            through = atomicAdd(&sm.arrived[buf], 1u);
+            __threadfence_block();
+        }
+        if (__shfl_sync(0xffffffffu, through, 0) != NT / 32 - 1) continue;
         // this batch's per-pair gradients, at each pair's emission index: the slot sums times
         // the pair's own factors (opacity, conic, -W/2, -H/2, -1/2 of backward.cu:537-551)
-        for (uint32_t e = tid; e < cnt; e += NT) {
+        for (uint32_t e = lane; e < cnt; e += 32) {
             float* dst = a.pgrad + (size_t)__float_as_uint(R[e].c.w) * NG;
             float sum[NG];
 #pragma unroll
             for (int q = 0; q < NG; q++) sum[q] = 0.f;
 #pragma unroll
             for (int sl = 0; sl < kSlots; sl++) {
-                float* acc = sm.acc[sl][e];
-                if (kOwnSlot && !((sm.live[sl][e >> 5] >> (e & 31)) & 1u)) continue;
+                float* acc = sm.acc[buf][sl][e];
 #pragma unroll
                 for (int q = 0; q < NG; q++) {
                     sum[q] += acc[q];
-                    if (!kOwnSlot) acc[q] = 0.f;
+                    acc[q] = 0.f;
                 }
             }
             const float4 ea = R[e].a, eb = R[e].b;  // conic (ea.z, ea.w, eb.x), opacity eb.y
             const float o = eb.y;
             dst[0] = sum[0];
             dst[1] = sum[1];
-            dst[2] = sum[2];
-            dst[3] = -ddelx_dx * (o * (ea.z * sum[3] + ea.w * sum[4]));
-            dst[4] = -ddely_dy * (o * (eb.x * sum[4] + ea.w * sum[3]));
-            dst[5] = -0.5f * (o * sum[5]);
-            dst[6] = -0.5f * (o * sum[6]);
-            dst[7] = -0.5f * (o * sum[7]);
-            dst[8] = sum[8];
+            dst[2] = sum[8];
+            dst[3] = -ddelx_dx * (o * __fmaf_rn(ea.z, sum[2], __fmul_rn(ea.w, sum[3])));
+            dst[4] = -ddely_dy * (o * __fmaf_rn(eb.x, sum[3], __fmul_rn(ea.w, sum[2])));
+            dst[5] = -0.5f * (o * sum[4]);
+            dst[6] = -0.5f * (o * sum[5]);
+            dst[7] = -0.5f * (o * sum[6]);
+            dst[8] = sum[7];
         }
-        if (tid == 0 && b + 2 < nb) {
-            const int nbuf = (int)((g + 2) % kBufs);
-            const uint32_t hi2 = n - (b + 2) * kBatch, lo2 = hi2 > (uint32_t)kBatch ? hi2 - kBatch : 0;
-            issue_batch(sm.rec[nbuf], &sm.bar[nbuf], recs, range.x + lo2, hi2 - lo2);
+        __syncwarp();
+        if (lane == 0) {
+            sm.arrived[buf] = 0;
+            __threadfence_block();
+            if (b + kBufs < nb) issue(b + kBufs);
         }
-        __syncthreads();
     }
+    __syncthreads();  // (the buffers and counters are free for the next tile)
     gb += (uint32_t)nb;
     // pairs at or past the tile's largest n_contrib touch no pixel: zero gradients
     for (uint32_t e = n + tid; e < range.y - range.x; e += NT) {
@@ -1461,7 +1540,8 @@ __device__ __forceinline__ void render_bwd_tile(BwdSmemT<PPT, kBatch>& sm, const
 template <typename Smem>
 __device__ __forceinline__ void bwd_smem_init(Smem& sm, int NT)
 {
-    float* acc = &sm.acc[0][0][0];
+    float* acc = &sm.acc[0][0][0][0];
+    if (threadIdx.x < kBufs) sm.arrived[threadIdx.x] = 0;
     for (int e = threadIdx.x; e < (int)(sizeof(sm.acc) / sizeof(float)); e += NT) acc[e] = 0.f;
     if (threadIdx.x == 0) {
         for (int i = 0; i < kBufs; i++) mbar_init(&sm.bar[i], 1);
@@ -1470,20 +1550,18 @@ __device__ __forceinline__ void bwd_smem_init(Smem& sm, int NT)
     __syncthreads();
 }
 
-// Resident CTAs per SM the multi-view backward is compiled for: 32 warps at 2 pixels
-// per thread (64 registers, a few spilled bytes) and 24 at 4 (80 registers and a few
-// spilled bytes instead of the 110 the compiler takes when left alone; with 64-record
-// batches the shared memory then lets all 12 CTAs in).  Measured: 4 pixels per thread
-// at 12 CTAs beats 10 (no spills) and 14 (more spills); 2 at 8 beats 6.  The
+// Resident CTAs per SM the multi-view backward is compiled for: 28 warps at 2 pixels per
+// thread (what the shared memory of 32-record batches lets in) and 24 at 4 (80 registers and
+// a few spilled bytes instead of the 94 the compiler takes when left alone).  The
 // single-view kernel keeps the compiler's allocation.
 template <int PPT>
-constexpr int bwd_multi_min_ctas() { return PPT == 2 ? 8 : (PPT == 4 ? 12 : 1); }
+constexpr int bwd_multi_min_ctas() { return PPT == 2 ? 7 : (PPT == 4 ? 12 : 1); }
 
 template <int PPT, int kBatch, bool kConsistent>
 __global__ void __launch_bounds__(256 / PPT) render_bwd_kernel(TileArgs a, ZeroList zero, unsigned* err)
 {
     extern __shared__ __align__(128) unsigned char bwd_dyn[];
-    BwdSmemT<PPT, kBatch>& sm = *reinterpret_cast<BwdSmemT<PPT, kBatch>*>(bwd_dyn);
+    BwdSmem<PPT, kBatch>& sm = *reinterpret_cast<BwdSmem<PPT, kBatch>*>(bwd_dyn);
     bwd_smem_init(sm, 256 / PPT);
     uint32_t gb = 0;
     render_bwd_tile<PPT, kBatch, kConsistent>(sm, a, blockIdx.x, gb, err);
@@ -1494,28 +1572,21 @@ __global__ void __launch_bounds__(256 / PPT) render_bwd_kernel(TileArgs a, ZeroL
 template <int PPT, int kBatch, bool kConsistent>
 __global__ void __launch_bounds__(256 / PPT, bwd_multi_min_ctas<PPT>())
     render_bwd_multi_kernel(const TileArgs* __restrict__ views, const uint32_t* __restrict__ begin, int nviews,
-                            uint32_t total, uint32_t* queue, uint32_t min_tiles, uint32_t max_tiles, unsigned* err)
+                            uint32_t total, uint32_t* queue, unsigned* err)
 {
-    // the items are the tiles of the views of min_tiles .. max_tiles tiles (total of them)
     extern __shared__ __align__(128) unsigned char bwd_dyn[];
-    BwdSmemT<PPT, kBatch>& sm = *reinterpret_cast<BwdSmemT<PPT, kBatch>*>(bwd_dyn);
+    BwdSmem<PPT, kBatch>& sm = *reinterpret_cast<BwdSmem<PPT, kBatch>*>(bwd_dyn);
     __shared__ uint32_t s_item;
     bwd_smem_init(sm, 256 / PPT);
     uint32_t gb = 0;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(queue, 1u);
         __syncthreads();
-        uint32_t item = s_item;
+        const uint32_t item = s_item;
         if (item >= total) break;
-        int v = 0;
-        for (; v < nviews; v++) {
-            const uint32_t tiles = begin[v + 1] - begin[v];
-            if (tiles < min_tiles || tiles > max_tiles) continue;
-            if (item < tiles) break;
-            item -= tiles;
-        }
+        const int v = view_of(begin, nviews, item);
         const TileArgs& a = views[v];  // fields read where used, not held in registers
-        render_bwd_tile<PPT, kBatch, kConsistent>(sm, a, (int)item, gb, err);
+        render_bwd_tile<PPT, kBatch, kConsistent>(sm, a, (int)(item - begin[v]), gb, err);
         __syncthreads();
     }
 }
@@ -1621,7 +1692,7 @@ template <int PPT, int B, int Tag, typename Kern>
 size_t bwd_smem_bytes(Kern k)
 {
     static bool done[64] = {};
-    const size_t bytes = sizeof(BwdSmemT<PPT, B>);
+    const size_t bytes = sizeof(BwdSmem<PPT, B>);
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !done[dev]) {
@@ -1730,7 +1801,7 @@ void fwd_multi_launch(const TileArgs* views, const uint32_t* begin, int nviews, 
 
 template <int PPT, int B, bool kConsistent>
 void bwd_multi_launch_mode(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total, uint32_t* queue,
-                           uint32_t min_tiles, uint32_t max_tiles, unsigned* err, cudaStream_t s)
+                           unsigned* err, cudaStream_t s)
 {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
@@ -1740,17 +1811,17 @@ void bwd_multi_launch_mode(const TileArgs* views, const uint32_t* begin, int nvi
                                                   smem);
     const int grid = sms * (per_sm > 0 ? per_sm : 1);
     render_bwd_multi_kernel<PPT, B, kConsistent><<<grid, 256 / PPT, smem, s>>>(views, begin, nviews, total, queue,
-                                                                               min_tiles, max_tiles, err);
+                                                                               err);
 }
 
 template <int PPT, int B>
 void bwd_multi_launch(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total, uint32_t* queue,
-                      uint32_t min_tiles, uint32_t max_tiles, int consistent, unsigned* err, cudaStream_t s)
+                      int consistent, unsigned* err, cudaStream_t s)
 {
     if (consistent)
-        bwd_multi_launch_mode<PPT, B, true>(views, begin, nviews, total, queue, min_tiles, max_tiles, err, s);
+        bwd_multi_launch_mode<PPT, B, true>(views, begin, nviews, total, queue, err, s);
     else
-        bwd_multi_launch_mode<PPT, B, false>(views, begin, nviews, total, queue, min_tiles, max_tiles, err, s);
+        bwd_multi_launch_mode<PPT, B, false>(views, begin, nviews, total, queue, err, s);
 }
 }  // namespace
 
@@ -1775,53 +1846,34 @@ void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const
                         s);
 }
 
-namespace {
-// The backward's shape until a caller sets one: 4 pixels per lane and 64-record batches (two
-// warps per tile) for views whose tiles fill the GPU; for smaller ones, whose time is that of
-// their longest tiles, more and shorter warps: 2 pixels per lane and 128-record batches.
-// Measured, at 2 / at 4: 144 tiles 451 / 496 us, 920 tiles 164 / 205, 2304 tiles 184 / 201, 3600
-// tiles 234 / 235, 8160 tiles 395 / 372; but in a batch, where the other views' tiles fill the
-// GPU, 4 is 11% faster at any size, so the line lies where one view alone still gains 10%.  It
-// is drawn by the view's own tiles, alone and in a batch: a lane adds its pixels' terms in an
-// order that depends on the shape, and a batch's gradients equal the per-view ones bit for bit.
-constexpr uint32_t kSmallViewTiles = 2048;
-void bwd_rule(RenderConfig& c, bool small)
-{
-    if (c.own_shape) return;
-    c.bwd_ppt = small ? 2 : 4;
-    c.bwd_batch = small ? 128 : 64;
-}
-}  // namespace
+// The backward's shape until a caller sets one: 2 pixels per lane and 32-record batches.
+// The gradients' bits are those of every shape of 2 or 4 pixels per lane, so the choice is free
+// (tests/test_gpu_composite.py); measured, in us, at (2, 32) / (2, 64) / (4, 32): a view of 256 tiles
+// 50 / 49 / 81, 4056 tiles 263 / 274 / 279, 8160 tiles 465 / 493 / 452, 16 of these 7065 / 7703 /
+// 7218, six views of 1200 to 5700 tiles 1705 / 1745 / 2045.
+constexpr int kBwdRulePpt = 2, kBwdRuleBatch = 32;
 
-void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, const uint32_t* host_begin, int nviews,
+void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
                              uint32_t* queue, int consistent, unsigned* err, cudaStream_t s)
 {
-    cudaMemsetAsync(queue, 0, 2 * sizeof(uint32_t), s);
-    RenderConfig c = g_cfg;
-    // the views of either kind: one launch each (one for all when the caller set the shape)
-    uint32_t items[2] = {0, 0};
-    for (int v = 0; v < nviews; v++) {
-        const uint32_t tiles = host_begin[v + 1] - host_begin[v];
-        items[!c.own_shape && tiles <= kSmallViewTiles] += tiles;
-    }
-    for (int small = 0; small < 2; small++) {
-        if (!items[small]) continue;
-        bwd_rule(c, small != 0);
-        const uint32_t lo = small || c.own_shape ? 0u : kSmallViewTiles + 1, hi = small ? kSmallViewTiles : 0xffffffffu;
-        FGS_RENDER_DISPATCH(bwd_multi_launch, c.bwd_ppt, c.bwd_batch, views, begin, nviews, items[small],
-                            queue + small, lo, hi, consistent, err, s);
-        note_launches(1);
-    }
+    cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
+    if (!g_cfg.own_shape)
+        bwd_multi_launch<kBwdRulePpt, kBwdRuleBatch>(views, begin, nviews, total_tiles, queue, consistent, err, s);
+    else
+        FGS_RENDER_DISPATCH(bwd_multi_launch, g_cfg.bwd_ppt, g_cfg.bwd_batch, views, begin, nviews, total_tiles, queue,
+                            consistent, err, s);
+    note_launches(1);
 }
 
 void launch_render_bwd(int W, int H, const ImageState& im, const BinState& b, const float* bg,
                        const float* dL_dpix, int consistent, const ZeroList& zero, unsigned* err, cudaStream_t s)
 {
     const int gx = (W + kTileX - 1) / kTileX, gy = (H + kTileY - 1) / kTileY;
-    RenderConfig c = g_cfg;
-    bwd_rule(c, (uint32_t)(gx * gy) <= kSmallViewTiles);
-    FGS_RENDER_DISPATCH(bwd_launch, c.bwd_ppt, c.bwd_batch, gx * gy, im, b, W, H, bg, dL_dpix, consistent, zero, err,
-                        s);
+    if (!g_cfg.own_shape)
+        bwd_launch<kBwdRulePpt, kBwdRuleBatch>(gx * gy, im, b, W, H, bg, dL_dpix, consistent, zero, err, s);
+    else
+        FGS_RENDER_DISPATCH(bwd_launch, g_cfg.bwd_ppt, g_cfg.bwd_batch, gx * gy, im, b, W, H, bg, dL_dpix, consistent,
+                            zero, err, s);
     note_launches(1);
 }
 

@@ -1,12 +1,11 @@
 """The compositing's record masks and warp sums, replayed on the CPU from their definitions in
-csrc/fgs_common.cuh (block_mask) and csrc/render.cu (strip_pair_sum9).
+csrc/fgs_common.cuh (block_mask) and csrc/render.cu (add_step_sums).
 
 * block_mask against every pixel of a tile: an 8x4 block outside the mask must have no pixel whose
   alpha, evaluated in float32 as the compositing does, reaches 1/255 -- over round, elongated
   (up to 1000:1) and degenerate conics, opacities down to 1/255 and means inside and around the
   tile.  It must also leave out most of the blocks that are not reached.
-* strip_pair_sum9: every component's total lands on the lane that the table names, with the bits of
-  the two strips' totals added.
+* add_step_sums: the totals of four steps, each with the bits of warp_transpose_sum9.
 """
 import os
 import re
@@ -111,23 +110,29 @@ def _sum9(v):
     return v[0] + v[0][np.arange(32) ^ 1]
 
 
-def test_strip_pair_sum9_has_the_bits_of_two_strips_added():
+def test_add_step_sums_has_the_bits_of_warp_transpose_sum9():
     rng = np.random.default_rng(5)
-    a, b = rng.standard_normal((2, 9, 32)).astype(F)
+    g = rng.standard_normal((4, 9, 32)).astype(F)    # four steps' sums of every lane
     lanes = np.arange(32)
-    hi = (lanes & 16) != 0
-    v = [np.where(hi, b[i], a[i]) + np.where(hi, a[i], b[i])[lanes ^ 16] for i in range(9)]
-    for m, o in ((5, 8), (3, 4), (2, 2), (1, 1)):
-        v = _level(v, m, o)
-    pair = v[0] + v[0][lanes ^ 16]
+    step, r, x = lanes >> 3, lanes & 3, lanes & 4
+    # the staged sums: a[step][half][place][i] holds sum 4 half + i of lane place ^ (4 half)
+    a = np.stack([np.stack([g[s, 4 * h:4 * h + 4, lanes ^ (4 * h)] for h in (0, 1)]) for s in range(4)])
+    at = lambda k: a[step, x >> 2, (r + 4 * k) ^ x]  # noqa: E731
+    v = [at(k) + at(k + 4) for k in range(4)]
+    v = (v[0] + v[2]) + (v[1] + v[3])
+    hi2, hi1 = (r & 2) != 0, (r & 1) != 0
+    s = [np.where(hi2, v[:, 2 + i], v[:, i]) + np.where(hi2, v[:, i], v[:, 2 + i])[lanes ^ 2] for i in (0, 1)]
+    tot = np.where(hi1, s[1], s[0]) + np.where(hi1, s[0], s[1])[lanes ^ 1]
+    b = lambda k: g[step, 8, (lanes & 7) + 8 * k]  # noqa: E731
+    z = (b(0) + b(2)) + (b(1) + b(3))
+    for o in (4, 2, 1):
+        z = z + z[lanes ^ o]
     src = open(os.path.join(CSRC, "fgs_common.cuh")).read()
     table = int(re.search(r"int sum9_component\(unsigned lane\).*?\(0x([0-9a-f]+)ull", src, re.S).group(1), 16)
-    one, two = _sum9(list(a)), _sum9(list(b))
-    seen = []
-    for lane in range(16):
-        q = (table >> (4 * lane)) & 15
-        if q < 9:
-            seen.append(q)
-            assert pair[lane] == one[2 * lane] + two[2 * lane], (lane, q)
-            assert np.isclose(pair[lane], a[q].sum(dtype=np.float64) + b[q].sum(dtype=np.float64), rtol=1e-5, atol=1e-5)
-    assert sorted(seen) == list(range(9))
+    place = {(table >> (4 * i)) & 15: 2 * i for i in range(16)}
+    for k in range(4):
+        want = _sum9(list(g[k]))
+        for q in range(8):
+            assert tot[8 * k + q] == want[place[q]], (k, q)
+        assert z[8 * k] == want[place[8]], k
+        assert np.allclose(want[[place[q] for q in range(9)]], g[k].sum(1, dtype=np.float64), rtol=1e-5, atol=1e-5)

@@ -180,14 +180,52 @@ print("rule ok", lengths)
 """
 
 
-def test_launch_rule_gives_the_same_bits(cuda):
-    """The shapes and the long tiles the launch rule picks (before any set_render_* call, so in a process
-    of its own) against one pixel per lane without bands: one view and batched, with and without
-    statistics, with long tiles of small splats, of large ones, and without any."""
+def _own_process(code):
     import os
     import subprocess
     import sys
     here = os.path.dirname(os.path.abspath(__file__))
-    code = _RULE.format(path=[here, os.path.dirname(here)])
-    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", code.format(path=[here, os.path.dirname(here)])], capture_output=True,
+                       text=True, timeout=300)
     assert r.returncode == 0 and "rule ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def test_launch_rule_gives_the_same_bits(cuda):
+    """The shapes and the long tiles the launch rule picks (before any set_render_* call, so in a process
+    of its own) against one pixel per lane without bands: one view and batched, with and without
+    statistics, with long tiles of small splats, of large ones, and without any."""
+    _own_process(_RULE)
+
+
+_BWD = """
+import sys
+import numpy as np, torch
+sys.path[:0] = {path!r}
+from _helpers import Case, S, ours, run_backward, run_forward
+from filtergs_b200 import _lib
+
+def case(P, W, H, **kw):
+    sc, cam = S.small_scene(P=P, seed=78, W=W, H=H)
+    sc["means3D"][: P // 2, :2] *= 0.1
+    return Case(sc, cam, **kw)
+
+cases = [case(1, 16, 16), case(60, 16, 16), case(9000, 333, 140, bg=np.array([0.2, 0.5, 0.9], np.float32)),
+         case(3000, 147, 133)]
+dL = [torch.randn(3, c.cam.H, c.cam.W, device="cuda", generator=torch.Generator("cuda").manual_seed(3)) for c in cases]
+runs = [(c, d, m) for c, d in zip(cases, dL) for m in ("ref_compat", "consistent")]
+grads = lambda: [run_backward(ours, c, run_forward(ours, c), d, backward_mode=m) for c, d, m in runs]  # noqa: E731
+want = grads()
+assert all(float(g[3].abs().sum()) > 0 for g in want)
+for ppt, batch in ((2, 64), (2, 256), (4, 64), (4, 128)):
+    _lib.set_render_config(2, 128, ppt, batch)
+    for x, y in zip(grads(), want):
+        for k, (u, v) in enumerate(zip(x, y)):
+            assert torch.equal(u, v), (ppt, batch, k)
+print("rule ok")
+"""
+
+
+def test_backward_has_the_same_bits_in_every_shape(cuda):
+    """Gradients of the default backward shape and of others of 2 and 4 pixels per lane: one record, a
+    last batch that is not full, lists of many batches, images whose edges cut tiles, either mode."""
+    _own_process(_BWD)
