@@ -604,24 +604,53 @@ __global__ void __launch_bounds__(128, 4)
     }
 }
 
-// The Gaussians some view saw (any vis bit set), appended in any order to list
-// (count[0] entries; the caller zeroes count).
+// The Gaussians some view saw (any vis bit set), appended in any order to list (count[0]
+// entries; the caller zeroes count).  A block appends those of 2048 Gaussians at once: with an
+// addition to the one counter per warp of 32, these additions were all of the time (4M
+// Gaussians, 85 us; 12 now).
+constexpr int kSeenPer = 8;
 __global__ void __launch_bounds__(256)
     seen_list_kernel(const uint32_t* __restrict__ vis, int words, int P, uint32_t* __restrict__ list,
                      unsigned long long* __restrict__ count)
 {
-    const int lane = threadIdx.x & 31;
-    for (int base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; base < P; base += gridDim.x * blockDim.x) {
-        const int i = base + lane;
-        bool any = false;
-        if (i < P)
-            for (int w = 0; w < words && !any; w++) any = vis[(size_t)w * P + i] != 0;
-        const uint32_t b = __ballot_sync(0xffffffffu, any);
-        if (!b) continue;
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(count, (unsigned long long)__popc(b));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (any) list[at + __popc(b & ((1u << lane) - 1))] = (uint32_t)i;
+    __shared__ uint32_t s_n[8 * kSeenPer];
+    __shared__ unsigned long long s_at;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (size_t base = (size_t)blockIdx.x * (256 * kSeenPer); base < (size_t)P; base += (size_t)gridDim.x * (256 * kSeenPer)) {
+        uint32_t any[kSeenPer], b[kSeenPer];
+#pragma unroll
+        for (int u = 0; u < kSeenPer; u++) {
+            const size_t i = base + u * 256 + threadIdx.x;
+            any[u] = i < (size_t)P ? vis[i] : 0u;
+        }
+        for (int w = 1; w < words; w++)
+#pragma unroll
+            for (int u = 0; u < kSeenPer; u++) {
+                const size_t i = base + u * 256 + threadIdx.x;
+                if (i < (size_t)P) any[u] |= vis[(size_t)w * P + i];
+            }
+#pragma unroll
+        for (int u = 0; u < kSeenPer; u++) {
+            b[u] = __ballot_sync(0xffffffffu, any[u] != 0);
+            if (lane == 0) s_n[8 * u + warp] = __popc(b[u]);
+        }
+        __syncthreads();
+        uint32_t total = 0, before[kSeenPer];
+#pragma unroll
+        for (int u = 0; u < kSeenPer; u++)
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                if (w == warp) before[u] = total;
+                total += s_n[8 * u + w];
+            }
+        if (threadIdx.x == 0 && total) s_at = atomicAdd(count, (unsigned long long)total);
+        __syncthreads();
+        const unsigned long long at = s_at;
+#pragma unroll
+        for (int u = 0; u < kSeenPer; u++)
+            if (any[u])
+                list[at + before[u] + __popc(b[u] & ((1u << lane) - 1u))] = (uint32_t)(base + u * 256 + threadIdx.x);
+        __syncthreads();  // s_n and s_at are written again
     }
 }
 
@@ -654,7 +683,7 @@ void fold_launch(const FoldView* views, const FoldView& single, int nviews, int 
 
 // One launch instead of a memset per buffer: a launch costs about 2 us of a small view's chain
 // each, and a large buffer is written at the memory's rate either way.
-__global__ void __launch_bounds__(256) zero_kernel(ZeroList z) { zero_share(z, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(256) zero_kernel(ZeroList z) { zero_share(z, blockIdx.x); }
 
 }  // namespace
 
@@ -663,7 +692,8 @@ void launch_zero(const ZeroList& z, cudaStream_t s)
     size_t words = 0;
     for (int b = 0; b < z.n; b++) words += z.words[b];
     if (!words) return;
-    zero_kernel<<<grid_for(words / 4 + 1, 8), 256, 0, s>>>(z);
+    const int grid = grid_for(words / 4 + 1, 8);
+    zero_kernel<<<grid, 256, 0, s>>>(ZeroList(z).split((size_t)grid));
     note_launches(1);
 }
 
@@ -701,7 +731,7 @@ void launch_fold_bwd(const FoldView* views, int nviews, int P, const uint32_t* v
 {
     if (P <= 0 || nviews <= 0) return;
     cudaMemsetAsync(count, 0, sizeof(unsigned long long), s);
-    seen_list_kernel<<<grid_for((size_t)P, 8), 256, 0, s>>>(vis, (nviews + 31) >> 5, P, list, count);
+    seen_list_kernel<<<grid_for(((size_t)P + kSeenPer - 1) / kSeenPer, 8), 256, 0, s>>>(vis, (nviews + 31) >> 5, P, list, count);
     note_launches(1);
     fold_launch(views, shared, nviews, P, list, count, (size_t)P, vis, consistent, sh, dmean3D, dopac, nullptr, dsh,
                 dscale, drot, dens, s);

@@ -396,29 +396,28 @@ int fgs_batch_backward(void* handle, void* stream)
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t P = (size_t)B->P;
     if (!B->g_means3D || !B->g_opacity) return FGS_ERR_ARG;
+    // the shared outputs are zeroed by the compositing's launch (the fold writes the rows of
+    // the Gaussians some view saw), as are the views' visibility bits
+    const bool sh = B->views[0].pre.shs && B->g_sh;
+    ZeroList zero;
+    zero.add(B->d_vis, sizeof(uint32_t) * (size_t)B->vis_words * P);
+    zero.add(B->g_means3D, sizeof(float) * 3 * P);
+    zero.add(B->g_opacity, sizeof(float) * P);
+    if (sh) zero.add(B->g_sh, sizeof(float) * 3 * (size_t)B->M * P);
+    if (B->has_sr) zero.add(B->g_scales, sizeof(float) * 3 * P);
+    if (B->has_sr) zero.add(B->g_rot, sizeof(float) * 4 * P);
     {
         StageTimer t(FGS_STAGE_RENDER_BWD, s);
-        launch_render_bwd_multi(B->d_args_bwd, B->d_begin, B->V, B->total_tiles, B->d_queue + 1, B->consistent,
+        launch_render_bwd_multi(B->d_args_bwd, B->d_begin, B->V, B->total_tiles, B->d_queue + 1, zero, B->consistent,
                                 B->d_err, s);
     }
     StageTimer t(FGS_STAGE_PREPROCESS_BWD, s);
     // Each view's screen-space gradients (the sums of its per-pair rows) and the
     // views that saw each Gaussian, the views spread over the front-end streams;
     // then one pass per Gaussian over all views writes every gradient row once.
-    cudaMemsetAsync(B->d_vis, 0, sizeof(uint32_t) * (size_t)B->vis_words * P, s);
     const int ns = (int)B->aux.size();
     if (cudaEventRecord(B->forked, s) != cudaSuccess) return FGS_ERR_CUDA;
     for (int i = 0; i < ns; i++) cudaStreamWaitEvent(B->aux[i], B->forked, 0);
-    // the shared outputs are zeroed while the gathers run (the fold writes the rows of
-    // the Gaussians some view saw)
-    const bool sh = B->views[0].pre.shs && B->g_sh;
-    ZeroList zero;
-    zero.add(B->g_means3D, sizeof(float) * 3 * P);
-    zero.add(B->g_opacity, sizeof(float) * P);
-    if (sh) zero.add(B->g_sh, sizeof(float) * 3 * (size_t)B->M * P);
-    if (B->has_sr) zero.add(B->g_scales, sizeof(float) * 3 * P);
-    if (B->has_sr) zero.add(B->g_rot, sizeof(float) * 4 * P);
-    launch_zero(zero, s);
     for (int vi = 0; vi < B->V; vi++) {
         ViewState& v = B->views[vi];
         launch_pair_grad_gather(v.g, v.b.pgrad, v.cap, v.dmean2D, v.dconic, v.dcolor, v.dopac,

@@ -120,6 +120,7 @@ struct ZeroList {
     static constexpr int kMax = 10;
     void* p[kMax];
     size_t words[kMax];
+    size_t share[kMax];  // 16-byte items per part (split)
     int n = 0;
     void add(void* ptr, size_t bytes)
     {
@@ -127,25 +128,34 @@ struct ZeroList {
         p[n] = ptr;
         words[n++] = bytes / 4;
     }
+    // Divided here: as 64-bit divisions of every thread the shares cost a 1080p view's backward
+    // more than the stores.
+    ZeroList& split(size_t parts)
+    {
+        for (int b = 0; b < n; b++) share[b] = (words[b] / 4 + parts) / parts;
+        return *this;
+    }
 };
 void launch_zero(const ZeroList& z, cudaStream_t s);
 #ifdef __CUDACC__
-// Block `part` of `parts` zeroes its share of every buffer: a run of whole 16-byte items, and the first
-// and last blocks the words before the first 16-byte boundary and after the last.
-__device__ __forceinline__ void zero_share(const ZeroList& z, uint32_t part, uint32_t parts)
+// Block `part` of the `parts` that z was split for zeroes its share of every buffer: a run of whole
+// 16-byte items, and the first block the words before the first 16-byte boundary and after the last.
+__device__ __forceinline__ void zero_share(const ZeroList& z, uint32_t part)
 {
     for (int b = 0; b < z.n; b++) {
         uint32_t* p = static_cast<uint32_t*>(z.p[b]);
         const size_t n = z.words[b];
         size_t head = ((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / 4;
         if (head > n) head = n;
-        const size_t items = (n - head) / 4;
-        const size_t i1 = items * (part + 1) / parts;
+        const size_t items = (n - head) / 4, i0 = z.share[b] * part;
+        const size_t i1 = i0 + z.share[b] < items ? i0 + z.share[b] : items;
         uint4* q = reinterpret_cast<uint4*>(p + head);
-        for (size_t i = items * part / parts + threadIdx.x; i < i1; i += blockDim.x) q[i] = make_uint4(0, 0, 0, 0);
-        if (part == 0 && threadIdx.x < head) p[threadIdx.x] = 0;
-        const size_t tail = head + 4 * items;
-        if (part == parts - 1 && threadIdx.x < n - tail) p[tail + threadIdx.x] = 0;
+        for (size_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) q[i] = make_uint4(0, 0, 0, 0);
+        if (part == 0) {
+            if (threadIdx.x < head) p[threadIdx.x] = 0;
+            const size_t tail = head + 4 * items;
+            if (threadIdx.x < n - tail) p[tail + threadIdx.x] = 0;
+        }
     }
 }
 #endif
@@ -262,8 +272,9 @@ struct TileArgs {
 void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const uint32_t* begin, int nviews,
                              uint32_t total_tiles, uint32_t* queue, uint32_t* long_list, uint32_t* long_ctr,
                              unsigned* err, cudaStream_t s);
+// zero: buffers that this launch zeroes, a share after each tile: its stores pass while others composite.
 void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
-                             uint32_t* queue, int consistent, unsigned* err, cudaStream_t s);
+                             uint32_t* queue, const ZeroList& zero, int consistent, unsigned* err, cudaStream_t s);
 
 // Render kernel shape: pixels per thread {1,2,4} and records per shared-memory batch {64,128,256}.
 struct RenderConfig {

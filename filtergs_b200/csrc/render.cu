@@ -1566,14 +1566,15 @@ __global__ void __launch_bounds__(256 / PPT) render_bwd_kernel(TileArgs a, ZeroL
     uint32_t gb = 0;
     render_bwd_tile<PPT, kBatch, kConsistent>(sm, a, blockIdx.x, gb, err);
     // last, so that the first blocks composite while later ones have not yet anything to store
-    zero_share(zero, blockIdx.x, gridDim.x);
+    zero_share(zero, blockIdx.x);
 }
 
 template <int PPT, int kBatch, bool kConsistent>
 __global__ void __launch_bounds__(256 / PPT, bwd_multi_min_ctas<PPT>())
     render_bwd_multi_kernel(const TileArgs* __restrict__ views, const uint32_t* __restrict__ begin, int nviews,
-                            uint32_t total, uint32_t* queue, unsigned* err)
+                            uint32_t total, uint32_t* queue, ZeroList zero, int zero_shift, unsigned* err)
 {
+    // (a share of `zero` after one tile in 1 << zero_shift)
     extern __shared__ __align__(128) unsigned char bwd_dyn[];
     BwdSmem<PPT, kBatch>& sm = *reinterpret_cast<BwdSmem<PPT, kBatch>*>(bwd_dyn);
     __shared__ uint32_t s_item;
@@ -1587,6 +1588,7 @@ __global__ void __launch_bounds__(256 / PPT, bwd_multi_min_ctas<PPT>())
         const int v = view_of(begin, nviews, item);
         const TileArgs& a = views[v];  // fields read where used, not held in registers
         render_bwd_tile<PPT, kBatch, kConsistent>(sm, a, (int)(item - begin[v]), gb, err);
+        if (!(item & ((1u << zero_shift) - 1u))) zero_share(zero, item >> zero_shift);
         __syncthreads();
     }
 }
@@ -1712,10 +1714,10 @@ void bwd_launch(int grid, const ImageState& im, const BinState& b, int W, int H,
     a.dL_dpix = dL; a.pgrad = b.pgrad;
     if (consistent) {
         const size_t smem = bwd_smem_bytes<PPT, B, 2>(render_bwd_kernel<PPT, B, true>);
-        render_bwd_kernel<PPT, B, true><<<grid, 256 / PPT, smem, s>>>(a, zero, err);
+        render_bwd_kernel<PPT, B, true><<<grid, 256 / PPT, smem, s>>>(a, ZeroList(zero).split((size_t)grid), err);
     } else {
         const size_t smem = bwd_smem_bytes<PPT, B, 0>(render_bwd_kernel<PPT, B, false>);
-        render_bwd_kernel<PPT, B, false><<<grid, 256 / PPT, smem, s>>>(a, zero, err);
+        render_bwd_kernel<PPT, B, false><<<grid, 256 / PPT, smem, s>>>(a, ZeroList(zero).split((size_t)grid), err);
     }
 }
 
@@ -1801,7 +1803,7 @@ void fwd_multi_launch(const TileArgs* views, const uint32_t* begin, int nviews, 
 
 template <int PPT, int B, bool kConsistent>
 void bwd_multi_launch_mode(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total, uint32_t* queue,
-                           unsigned* err, cudaStream_t s)
+                           const ZeroList& zero, unsigned* err, cudaStream_t s)
 {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
@@ -1810,18 +1812,21 @@ void bwd_multi_launch_mode(const TileArgs* views, const uint32_t* begin, int nvi
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, render_bwd_multi_kernel<PPT, B, kConsistent>, 256 / PPT,
                                                   smem);
     const int grid = sms * (per_sm > 0 ? per_sm : 1);
-    render_bwd_multi_kernel<PPT, B, kConsistent><<<grid, 256 / PPT, smem, s>>>(views, begin, nviews, total, queue,
-                                                                               err);
+    int shift = 0;
+    while (shift < 4 && (total >> (shift + 1)) >= 4u * (uint32_t)grid) shift++;
+    const size_t parts = (total + (1u << shift) - 1u) >> shift;
+    render_bwd_multi_kernel<PPT, B, kConsistent><<<grid, 256 / PPT, smem, s>>>(
+        views, begin, nviews, total, queue, ZeroList(zero).split(parts), shift, err);
 }
 
 template <int PPT, int B>
 void bwd_multi_launch(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total, uint32_t* queue,
-                      int consistent, unsigned* err, cudaStream_t s)
+                      const ZeroList& zero, int consistent, unsigned* err, cudaStream_t s)
 {
     if (consistent)
-        bwd_multi_launch_mode<PPT, B, true>(views, begin, nviews, total, queue, err, s);
+        bwd_multi_launch_mode<PPT, B, true>(views, begin, nviews, total, queue, zero, err, s);
     else
-        bwd_multi_launch_mode<PPT, B, false>(views, begin, nviews, total, queue, err, s);
+        bwd_multi_launch_mode<PPT, B, false>(views, begin, nviews, total, queue, zero, err, s);
 }
 }  // namespace
 
@@ -1854,14 +1859,15 @@ void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const
 constexpr int kBwdRulePpt = 2, kBwdRuleBatch = 32;
 
 void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
-                             uint32_t* queue, int consistent, unsigned* err, cudaStream_t s)
+                             uint32_t* queue, const ZeroList& zero, int consistent, unsigned* err, cudaStream_t s)
 {
     cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
     if (!g_cfg.own_shape)
-        bwd_multi_launch<kBwdRulePpt, kBwdRuleBatch>(views, begin, nviews, total_tiles, queue, consistent, err, s);
+        bwd_multi_launch<kBwdRulePpt, kBwdRuleBatch>(views, begin, nviews, total_tiles, queue, zero, consistent, err,
+                                                     s);
     else
         FGS_RENDER_DISPATCH(bwd_multi_launch, g_cfg.bwd_ppt, g_cfg.bwd_batch, views, begin, nviews, total_tiles, queue,
-                            consistent, err, s);
+                            zero, consistent, err, s);
     note_launches(1);
 }
 
