@@ -140,103 +140,147 @@ __device__ __forceinline__ void load_sh_row(const float* __restrict__ shrow, int
 
 // Screen-space gradients of the visible Gaussians: the sum of each Gaussian's
 // per-pair gradients (pgrad rows at its emission indices, its tiles row-major).
-// Gaussians are taken in depth rank j, whose pairs are the contiguous rows
-// [pair_off[j], pair_off[j + 1]) (the last ends at K), so a warp reads its next
-// Gaussian's row range while it sums the current one.  One warp per Gaussian:
-// lane l takes rows l, l+32, ... (coalesced 36-byte rows, 64 rows in flight per
-// round trip, so a splat over thousands of tiles does not stall the kernel) and a
-// fixed shuffle tree adds them, 32 rows at a time in emission order -- the same
-// sum on every run.  Two Gaussians of at most 32 rows each (the common case) share
-// one round trip.  Row layout: dcolor r,g,b | dmean2D x,y | dconic x,y,w |
-// dopacity.  vis (optional): the view sets vis_bit in vis[idx] for every Gaussian
-// it sees.  Compiled for 4 blocks per SM (64 registers; measured faster than the
-// compiler's 76 with fewer warps).
-__global__ void __launch_bounds__(256, 4)
+// Gaussians are taken by depth rank j, whose pairs are the contiguous rows
+// [pair_off[j], pair_off[j + 1]) (the last ends at K).  A block copies the rows of 16 Gaussians
+// to shared memory (up to kGatherRows at a time), and a thread per (Gaussian, component)
+// adds them from there, 32 at a time in the order of warp_transpose_sum9 (rows 16 apart
+// first, then 8, 4, 2, 1; missing rows are zeros), the groups added to 0 in turn: the same sum on
+// every run.  A Gaussian with more rows than that is summed by all warps from memory.  The
+// 16 are four runs of four ranks a quarter of the view apart, because the nearest Gaussians are the largest:
+// in a run of 16 ranks the first block had seven of more than 512 rows, and the kernel
+// waited for it.  Row layout: dcolor r,g,b | dmean2D x,y | dconic x,y,w | dopacity.  vis
+// (optional): the view sets vis_bit in vis[idx] for every Gaussian it sees.
+// Bound by the latency of the copies and the scattered stores.  131K Gaussians with 2.1M rows
+// (75 MB): 49 us, 10K with 90K rows 4; with a warp per Gaussian, a row per lane and a
+// shuffle tree per 32 rows 74 and 23.
+constexpr int kGatherRanks = 16, kGatherRun = 4, kGatherRows = 512, kGatherThreads = 160;
+static_assert(kGatherThreads >= 9 * kGatherRanks, "a thread per Gaussian and component");
+__global__ void __launch_bounds__(kGatherThreads, 8)
     pair_grad_gather_kernel(const uint32_t* __restrict__ visible_ids, const unsigned long long* __restrict__ totals,
                             const uint32_t* __restrict__ pair_off, const float* __restrict__ pgrad,
                             float* __restrict__ dmean2D, float* __restrict__ dconic, float* __restrict__ dcolor,
                             float* __restrict__ dopac, uint32_t* __restrict__ vis, uint32_t vis_bit, uint32_t rows)
 {
+    __shared__ float s_f[kGatherRows * 9];
+    __shared__ uint32_t s_e0[kGatherRanks], s_ne[kGatherRanks], s_at[kGatherRanks];
+    __shared__ int s_id[kGatherRanks];
     const uint32_t K = (uint32_t)totals[0], V = (uint32_t)totals[1];
-    const int lane = threadIdx.x & 31;
-    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-    uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    // rows past `rows` (a batched view truncated at its pair capacity) were never
-    // written: each range is clamped to the buffer
-    auto range = [&](uint32_t jj, uint32_t& e0, uint32_t& e1, int& idx) {
-        e0 = min(__ldg(pair_off + jj), rows);
-        e1 = max(e0, min(jj + 1 < V ? __ldg(pair_off + jj + 1) : K, rows));
-        idx = (int)__ldg(visible_ids + jj);
+    const int tid = threadIdx.x, lane = tid & 31;
+    auto store = [&](int idx, int q, float acc) {
+        if (vis && q == 0) atomicOr(vis + idx, vis_bit);  // this view sees Gaussian idx
+        float* dst = q < 3 ? dcolor + 3 * (size_t)idx + q
+                   : q < 5 ? dmean2D + 3 * (size_t)idx + (q - 3)
+                   : q == 7 ? dconic + 4 * (size_t)idx + 3
+                   : q < 8 ? dconic + 4 * (size_t)idx + (q - 5)
+                           : dopac + idx;
+        *dst = acc;
     };
-    // sum of rows [e0, e1), component sum9_component(lane) on each lane: 32 rows at a time in
-    // emission order, each group through the same shuffle tree, added to 0 in turn
-    auto sum_rows = [&](uint32_t e0, uint32_t e1) {
-        const uint32_t ne = e1 - e0;
-        float acc = 0.f;
-        for (uint32_t k = 0; k < ne; k += 64) {
-            float v[2][9];
+    const uint32_t nch = (V + kGatherRanks - 1) / kGatherRanks;
+    uint32_t ne_next = 0, e0_next = 0;
+    int id_next = -1;  // no Gaussian
+    auto fetch = [&](uint32_t c) {
+        ne_next = e0_next = 0;
+        id_next = -1;
+        const uint32_t j = (c + tid / kGatherRun * nch) * kGatherRun + tid % kGatherRun;
+        if (tid >= kGatherRanks || c >= nch || j >= V) return;
+        // rows past `rows` (a batched view truncated at its pair capacity) were never
+        // written: each range is clamped to the buffer
+        e0_next = min(__ldg(pair_off + j), rows);
+        ne_next = max(e0_next, min(j + 1 < V ? __ldg(pair_off + j + 1) : K, rows)) - e0_next;
+        id_next = (int)__ldg(visible_ids + j);
+    };
+    fetch(blockIdx.x);
+    constexpr uint32_t m = kGatherRanks;
+    for (uint32_t c0 = blockIdx.x; c0 < nch; c0 += gridDim.x) {
+        if (tid < kGatherRanks) {
+            s_e0[tid] = e0_next;
+            s_ne[tid] = ne_next;
+            s_id[tid] = id_next;
+        }
+        __syncthreads();
+        fetch(c0 + gridDim.x);  // in flight meanwhile
+        for (uint32_t g = 0; g < m;) {
+            // the Gaussians from g on whose rows fit, and where each one's start (the same on
+            // every warp)
+            const uint32_t e0 = s_e0[g];
+            const uint32_t mine = (uint32_t)lane >= g && (uint32_t)lane < m ? s_ne[lane] : 0u;
+            unsigned long long upto = mine;
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                if (k + 32 * u >= ne) continue;  // (warp-uniform) no rows in this group
-                const uint32_t r = k + 32 * u + lane;
-                const float* src = pgrad + (size_t)(e0 + r) * 9;
-#pragma unroll
-                for (int q = 0; q < 9; q++) v[u][q] = r < ne ? __ldg(src + q) : 0.f;
+            for (int o = 1; o < kGatherRanks; o <<= 1) {
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += y;
             }
+            const bool fits = (uint32_t)lane >= g && (uint32_t)lane < m && upto <= (unsigned long long)kGatherRows;
+            const uint32_t h = g + __popc(__ballot_sync(0xffffffffu, fits));
+            if (fits && tid < 32) s_at[lane] = (uint32_t)upto - mine;
+            if (h == g) {
+                // more rows than that: every warp adds 64 of them at a time from memory, and the
+                // 32-row groups' sums are added in turn
+                const uint32_t ne = s_ne[g];
+                const int q = sum9_component(lane);
+                float acc = 0.f;
+                for (uint32_t k0 = 0; k0 < ne; k0 += 32 * kGatherRows) {
+                    const uint32_t groups = (min(ne - k0, 32u * kGatherRows) + 31) / 32;
+                    for (uint32_t c = 2 * (tid >> 5); c < groups; c += 2 * (kGatherThreads / 32)) {
+                        float v[2][9];
 #pragma unroll
-            for (int u = 0; u < 2; u++)
-                if (k + 32 * u < ne) acc += warp_transpose_sum9(v[u]);
-        }
-        return acc;
-    };
-    auto store = [&](int idx, float acc) {
-        if (vis && lane == 0) atomicOr(vis + idx, vis_bit);  // this view sees Gaussian idx
-        const int q = sum9_component(lane);
-        if (q < 9 && !(lane & 1)) {
-            float* dst = q < 3 ? dcolor + 3 * idx + q
-                       : q < 5 ? dmean2D + 3 * idx + (q - 3)
-                       : q == 7 ? dconic + 4 * idx + 3
-                       : q < 8 ? dconic + 4 * idx + (q - 5)
-                               : dopac + idx;
-            *dst = acc;
-        }
-    };
-    // Gaussians j and j + nwarps together when both have at most 32 rows (most do:
-    // a Gaussian covers ~20 tiles at 1080p), so one round trip brings two row sets
-    // while the next pair's ranges are fetched; the sums are the ones sum_rows forms.
-    uint32_t a0 = 0, a1 = 0, b0 = 0, b1 = 0;
-    int ia = 0, ib = 0;
-    if (j < V) range(j, a0, a1, ia);
-    if (j + nwarps < V) range(j + nwarps, b0, b1, ib);
-    while (j < V) {
-        const uint32_t jb = j + nwarps, jc = jb + nwarps, jd = jc + nwarps;
-        uint32_t c0 = 0, c1 = 0, d0 = 0, d1 = 0;
-        int ic = 0, id = 0;
-        if (jb < V && a1 - a0 <= 32 && b1 - b0 <= 32) {
-            if (jc < V) range(jc, c0, c1, ic);  // the next pair, in flight meanwhile
-            if (jd < V) range(jd, d0, d1, id);
-            float va[9], vb[9];
-            const float* sa = pgrad + (size_t)(a0 + lane) * 9;
-            const float* sb = pgrad + (size_t)(b0 + lane) * 9;
+                        for (int u = 0; u < 2; u++) {
+                            const uint32_t r = k0 + 32 * (c + u) + lane;
+                            const float* src = pgrad + (size_t)(e0 + r) * 9;
 #pragma unroll
-            for (int q = 0; q < 9; q++) {
-                va[q] = lane < a1 - a0 ? __ldg(sa + q) : 0.f;
-                vb[q] = lane < b1 - b0 ? __ldg(sb + q) : 0.f;
+                            for (int i = 0; i < 9; i++) v[u][i] = r < ne ? __ldg(src + i) : 0.f;
+                        }
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            const float sum = warp_transpose_sum9(v[u]);
+                            if (c + u < groups && q < 9 && !(lane & 1)) s_f[9 * (c + u) + q] = sum;
+                        }
+                    }
+                    __syncthreads();
+                    if (tid < 9)
+#pragma unroll 8
+                        for (uint32_t c = 0; c < groups; c++) acc += s_f[9 * c + tid];
+                    __syncthreads();
+                }
+                if (tid < 9) store(s_id[g], tid, acc);
+                g++;
+                continue;
             }
-            const float ta = warp_transpose_sum9(va), tb = warp_transpose_sum9(vb);
-            store(ia, a1 > a0 ? 0.f + ta : 0.f);
-            store(ib, b1 > b0 ? 0.f + tb : 0.f);
-            j = jc;
-            a0 = c0; a1 = c1; ia = ic;
-            b0 = d0; b1 = d1; ib = id;
-            continue;
+            __syncthreads();
+            if (tid < 32 * (kGatherRanks / kGatherRun)) {
+                // a warp per run: the rows of its Gaussians in [g, h) are consecutive
+                const uint32_t a = max(g, (uint32_t)(tid >> 5) * kGatherRun), z = min(h, (uint32_t)((tid >> 5) + 1) * kGatherRun);
+                const uint32_t n = a < z ? 9 * (s_at[z - 1] + s_ne[z - 1] - s_at[a]) : 0u;
+                const float* src = pgrad + (size_t)s_e0[a] * 9;
+                float* dst = s_f + 9 * s_at[a];
+                for (uint32_t i = lane; i < n; i += 32)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + i)),
+                                 "l"(src + i)
+                                 : "memory");
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            if ((uint32_t)tid < (h - g) * 9) {
+                const uint32_t gi = g + tid / 9, q = tid % 9;
+                const uint32_t ne = s_ne[gi];
+                const float* r = s_f + 9 * s_at[gi] + q;
+                float acc = 0.f;
+                for (uint32_t k = 0; k < ne; k += 32, r += 32 * 9) {
+                    const uint32_t left = ne - k;
+                    auto row = [&](uint32_t i) { return i < left ? r[i * 9] : 0.f; };
+                    float v[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) v[i] = (row(i) + row(i + 16)) + (row(i + 8) + row(i + 24));
+#pragma unroll
+                    for (int i = 0; i < 4; i++) v[i] += v[i + 4];
+                    acc += (v[0] + v[2]) + (v[1] + v[3]);
+                }
+                if (s_id[gi] >= 0) store(s_id[gi], (int)q, acc);
+            }
+            __syncthreads();
+            g = h;
         }
-        // one Gaussian (long row ranges, or the last one): the next ranges in flight
-        if (jc < V) range(jc, c0, c1, ic);
-        store(ia, sum_rows(a0, a1));
-        j = jb;
-        a0 = b0; a1 = b1; ia = ib;
-        b0 = c0; b1 = c1; ib = ic;
+        __syncthreads();  // s_e0 and the like are written again
     }
 }
 
@@ -662,6 +706,11 @@ int grid_for(size_t n, int per_sm)
     return (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, (size_t)sms * per_sm));
 }
 
+uint32_t gather_blocks(int P)
+{
+    return std::min(resident_ctas(pair_grad_gather_kernel, kGatherThreads), ((uint32_t)P + kGatherRanks - 1) / kGatherRanks);
+}
+
 // The two passes over the list (the caller has zeroed the output rows, which the
 // passes overwrite for the listed Gaussians only).  list_bound sizes the grids.
 void fold_launch(const FoldView* views, const FoldView& single, int nviews, int P, const uint32_t* list,
@@ -703,7 +752,7 @@ void launch_preprocess_bwd(const PreParams& p, const GeomState& g, const float* 
 {
     if (p.P <= 0) return;
     const bool sh = p.shs && dsh;
-    pair_grad_gather_kernel<<<grid_for((size_t)p.P, 8), 256, 0, s>>>(g.sort_ids_b, g.total, g.pair_off, pgrad,
+    pair_grad_gather_kernel<<<gather_blocks(p.P), kGatherThreads, 0, s>>>(g.sort_ids_b, g.total, g.pair_off, pgrad,
                                                                      dmean2D, dconic, dcolor, dopac, nullptr, 0u,
                                                                      0xffffffffu);
     note_launches(1);
@@ -720,7 +769,7 @@ void launch_pair_grad_gather(const GeomState& g, const float* pgrad, long long r
 {
     if (P <= 0) return;
     const uint32_t r = rows < 0 ? 0u : (rows > 0xffffffffll ? 0xffffffffu : (uint32_t)rows);
-    pair_grad_gather_kernel<<<grid_for((size_t)P, 8), 256, 0, s>>>(g.sort_ids_b, g.total, g.pair_off, pgrad,
+    pair_grad_gather_kernel<<<gather_blocks(P), kGatherThreads, 0, s>>>(g.sort_ids_b, g.total, g.pair_off, pgrad,
                                                                    dmean2D, dconic, dcolor, dopac, vis, vis_bit, r);
     note_launches(1);
 }
