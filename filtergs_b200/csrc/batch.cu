@@ -368,13 +368,13 @@ int fgs_batch_forward(void* handle, void* stream)
                 launch_duplicate(v.g, v.b, (uint32_t)B->P, (uint32_t)v.cap, v.pre.W, v.pre.H, v.tile_bits, vs);
             }
             StageTimer t(FGS_STAGE_TILE_SORT, vs);
-            launch_tile_sort(v.g, v.b, v.cap, v.tile_bits, v.pre.W, v.pre.H, vs, v.g.total);
+            launch_tile_sort(v.g, v.b, v.cap, v.tile_bits, vs, v.g.total);
         }
         StageTimer t(FGS_STAGE_RANGES, vs);
         LongList lng{};
         if (rc.rule_long())
             lng = LongList{B->d_long, long_ctr, B->total_tiles, B->h_begin[vi], v.g.total, nullptr, nullptr};
-        launch_ranges(v.b, v.im, v.cap, v.num_tiles, vs, v.g.total, lng);
+        launch_ranges(v.g, v.b, v.im, v.cap, B->P, v.pre.W, v.num_tiles, vs, v.g.total, lng);
     }
     for (int i = 0; i < ns; i++) {
         cudaEventRecord(B->joined[i], B->aux[i]);

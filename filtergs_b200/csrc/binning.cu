@@ -65,8 +65,6 @@ struct SortSmem {
 
 // One onesweep pass over `n` 32-bit keys with 32-bit values.
 //   vals_in == nullptr: values are the element indices.
-//   rec_out != nullptr (last tile pass): also gathers the per-Gaussian render
-//   record of each value into sorted position.
 //   n_dev != nullptr: the live count is min(n, *n_dev) (the grid covers n).
 // Persistent: each CTA takes chunks from the counter until none is left, so a
 // grid sized for a bound costs nothing for the chunks that are not live.  Per
@@ -83,14 +81,14 @@ struct SortSmem {
 // view and beside seven other views in a batch, takes 512: at least 2048 keys per chunk
 // are then four per thread instead of eight, a shorter chain of ranks.
 // A 1080p view of 2M Gaussians with 2.1M pairs: the four depth passes 84 -> 70 us, the two
-// tile passes 126 -> 110; a 256x256 view of 10K Gaussians, all six passes: 59 -> 51 us.
+// tile passes 126 -> 110 (62 without the records, which place_kernel writes); a 256x256 view
+// of 10K Gaussians, all six passes: 59 -> 51 us.
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
     onesweep_kernel(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
                     const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ vals_out, uint32_t n, int shift,
                     int nbits, const uint32_t* __restrict__ pass_hist, uint32_t* status, uint32_t* chunk_counter,
-                    unsigned* err, const PairRecord* __restrict__ grec, PairRecord* __restrict__ rec_out,
-                    const unsigned long long* __restrict__ n_dev, const int2* __restrict__ erow, int gx,
+                    unsigned* err, const unsigned long long* __restrict__ n_dev,
                     unsigned long long wait_ns = kWaitLimitNs, uint32_t skip_chunk = 0xffffffffu)
 {
     constexpr int kWarps = kThreads / 32, kItemsMin = kSortTileMin / kThreads;
@@ -197,20 +195,6 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
             }
             if (keys_out) keys_out[gp] = k;
             vals_out[gp] = v;
-            if (rec_out) {
-                // The record also carries the pair's emission index: the Gaussian's first
-                // pair plus this tile's row-major place in its tile rectangle (the order in
-                // which emit_pairs_kernel emitted them), from the row base and width that
-                // pair_offsets_kernel left per Gaussian.  The backward writes the pair's
-                // gradients there, so each Gaussian's pairs are contiguous and are summed
-                // in a fixed order.
-                PairRecord r = grec[v];
-                const int2 er = __ldg(erow + v);
-                const uint32_t ty = k / (uint32_t)gx, tx = k - ty * (uint32_t)gx;
-                r.c.w = __uint_as_float((uint32_t)er.x + ty * (uint32_t)er.y + tx);
-                r.c.z = __uint_as_float(block_mask(r, (float)(tx * kTileX), (float)(ty * kTileY)));
-                rec_out[gp] = r;
-            }
         }
         __syncthreads();  // shared buffers are reused by the next chunk
     }
@@ -403,13 +387,11 @@ __global__ void __launch_bounds__(256)
 // neighbours needs a zeroed table first and 16 bytes per pair of traffic (9.4 us plus the
 // memset for 1.75M pairs; this one 5 us for both).  The same warps list the tiles that the
 // launch rule renders in bands, one atomic per warp and bin.
-__global__ void __launch_bounds__(128) ranges_kernel(const uint32_t* __restrict__ tile, uint32_t K,
-                                                     uint2* __restrict__ ranges, uint32_t num_tiles,
-                                                     const unsigned long long* __restrict__ n_dev, LongList lng)
+__device__ __forceinline__ void find_ranges(const uint32_t* __restrict__ tile, uint32_t K, uint2* __restrict__ ranges,
+                                            uint32_t num_tiles, uint32_t warp, const LongList& lng)
 {
-    if (n_dev) K = (uint32_t)min((unsigned long long)K, *n_dev);
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 31 + lane;
+    const uint32_t t = warp * 31 + lane;
     uint32_t lo = 0, hi = K;  // the first pair whose tile is >= t lies in [lo, hi]
     while (lo < hi) {
         const uint32_t q = (hi - lo) >> 2;
@@ -453,6 +435,70 @@ __global__ void __launch_bounds__(128) ranges_kernel(const uint32_t* __restrict_
     }
 }
 
+// What follows the tile sort: the first range_blocks blocks find the tiles' ranges, the others
+// write the pairs' records in sorted order, 32 per warp.  A warp moves these as 96 items of 16
+// bytes, lane by lane along the records, both from the Gaussians' table and to the sorted
+// list, and meets them whole in shared memory in between.  The last sort pass wrote the records
+// before, at one block of 1024 threads per SM, eight to sixteen records in a row per thread;
+// with 2048 threads per SM their masks (some 200 instructions each) and the gathers overlap,
+// and so do the searches, which wait for memory.  2.1M pairs: last pass and ranges
+// 90 us, last pass and this launch 75.
+constexpr int kPlaceThreads = 256;
+__global__ void __launch_bounds__(kPlaceThreads, 6)
+    place_kernel(const uint32_t* __restrict__ tile, const uint32_t* __restrict__ vals, uint32_t K,
+                 const unsigned long long* __restrict__ n_dev, uint2* __restrict__ ranges, uint32_t num_tiles,
+                 LongList lng, uint32_t range_blocks, const PairRecord* __restrict__ grec,
+                 const int2* __restrict__ erow, uint32_t P, uint32_t gx, PairRecord* __restrict__ rec_out, unsigned* err)
+{
+    __shared__ float4 s_rec[kPlaceThreads / 32][96];
+    if (n_dev) K = (uint32_t)min((unsigned long long)K, *n_dev);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x < range_blocks) {
+        find_ranges(tile, K, ranges, num_tiles, blockIdx.x * (kPlaceThreads / 32) + warp, lng);
+        return;
+    }
+    const uint32_t p0 = (blockIdx.x - range_blocks) * kPlaceThreads + 32 * warp, p = p0 + lane;
+    if (p0 >= K) return;  // (the same on the whole warp)
+    float4* W = s_rec[warp];
+    uint32_t k = 0, v = 0xffffffffu;
+    if (p < K) {
+        k = __ldg(tile + p);
+        v = __ldg(vals + p);
+        if (v >= P) {  // cannot happen with consistent histograms; never read out of bounds
+            set_error(err, FGS_ERR_OVERFLOW);
+            v = 0xffffffffu;
+        }
+    }
+    int2 er = make_int2(0, 0);
+    if (v != 0xffffffffu) er = __ldg(erow + v);
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+        const uint32_t q = 32 * t + lane, j = q / 3, part = q - 3 * j;
+        const uint32_t vj = __shfl_sync(0xffffffffu, v, j);
+        W[q] = vj != 0xffffffffu ? __ldg(reinterpret_cast<const float4*>(grec + vj) + part) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncwarp();
+    if (v != 0xffffffffu) {
+        // The record also carries the pair's emission index: the Gaussian's first pair plus
+        // this tile's row-major place in its tile rectangle (the order in which
+        // emit_pairs_kernel emitted them), from the row base and width that
+        // pair_offsets_kernel left per Gaussian.  The backward writes the pair's gradients
+        // there, so each Gaussian's pairs are contiguous and are summed in a fixed order.
+        const PairRecord r = {W[3 * lane], W[3 * lane + 1], W[3 * lane + 2]};
+        const uint32_t ty = k / gx, tx = k - ty * gx;
+        W[3 * lane + 2].z = __uint_as_float(block_mask(r, (float)(tx * kTileX), (float)(ty * kTileY)));
+        W[3 * lane + 2].w = __uint_as_float((uint32_t)er.x + ty * (uint32_t)er.y + tx);
+    }
+    __syncwarp();
+    float4* out = reinterpret_cast<float4*>(rec_out + p0);
+    const uint32_t n = 3 * min(32u, K - p0);
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+        const uint32_t q = 32 * t + lane;
+        if (q < n) out[q] = W[q];
+    }
+}
+
 inline uint32_t chunks_of(long long n, int tile) { return (uint32_t)((n + tile - 1) / tile); }
 
 // Test hook of the first depth-sort pass (fgs_debug_lookback_fault): the chunk
@@ -491,7 +537,7 @@ void launch_depth_sort(const GeomState& g, int P, cudaStream_t s)
     for (int pass = 0; pass < 4; pass++) {
         onesweep_kernel<kDepthThreads><<<grid, kDepthThreads, smem, s>>>(
             kin[pass], kout[pass], vin[pass], vout[pass], n, 8 * pass, 8, g.hist + pass * kRadix,
-            g.status + (size_t)pass * nch * kRadix, g.counters + pass, g.err, nullptr, nullptr, V, nullptr, 1,
+            g.status + (size_t)pass * nch * kRadix, g.counters + pass, g.err, V,
             pass ? kWaitLimitNs : g_fault_wait_ns, pass ? 0xffffffffu : g_fault_skip_chunk);
     }
 }
@@ -517,12 +563,10 @@ void launch_duplicate(const GeomState& g, const BinState& b, uint32_t V, uint32_
     note_launches(2);
 }
 
-void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int tile_bits, int W, int H, cudaStream_t s,
+void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int tile_bits, cudaStream_t s,
                       const unsigned long long* n_dev)
 {
     if (K <= 0) return;
-    const int gx = (W + kTileX - 1) / kTileX;  // tile ids are row-major over gx columns
-    (void)H;
     const uint32_t n = (uint32_t)K;
     const uint32_t nch = chunks_of(n, kSortTileMin);
     const size_t smem = sizeof(SortSmem<kTileThreads>);
@@ -531,29 +575,29 @@ void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int ti
     const uint32_t* ki = (passes & 1) ? b.tile_a : b.tile_b;
     const uint32_t* vi = (passes & 1) ? b.val_a : b.val_b;
     for (int pass = 0; pass < passes; pass++) {
-        const bool last = pass == passes - 1;
         const int nbits = min(8, tile_bits - 8 * pass);
         uint32_t* ko = (ki == b.tile_a) ? b.tile_b : b.tile_a;
         uint32_t* vo = (vi == b.val_a) ? b.val_b : b.val_a;
         onesweep_kernel<kTileThreads><<<grid, kTileThreads, smem, s>>>(
             ki, ko, vi, vo, n, 8 * pass, nbits, g.hist + (4 + pass) * kRadix,
-            b.status + (size_t)pass * nch * kRadix, g.counters + 4 + pass, g.err, last ? g.grec : nullptr,
-            last ? b.rec : nullptr, n_dev, g.erow, gx);
+            b.status + (size_t)pass * nch * kRadix, g.counters + 4 + pass, g.err, n_dev);
         ki = ko;
         vi = vo;
     }
     note_launches(passes);
 }
 
-void launch_ranges(const BinState& b, const ImageState& im, long long K, int num_tiles, cudaStream_t s,
-                   const unsigned long long* n_dev, const LongList& lng)
+void launch_ranges(const GeomState& g, const BinState& b, const ImageState& im, long long K, int P, int W, int num_tiles,
+                   cudaStream_t s, const unsigned long long* n_dev, const LongList& lng)
 {
     if (K <= 0) {
         cudaMemsetAsync(im.ranges, 0, sizeof(uint2) * (size_t)num_tiles, s);
         return;
     }
-    const uint32_t warps = chunks_of(num_tiles, 31);
-    ranges_kernel<<<(warps + 3) / 4, 128, 0, s>>>(b.tile_b, (uint32_t)K, im.ranges, (uint32_t)num_tiles, n_dev, lng);
+    const uint32_t range_blocks = chunks_of(chunks_of(num_tiles, 31), kPlaceThreads / 32);
+    place_kernel<<<range_blocks + chunks_of(K, kPlaceThreads), kPlaceThreads, 0, s>>>(
+        b.tile_b, b.val_b, (uint32_t)K, n_dev, im.ranges, (uint32_t)num_tiles, lng, range_blocks, g.grec, g.erow,
+        (uint32_t)P, (uint32_t)((W + kTileX - 1) / kTileX), b.rec, g.err);
     note_launches(1);
 }
 

@@ -448,11 +448,12 @@ int fgs_forward_render(const fgs_raster_args* a, void* geom, void* image, void* 
             launch_duplicate(g, bc.b, (uint32_t)p.P, (uint32_t)K, W, H, tbits, s);
         }
         StageTimer t(FGS_STAGE_TILE_SORT, s);
-        launch_tile_sort(g, bc.b, K, tbits, W, H, s);
+        launch_tile_sort(g, bc.b, K, tbits, s);
     }
     {
         StageTimer t(FGS_STAGE_RANGES, s);
-        launch_ranges(bc.b, im, K, num_tiles, s, nullptr, long_list_of(rc, im, num_tiles, g.total, stats ? &bc.b : nullptr));
+        launch_ranges(g, bc.b, im, K, a->P, W, num_tiles, s, nullptr,
+                      long_list_of(rc, im, num_tiles, g.total, stats ? &bc.b : nullptr));
     }
     {
         StageTimer t_render(FGS_STAGE_RENDER_FWD, s);

@@ -113,7 +113,7 @@ void launch_duplicate(const GeomState& g, const BinState& b, uint32_t V, uint32_
                       cudaStream_t s);
 int sort_chunk_size();
 // K is the pair count, or the capacity when n_dev (device-side count) is given.
-void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int tile_bits, int W, int H, cudaStream_t s,
+void launch_tile_sort(const GeomState& g, const BinState& b, long long K, int tile_bits, cudaStream_t s,
                       const unsigned long long* n_dev = nullptr);
 // Buffers zeroed by one launch (whole 4-byte words from 4-byte boundaries).
 struct ZeroList {
@@ -174,8 +174,9 @@ struct LongList {
     uint32_t* kv_cnt;
 };
 // Tile ranges of the K sorted pairs; lists the long tiles when lng.list is set.
-void launch_ranges(const BinState& b, const ImageState& im, long long K, int num_tiles, cudaStream_t s,
-                   const unsigned long long* n_dev, const LongList& lng);
+// The tiles' ranges and the sorted pairs' records.
+void launch_ranges(const GeomState& g, const BinState& b, const ImageState& im, long long K, int P, int W, int num_tiles,
+                   cudaStream_t s, const unsigned long long* n_dev, const LongList& lng);
 // K: the pair count (or capacity) of b, for the statistics' zeroing when long tiles are split;
 // totals as in LongList (the long tiles are in im when the launch rule is in force).
 void launch_render_fwd(const RenderConfig& c, int W, int H, const ImageState& im, const BinState& b, long long K,

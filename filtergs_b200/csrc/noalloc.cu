@@ -110,11 +110,11 @@ int fgs_forward_noalloc(const fgs_raster_args* a, int* radii, float* out_color, 
     if (K > 0) {
         cudaMemsetAsync(b.status, 0, sizeof(uint32_t) * (b.status_words + b.scan_words), s);
         launch_duplicate(g, b, (uint32_t)p.P, (uint32_t)K, p.W, p.H, tbits, s);
-        launch_tile_sort(g, b, K, tbits, p.W, p.H, s);
+        launch_tile_sort(g, b, K, tbits, s);
     }
     const RenderConfig rc = get_render_config();
     if (rc.rule_long()) cudaMemsetAsync(im.long_ctr, 0, kLongCtrBytes, s);
-    launch_ranges(b, im, K, num_tiles, s, nullptr, long_list_of(rc, im, num_tiles, g.total, nullptr));
+    launch_ranges(g, b, im, K, p.P, p.W, num_tiles, s, nullptr, long_list_of(rc, im, num_tiles, g.total, nullptr));
     launch_render_fwd(rc, p.W, p.H, im, b, K, g.total, a->background, out_color, out_point_id, out_point_weight_pixel,
                       out_point_weight, false, g.err, s);
     cudaMemcpyAsync(&err, g.err, sizeof(err), cudaMemcpyDeviceToHost, s);
