@@ -2,20 +2,20 @@
 // (antialias/cuda_rasterizer/forward.cu:406-567, backward.cu:399-557).
 //
 // One CTA per 16x16 tile.  The tile's sorted pairs are contiguous 48-byte
-// records (written by the last sort pass), so each record batch is ONE bulk copy
+// records (written after the tile sort), so each record batch is ONE bulk copy
 // (cp.async.bulk, the TMA engine's 1-D form) into shared memory, completed on an
 // mbarrier.  Three record buffers keep two batches in flight while the current
 // one is composited.  A warp owns a block of pixels (PPT of one column per lane), and a
 // record carries the mask of the tile's eight 8x4 blocks it can reach (block_mask,
-// written by the sort): one ballot per 32 records tells a warp which to composite.
+// written with it): one ballot per 32 records tells a warp which to composite.
 //
-// Both directions are bound by instruction issue (86% and 73% of the issue slots of
+// Both directions are bound by instruction issue (83% and 78% of the issue slots of
 // 1080p views), so two pixels of a lane are composited per instruction with packed
 // fma / mul / add.f32x2, which round each half as the scalar operation does, and a
 // record's masks are formed once, not once per warp and direction.  Sixteen 1080p views
-// (27.9M pairs) at the best shape: forward 4.81 -> 3.68 ms, backward 7.81 -> 6.55 ms; one
-// such view: 361 -> 284 and 505 -> 372 us; 10,000 Gaussians at 256x256: 72 -> 44 and
-// 93 -> 58 us at 2 pixels per lane.
+// (27.9M pairs): forward 4.81 -> 3.67 ms, backward 7.81 -> 6.93 ms (6.55 with the sums of 8x8
+// quads, whose order depended on the shape); one such view: 361 -> 296 and 505 -> 415 us with
+// the gradient buffers zeroed; 10,000 Gaussians at 256x256: 72 -> 60 and 93 -> 48 us.
 //
 // Per-Gaussian outputs that the reference updates from every pixel (the
 // racy out_point_weight max, the KPC statistics, the backward's 9 gradient
@@ -917,8 +917,9 @@ __global__ void __launch_bounds__(LongTile<BW, BH>::kThreads)
 // in flight meanwhile), compacts the survivors (about a seventh) in order, loads only
 // those records and tests only those against the bands.  Per pixel the same records in
 // the same order with the same arithmetic as on the tile path.  8M-node LoD views at
-// 1080p with 2.7M / 6.4M / 8.5M pairs: 0.60 / 1.08 / 1.06 ms; in bands that stage every
-// record 0.78 / 1.42 / 1.36; one CTA per tile 1.66 / 2.63 / 5.59.
+// 1080p with 2.7M / 6.4M / 8.5M pairs: 0.60 / 1.08 / 1.06 ms with masks of 8x8 quads (a
+// quarter survived; the 8x4 blocks take another tenth off: 462 -> 418 us of a smaller view);
+// in bands that stage every record 0.78 / 1.42 / 1.36; one CTA per tile 1.66 / 2.63 / 5.59.
 constexpr int kUnitIn = 512, kUnitRecs = 256, kUnits = 8, kUnitThreads = 128;
 
 struct UnitSmem {
@@ -1277,7 +1278,8 @@ __device__ __forceinline__ bool bwd_pair_step(BwdPixels<NP>& s, int q, const flo
 // instructions, this about 20 with the stores: with it, and with warps that do not wait for
 // one another at each batch, the backward of a 1237x823 view of 300K Gaussians takes 263 us
 // (308 before), of 2M at 1080p 465 (476), of 16 such views 7.07 ms (7.25), of six smaller
-// views 1.70 ms (2.03), of 10K at 256x256 50 us (62).  Two steps at a time, in half the shared
+// views 1.70 ms (2.03), of 10K at 256x256 50 us (62).  (The single-view figures hold the zeroing of
+// the gradient buffers, whose shares each thread then still divided for: 415 us at 2M without.)  Two steps at a time, in half the shared
 // memory and with one more CTA per SM: 491 us at 2M.
 template <bool kAtomic>
 __device__ __forceinline__ void add_step_sums(const StepSums& u, float (*acc)[9], int count)
@@ -1851,23 +1853,26 @@ void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const
                         s);
 }
 
-// The backward's shape until a caller sets one: 2 pixels per lane and 32-record batches.
-// The gradients' bits are those of every shape of 2 or 4 pixels per lane, so the choice is free
-// (tests/test_gpu_composite.py); measured, in us, at (2, 32) / (2, 64) / (4, 32): a view of 256 tiles
-// 50 / 49 / 81, 4056 tiles 263 / 274 / 279, 8160 tiles 465 / 493 / 452, 16 of these 7065 / 7703 /
-// 7218, six views of 1200 to 5700 tiles 1705 / 1745 / 2045.
-constexpr int kBwdRulePpt = 2, kBwdRuleBatch = 32;
+// The backward's shapes.  Its batches hold 32 records whatever batch a caller sets: the gradients'
+// bits do not depend on it, and as warps do not wait for one another at a batch, larger ones only
+// take shared memory from resident warps.  Until a caller sets a shape it is 2 pixels per lane.
+// Measured, in us, at (2, 32) / (2, 64) / (4, 32): a view of 256 tiles 50 / 49 / 81, 4056 tiles 263 /
+// 274 / 279, 8160 tiles 465 / 493 / 452, 16 of these 7065 / 7703 / 7218, six views of 1200 to 5700
+// tiles 1705 / 1745 / 2045.
+constexpr int kBwdRulePpt = 2, kBwdBatch = 32;
+#define FGS_BWD_DISPATCH(FN, ...)                                        \
+    do {                                                                 \
+        const int ppt_ = g_cfg.own_shape ? g_cfg.bwd_ppt : kBwdRulePpt;  \
+        if (ppt_ == 1) FN<1, kBwdBatch>(__VA_ARGS__);                    \
+        else if (ppt_ == 2) FN<2, kBwdBatch>(__VA_ARGS__);               \
+        else FN<4, kBwdBatch>(__VA_ARGS__);                              \
+    } while (0)
 
 void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
                              uint32_t* queue, const ZeroList& zero, int consistent, unsigned* err, cudaStream_t s)
 {
     cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
-    if (!g_cfg.own_shape)
-        bwd_multi_launch<kBwdRulePpt, kBwdRuleBatch>(views, begin, nviews, total_tiles, queue, zero, consistent, err,
-                                                     s);
-    else
-        FGS_RENDER_DISPATCH(bwd_multi_launch, g_cfg.bwd_ppt, g_cfg.bwd_batch, views, begin, nviews, total_tiles, queue,
-                            zero, consistent, err, s);
+    FGS_BWD_DISPATCH(bwd_multi_launch, views, begin, nviews, total_tiles, queue, zero, consistent, err, s);
     note_launches(1);
 }
 
@@ -1875,11 +1880,7 @@ void launch_render_bwd(int W, int H, const ImageState& im, const BinState& b, co
                        const float* dL_dpix, int consistent, const ZeroList& zero, unsigned* err, cudaStream_t s)
 {
     const int gx = (W + kTileX - 1) / kTileX, gy = (H + kTileY - 1) / kTileY;
-    if (!g_cfg.own_shape)
-        bwd_launch<kBwdRulePpt, kBwdRuleBatch>(gx * gy, im, b, W, H, bg, dL_dpix, consistent, zero, err, s);
-    else
-        FGS_RENDER_DISPATCH(bwd_launch, g_cfg.bwd_ppt, g_cfg.bwd_batch, gx * gy, im, b, W, H, bg, dL_dpix, consistent,
-                            zero, err, s);
+    FGS_BWD_DISPATCH(bwd_launch, gx * gy, im, b, W, H, bg, dL_dpix, consistent, zero, err, s);
     note_launches(1);
 }
 

@@ -347,9 +347,11 @@ int fgs_profile_enable(int on);
 /* Render kernel shape used by forward/backward in this process (no reference
  * counterpart; the reference hard-codes one pixel per thread and 256-record
  * batches): pixels per thread 1|2|4 and shared-memory batch 64|128|256 for
- * each of the forward and backward compositing kernels.  Until this is
- * called the library chooses them per launch from the view's tiles and pairs
- * (the get call then reads 2, 256, 2, 256); the autotuner
+ * each of the forward and backward compositing kernels (the backward stages
+ * 32 records at a time whatever its batch says; it is kept and read back).
+ * Until this is called the library chooses the shapes itself, the forward's
+ * long tiles from the view's tiles and pairs (the get call then reads
+ * 2, 256, 2, 256); the autotuner
  * (filtergs_b200/autotune.py) sets them from measurements.  cfg: int[4] out. */
 int fgs_set_render_config(int fwd_ppt, int fwd_batch, int bwd_ppt, int bwd_batch);
 int fgs_get_render_config(int *cfg);
