@@ -12,7 +12,7 @@
 //
 // Every sort pass is one onesweep kernel (Adinets & Merrill 2022): chunks
 // take ascending indices from an atomic counter, rank their keys with
-// warp-level match/ballot, and learn their global offsets per digit from a
+// warp-level ballots, and learn their global offsets per digit from a
 // decoupled look-back over the preceding chunks (fgs_scan.cuh: windowed,
 // bounded; on timeout the kernel records FGS_ERR_TIMEOUT and moves on).
 #include "fgs_common.cuh"

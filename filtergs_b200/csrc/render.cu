@@ -1098,7 +1098,7 @@ __device__ __forceinline__ void unit_loop(unsigned char* dyn, const TileArgs* __
 // ---------------------------------------------------------------- the launch rule's forward
 // Used until a caller sets a shape or a split: 2 pixels per lane and 128-record batches
 // (over all shapes within 5% of the best on views of 256x256 to 1080p, one or sixteen),
-// and the long tiles (listed by ranges_kernel) in units by the same launch: its first
+// and the long tiles (listed by place_kernel) in units by the same launch: its first
 // blocks, one resident set, take them from the queue before the tiles' own blocks start,
 // so a view without long tiles pays for no second kernel and no listing pass (10 us of
 // 300), only for blocks that leave at once.
