@@ -74,10 +74,11 @@ class _RasterizeGaussians(torch.autograd.Function):
     def backward(ctx, grad_out_color, radii, point_id, point_weight_pixel, point_weight):
         num_rendered = ctx.num_rendered
         rs = ctx.raster_settings
-        if grad_out_color is None:  # the image is not part of the loss
-            grad_out_color = torch.zeros(3, int(rs.image_height), int(rs.image_width), device=ctx.saved_tensors[1].device)
         colors_precomp, means3D, scales, rotations, cov3Ds_precomp, radii, sh, geomBuffer, binningBuffer, \
             imgBuffer = ctx.saved_tensors
+        if grad_out_color is None:  # the image is not part of the loss
+            grad_out_color = torch.zeros(3, int(rs.image_height), int(rs.image_width), dtype=torch.float32,
+                                         device=means3D.device)
         args = (rs.bg, means3D, radii, colors_precomp, scales, rotations, rs.scale_modifier, cov3Ds_precomp,
                 rs.viewmatrix, rs.projmatrix, rs.tanfovx, rs.tanfovy, grad_out_color, sh, rs.sh_degree, rs.campos,
                 geomBuffer, num_rendered, binningBuffer, imgBuffer, rs.debug)
