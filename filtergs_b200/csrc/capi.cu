@@ -269,17 +269,19 @@ uint32_t resident_ctas_query(const void* kernel, int threads, size_t smem)
     };
     static std::mutex mu;
     static std::vector<Entry> cache;
+    // The opt-in belongs to the context, not to the device: made for every launch, it also holds in
+    // the context that follows a device reset.  (A refusal leaves its error for the check after the launch.)
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lock(mu);
     for (const Entry& e : cache)
         if (e.k == kernel && e.threads == threads && e.dev == dev && e.smem == smem) return e.ctas;
-    int sms = 148, per = 1;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
-    const uint32_t r = (uint32_t)(sms * (per > 0 ? per : 1));
+    int sms = 148, per = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess || per < 1)
+        return (uint32_t)sms;  // not kept: the next call asks again
+    const uint32_t r = (uint32_t)(sms * per);
     cache.push_back(Entry{kernel, threads, dev, smem, r});
     return r;
 }

@@ -94,9 +94,9 @@ int tile_bits_for(int num_tiles);
 
 // ---------------------------------------------------------------- launchers
 // Resident CTAs of a kernel on this device (persistent grids never exceed it), with `smem` bytes
-// of dynamic shared memory, which the first query on a device opts the kernel in to.
-// Cached per (kernel, block size, shared memory, device): kernels of the same signature have
-// their own entries.
+// of dynamic shared memory, which every query opts the kernel in to: one query per launch.
+// The count is cached per (kernel, block size, shared memory, device): kernels of the same
+// signature have their own entries.
 uint32_t resident_ctas_query(const void* kernel, int threads, size_t smem);
 template <typename Kern>
 inline uint32_t resident_ctas(Kern k, int threads, size_t smem = 0)
