@@ -103,9 +103,36 @@ __device__ __forceinline__ void row_window(const float* __restrict__ row, int c,
 // is kept as three maps (d/dmu_x, d/dE[x^2], d/dE[xy]) of `gpitch` floats per row, zero past
 // the last output; the SSIM values of the tile are summed in a fixed order.
 // 1920x1080, three channels: 118 -> 80 us (scalar sums, 32x16 tiles before), the same bits.
-constexpr int kRowsPer = 8;  // outputs of one column per thread
+constexpr int kRowsPer = 8;   // outputs of one column per thread
 constexpr int kLossThreads = kTX * kTY / kRowsPer;
-constexpr int kSeg = 8;      // outputs of one row per row-pass item
+constexpr int kSeg = 8;       // outputs of one row per row-pass item
+constexpr int kSumRows = 16;  // rows of values that one float32 partial sum spans
+
+// A tile's float32 partial sums, one per kSumRows rows, from a thread's sums over the upper and
+// lower four of its eight rows: lanes by a tree, then the four strips of four rows in turn.
+// (Sums over all 32 rows would carry twice as many values in float32 before the double sum of
+// loss_reduce_kernel.)  Partials lie [channel][rows / kSumRows][tile column].
+constexpr int kStrips = kSumRows / (kRowsPer / 2);
+static_assert(kStrips == 4 && kLossThreads / 32 * 2 == kTY / kSumRows * kStrips, "two strips per warp");
+__device__ __forceinline__ void tile_partials(float upper, float lower, float (&red)[kTY / kSumRows][kStrips], int rows,
+                                              float* __restrict__ partial)
+{
+    const int tid = threadIdx.x;
+    // both trees at once: after lanes 16 apart, the lower half warp goes on with the upper rows' sum
+    const bool second = tid & 16;
+    float v = (second ? lower : upper) + __shfl_xor_sync(0xffffffffu, second ? upper : lower, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((tid & 15) == 0) (&red[0][0])[tid >> 4] = v;
+    __syncthreads();
+    const int blocks = (rows + kSumRows - 1) / kSumRows, by = blockIdx.y * (kTY / kSumRows) + tid;
+    if (tid < kTY / kSumRows && by < blocks) {
+        float t = 0.f;
+#pragma unroll
+        for (int k = 0; k < kStrips; k++) t += red[tid][k];
+        partial[((size_t)blockIdx.z * blocks + by) * gridDim.x + blockIdx.x] = t;
+    }
+}
 
 template <bool kVec>
 __global__ void __launch_bounds__(kLossThreads)
@@ -115,7 +142,7 @@ __global__ void __launch_bounds__(kLossThreads)
     __shared__ __align__(16) float sx[kIn][kPitch], sy[kIn][kPitch];
     __shared__ ulonglong2 hq[kIn][kTX + 1];  // {mean x, mean y}, {mean x^2, mean y^2} along the row
     __shared__ float hp[kIn][kTX + 1];       // mean x y
-    __shared__ float red[kLossThreads / 32];
+    __shared__ float red[kTY / kSumRows][kStrips];
     const int Wo = W - kHalo, Ho = H - kHalo;
     const int c = blockIdx.z;
     const int ox0 = blockIdx.x * kTX, oy0 = blockIdx.y * kTY;
@@ -178,7 +205,7 @@ __global__ void __launch_bounds__(kLossThreads)
             p[q] = __fmaf_rn(f2_lo(w[tap(j)]), uv, p[q]);
         }
     }
-    float s = 0.f;
+    float s[2] = {0.f, 0.f};
     const size_t plane = (size_t)gpitch * Ho;
     float* gm = gmap + (size_t)c * 3 * plane;
 #pragma unroll
@@ -199,22 +226,13 @@ __global__ void __launch_bounds__(kLossThreads)
             gm[o] = -ssim_grad_scale * d_m1;
             gm[plane + o] = -ssim_grad_scale * d_e11;
             gm[2 * plane + o] = -ssim_grad_scale * d_e12;
-            s += ss;
+            s[rr / (kRowsPer / 2)] += ss;
         } else if (ox < gpitch && oy < Ho) {
             const size_t o = (size_t)oy * gpitch + ox;
             gm[o] = gm[plane + o] = gm[2 * plane + o] = 0.f;
         }
     }
-    // fixed-order block sum of the tile's SSIM values
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) red[tid >> 5] = s;
-    __syncthreads();
-    if (tid == 0) {
-        float t = 0.f;
-        for (int k = 0; k < kLossThreads / 32; k++) t += red[k];
-        partial[((size_t)c * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = t;
-    }
+    tile_partials(s[0], s[1], red, Ho, partial);
 }
 
 // ---------------------------------------------------------------- loss gradient per pixel
@@ -232,7 +250,7 @@ __global__ void __launch_bounds__(kLossThreads)
     __shared__ __align__(16) float sg[3][kIn][kPitch];  // from column px0 - kHalo - kLead
     __shared__ float2 ha[kIn][kTX + 1];
     __shared__ float hb[kIn][kTX + 1];
-    __shared__ float red[kLossThreads / 32];
+    __shared__ float red[kTY / kSumRows][kStrips];
     const int Ho = H - kHalo;
     const int c = blockIdx.z;
     const int px0 = blockIdx.x * kTX, py0 = blockIdx.y * kTY;
@@ -310,7 +328,7 @@ __global__ void __launch_bounds__(kLossThreads)
             b[q] = __fmaf_rn(f2_lo(w[tap(j)]), v, b[q]);
         }
     }
-    float l1 = 0.f;
+    float l1[2] = {0.f, 0.f};
 #pragma unroll
     for (int rr = 0; rr < kRowsPer; rr++) {
         const int py = py0 + ty0 + rr;
@@ -320,18 +338,10 @@ __global__ void __launch_bounds__(kLossThreads)
             const float d = xv - yv;
             const float sgn = d > 0.f ? 1.f : (d < 0.f ? -1.f : 0.f);
             dpred[o] = f2_lo(a[rr]) + 2.f * xv * f2_hi(a[rr]) + yv * b[rr] + l1_grad_scale * sgn;
-            l1 += fabsf(d);
+            l1[rr / (kRowsPer / 2)] += fabsf(d);
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
-    if (lane == 0) red[tid >> 5] = l1;
-    __syncthreads();
-    if (tid == 0) {
-        float t = 0.f;
-        for (int k = 0; k < kLossThreads / 32; k++) t += red[k];
-        partial[((size_t)c * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = t;
-    }
+    tile_partials(l1[0], l1[1], red, H, partial);
 }
 
 // sums[0] += sum(l1 partials), sums[1] += sum(ssim partials), by one block in a
@@ -345,8 +355,11 @@ __global__ void __launch_bounds__(1024) loss_reduce_kernel(const float* __restri
 {
     __shared__ double s_a[32], s_b[32];
     double a = 0.0, b = 0.0;
-    for (int i = threadIdx.x; i < nl1; i += blockDim.x) a += l1p[i];
-    for (int i = threadIdx.x; i < ns; i += blockDim.x) b += sp[i];
+    // (eight loads in flight at a time, added in turn)
+#pragma unroll 8
+    for (int i = threadIdx.x; i < nl1; i += 1024) a += l1p[i];
+#pragma unroll 8
+    for (int i = threadIdx.x; i < ns; i += 1024) b += sp[i];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
@@ -629,8 +642,8 @@ size_t fgs_loss_scratch_bytes(int width, int height)
 {
     if (width <= kHalo || height <= kHalo) return 0;
     const size_t Wo = (size_t)width - kHalo, Ho = (size_t)height - kHalo;
-    const size_t nso = 3 * ((Wo + kTX - 1) / kTX) * ((Ho + kTY - 1) / kTY);
-    const size_t nl1 = 3 * (((size_t)width + kTX - 1) / kTX) * (((size_t)height + kTY - 1) / kTY);
+    const size_t nso = 3 * ((Wo + kTX - 1) / kTX) * ((Ho + kSumRows - 1) / kSumRows);
+    const size_t nl1 = 3 * (((size_t)width + kTX - 1) / kTX) * (((size_t)height + kSumRows - 1) / kSumRows);
     return sizeof(float) * (9 * ((Wo + 3) / 4 * 4) * Ho + nso + nl1) + 256;
 }
 
@@ -646,7 +659,9 @@ int fgs_loss_l1_ssim(int width, int height, const float* pred, const float* targ
     const dim3 go((Wo + kTX - 1) / kTX, (Ho + kTY - 1) / kTY, 3);
     const dim3 gp((width + kTX - 1) / kTX, (height + kTY - 1) / kTY, 3);
     float* sp = gmap + (size_t)9 * gpitch * Ho;
-    float* l1p = sp + (size_t)go.x * go.y * go.z;
+    const int nso = (int)(3 * go.x) * ((Ho + kSumRows - 1) / kSumRows);
+    const int nl1 = (int)(3 * gp.x) * ((height + kSumRows - 1) / kSumRows);
+    float* l1p = sp + nso;
     static const Window win = make_window();
     const bool vec = width % 4 == 0 && ((reinterpret_cast<uintptr_t>(pred) | reinterpret_cast<uintptr_t>(target)) & 15u) == 0;
     if (vec)
@@ -657,7 +672,7 @@ int fgs_loss_l1_ssim(int width, int height, const float* pred, const float* targ
                                                                gpitch, sp);
     loss_grad_kernel<<<gp, kLossThreads, 0, s>>>(width, height, pred, target, win, gmap, gpitch, l1_grad_scale,
                                                  dL_dpred, l1p);
-    loss_reduce_kernel<<<1, 1024, 0, s>>>(l1p, (int)(gp.x * gp.y * gp.z), sp, (int)(go.x * go.y * go.z), sums);
+    loss_reduce_kernel<<<1, 1024, 0, s>>>(l1p, nl1, sp, nso, sums);
     note_launches(3);
     return cudaGetLastError() == cudaSuccess ? FGS_OK : FGS_ERR_CUDA;
 }
