@@ -446,13 +446,13 @@ def autotune(args, fn, key, rank):
         return None
     from filtergs_b200.autotune import tune_render
     it = iter(range(1 << 30))
-    tuned, table = tune_render(lambda: fn(next(it)), key=key,
-                               splits=((0, 0), (512, 0), (512, 1), (512, 2), (512, 3), (4096, 2)))
+    _, table = tune_render(lambda: fn(next(it)), key=key,
+                           splits=((0, 0), (512, 0), (512, 1), (512, 2), (512, 3), (4096, 2)))
     if rank == 0:
-        print(f"autotune {key[0]} (ppt,batch)->(fwd ms, bwd ms), then long-tile split->fwd ms: " +
+        print(f"autotune {key[0]} library's choice, (ppt,batch)->(fwd ms, bwd ms), then long-tile split->fwd ms: " +
               ", ".join(f"{k}:{v[0]:.3f}/{v[1]:.3f}" for k, v in sorted(table.items(), key=lambda kv: str(kv[0]))),
               file=sys.stderr)
-    return list(tuned) + list(_lib.get_render_split())
+    return list(_lib.render_settings())  # 0, 0 for a shape and 0, -1 for a split that the library chooses
 
 
 def measure_plain(args, mod, scene, views, bg, dev, dist, rank, ours=True, clocks=None, profile=False):

@@ -159,32 +159,56 @@ def profile_read(reset=True):
     return {n: (float(ms[i]), int(calls[i])) for i, n in enumerate(STAGES)}
 
 
-def set_render_config(fwd_ppt=2, fwd_batch=256, bwd_ppt=2, bwd_batch=256):
-    """Fix the compositing shapes (until the first call the library chooses them per launch)."""
-    check(lib().fgs_set_render_config(int(fwd_ppt), int(fwd_batch), int(bwd_ppt), int(bwd_batch)),
+class Chosen(int):
+    """A compositing setting that the library chooses: the number get_render_* report for it.  Given back to
+    set_render_* (all settings of a direction, or of the split), it leaves the choice to the library again, so
+    setting what was read restores what was in force."""
+
+
+# what the launch rule of csrc/render.cu uses (the backward has no batch of its own: 32 records whatever is set)
+_RULE_FWD, _RULE_BWD, _RULE_SPLIT = ((Chosen(2), Chosen(128)), (Chosen(2), Chosen(256)), (Chosen(0), Chosen(0)))
+
+
+def _setting(values, chosen):
+    """The C values of one direction's settings: `chosen` when the library is to choose them."""
+    return chosen if all(isinstance(v, Chosen) for v in values) else tuple(int(v) for v in values)
+
+
+def set_render_config(fwd_ppt=_RULE_FWD[0], fwd_batch=Chosen(256), bwd_ppt=_RULE_BWD[0], bwd_batch=_RULE_BWD[1]):
+    """Fix the compositing shapes; a direction without arguments, or with Chosen ones, is left to the library."""
+    check(lib().fgs_set_render_config(*_setting((fwd_ppt, fwd_batch), (0, 0)), *_setting((bwd_ppt, bwd_batch), (0, 0))),
           "fgs_set_render_config")
 
 
 BAND_SHAPES = {0: (16, 2), 1: (8, 4), 2: (4, 4), 3: (4, 2)}
 
 
-def set_render_split(min_records=0, band_shape=0):
+def set_render_split(min_records=_RULE_SPLIT[0], band_shape=_RULE_SPLIT[1]):
     """Forward tiles with at least min_records pairs are rendered in bands (0: never) of
-    BAND_SHAPES[band_shape] pixels, one warp each."""
-    check(lib().fgs_set_render_split(int(min_records), int(band_shape)), "fgs_set_render_split")
+    BAND_SHAPES[band_shape] pixels, one warp each.  Without arguments, or with Chosen ones, the
+    library chooses the long tiles (while the forward's shape is its choice too)."""
+    check(lib().fgs_set_render_split(*_setting((min_records, band_shape), (0, -1))), "fgs_set_render_split")
+
+
+def render_settings():
+    """The six settings as the C interface has them: (fwd_ppt, fwd_batch, bwd_ppt, bwd_batch, min_records,
+    band_shape), 0 and 0 for a shape and (0, -1) for a split that the library chooses."""
+    cfg, split = (C.c_int * 4)(), (C.c_int * 2)()
+    check(lib().fgs_get_render_config(C.cast(cfg, vp)), "fgs_get_render_config")
+    check(lib().fgs_get_render_split(C.cast(split, vp)), "fgs_get_render_split")
+    return tuple(cfg) + tuple(split)
 
 
 def get_render_split():
     """(min_records, band_shape) of the forward's long-tile bands."""
-    cfg = (C.c_int * 2)()
-    check(lib().fgs_get_render_split(C.cast(cfg, vp)), "fgs_get_render_split")
-    return int(cfg[0]), int(cfg[1])
+    split = render_settings()[4:]
+    return _RULE_SPLIT if split == (0, -1) else split
 
 
 def get_render_config():
-    cfg = (C.c_int * 4)()
-    check(lib().fgs_get_render_config(C.cast(cfg, vp)), "fgs_get_render_config")
-    return tuple(cfg)
+    """(fwd_ppt, fwd_batch, bwd_ppt, bwd_batch) of the compositing kernels."""
+    cfg = render_settings()[:4]
+    return (cfg[:2] if cfg[0] else _RULE_FWD) + (cfg[2:] if cfg[2] else _RULE_BWD)
 
 
 def launch_count():

@@ -719,7 +719,7 @@ int fgs_debug_lookback_fault(unsigned int skip_chunk, unsigned long long wait_ns
 int fgs_set_render_config(int fwd_ppt, int fwd_batch, int bwd_ppt, int bwd_batch)
 {
     const RenderConfig cur = get_render_config();
-    const RenderConfig c{fwd_ppt, fwd_batch, bwd_ppt, bwd_batch, cur.fwd_split, cur.fwd_band, true, cur.own_split};
+    const RenderConfig c{fwd_ppt, fwd_batch, bwd_ppt, bwd_batch, cur.fwd_split, cur.fwd_band};
     if (!valid_render_config(c)) return FGS_ERR_ARG;
     set_render_config(c);
     return FGS_OK;
@@ -730,7 +730,6 @@ int fgs_set_render_split(int min_records, int band_shape)
     RenderConfig c = get_render_config();
     c.fwd_split = min_records;
     c.fwd_band = band_shape;
-    c.own_split = true;
     if (!valid_render_config(c)) return FGS_ERR_ARG;
     set_render_config(c);
     return FGS_OK;

@@ -277,15 +277,19 @@ void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const
 void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
                              uint32_t* queue, const ZeroList& zero, int consistent, unsigned* err, cudaStream_t s);
 
-// Render kernel shape: pixels per thread {1,2,4} and records per shared-memory batch {64,128,256}.
+// Render kernel shape: pixels per thread {1,2,4} and records per shared-memory batch {64,128,256};
+// 0 and 0 leave a direction's shape, and a band shape of -1 the long tiles, to the launch rule
+// (render.cu), as they are until a caller sets them.
 struct RenderConfig {
     int fwd_ppt, fwd_batch, bwd_ppt, bwd_batch;
     int fwd_split;  // forward: tiles with at least this many records are rendered in bands (0: never)
-    int fwd_band;   // band shape: 0 = 16x2, 1 = 8x4, 2 = 4x4, 3 = 4x2 pixels per warp
-    // Until a caller sets them, the shapes and the split are chosen per launch (render.cu):
-    bool own_shape;  // the four shape fields were set (fgs_set_render_config)
-    bool own_split;  // the split fields were set (fgs_set_render_split)
-    bool rule_long() const { return !own_shape && !own_split; }  // long tiles by the launch rule
+    int fwd_band;   // band shape: 0 = 16x2, 1 = 8x4, 2 = 4x4, 3 = 4x2 pixels per warp; -1: launch rule
+    bool own_fwd() const { return fwd_ppt != 0; }
+    bool own_bwd() const { return bwd_ppt != 0; }
+    bool own_split() const { return fwd_band >= 0; }
+    // long tiles in units by the launch rule: its kernel has one shape (a caller's own shape without
+    // a split of its own renders every tile whole)
+    bool rule_long() const { return !own_fwd() && !own_split(); }
 };
 LongList long_list_of(const RenderConfig& c, const ImageState& im, int num_tiles, const unsigned long long* totals,
                       const BinState* stats);

@@ -1598,7 +1598,7 @@ __global__ void __launch_bounds__(256 / PPT, bwd_multi_min_ctas<PPT>())
 }  // namespace
 
 namespace {
-RenderConfig g_cfg{2, 256, 2, 256, 0, 0, false, false};
+RenderConfig g_cfg{0, 0, 0, 0, 0, -1};
 
 // Dynamic shared memory of a forward launch: the whole FwdSmem with statistics,
 // up to its statistics sums without.
@@ -1740,10 +1740,11 @@ void bwd_launch(int grid, const ImageState& im, const BinState& b, int W, int H,
 
 bool valid_render_config(const RenderConfig& c)
 {
-    auto ok_p = [](int v) { return v == 1 || v == 2 || v == 4; };
-    auto ok_b = [](int v) { return v == 64 || v == 128 || v == 256; };
-    return ok_p(c.fwd_ppt) && ok_p(c.bwd_ppt) && ok_b(c.fwd_batch) && ok_b(c.bwd_batch) && c.fwd_split >= 0 &&
-           c.fwd_band >= 0 && c.fwd_band <= 3;
+    auto shape = [](int p, int b) {
+        return (p == 0 && b == 0) || ((p == 1 || p == 2 || p == 4) && (b == 64 || b == 128 || b == 256));
+    };
+    const bool split = c.own_split() ? c.fwd_split >= 0 && c.fwd_band <= 3 : c.fwd_split == 0 && c.fwd_band == -1;
+    return shape(c.fwd_ppt, c.fwd_batch) && shape(c.bwd_ppt, c.bwd_batch) && split;
 }
 void set_render_config(const RenderConfig& c) { g_cfg = c; }
 RenderConfig get_render_config() { return g_cfg; }
@@ -1775,7 +1776,7 @@ void launch_render_fwd(const RenderConfig& c, int W, int H, const ImageState& im
         else fwd_rule_launch<kWeights>(gx * gy, a, im, err, s);
         return;
     }
-    FGS_RENDER_DISPATCH(fwd_launch, c.own_shape ? c.fwd_ppt : kRulePpt, c.own_shape ? c.fwd_batch : kRuleBatch,
+    FGS_RENDER_DISPATCH(fwd_launch, c.own_fwd() ? c.fwd_ppt : kRulePpt, c.own_fwd() ? c.fwd_batch : kRuleBatch,
                         gx * gy, im, b, K, W, H, bg, out_color, point_id, pw_pixel, point_weight, stats, c.fwd_split,
                         c.fwd_band, err, s);
 }
@@ -1848,7 +1849,7 @@ void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const
             views, begin, nviews, total_tiles, queue, long_list, long_ctr, err);
         return;
     }
-    FGS_RENDER_DISPATCH(fwd_multi_launch, c.own_shape ? c.fwd_ppt : kRulePpt, c.own_shape ? c.fwd_batch : kRuleBatch,
+    FGS_RENDER_DISPATCH(fwd_multi_launch, c.own_fwd() ? c.fwd_ppt : kRulePpt, c.own_fwd() ? c.fwd_batch : kRuleBatch,
                         views, begin, nviews, total_tiles, queue, long_list, long_ctr, c.fwd_split, c.fwd_band, err,
                         s);
 }
@@ -1862,7 +1863,7 @@ void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const
 constexpr int kBwdRulePpt = 2, kBwdBatch = 32;
 #define FGS_BWD_DISPATCH(FN, ...)                                        \
     do {                                                                 \
-        const int ppt_ = g_cfg.own_shape ? g_cfg.bwd_ppt : kBwdRulePpt;  \
+        const int ppt_ = g_cfg.own_bwd() ? g_cfg.bwd_ppt : kBwdRulePpt;  \
         if (ppt_ == 1) FN<1, kBwdBatch>(__VA_ARGS__);                    \
         else if (ppt_ == 2) FN<2, kBwdBatch>(__VA_ARGS__);               \
         else FN<4, kBwdBatch>(__VA_ARGS__);                              \

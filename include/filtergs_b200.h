@@ -349,16 +349,19 @@ int fgs_profile_enable(int on);
  * batches): pixels per thread 1|2|4 and shared-memory batch 64|128|256 for
  * each of the forward and backward compositing kernels (the backward stages
  * 32 records at a time whatever its batch says; it is kept and read back).
- * Until this is called the library chooses the shapes itself, the forward's
- * long tiles from the view's tiles and pairs (the get call then reads
- * 2, 256, 2, 256); the autotuner
- * (filtergs_b200/autotune.py) sets them from measurements.  cfg: int[4] out. */
+ * 0 pixels and 0 records leave a direction to the library, as both are until
+ * this is called; the get call reads 0 and 0 then, so that setting what was
+ * read restores what was in force.  A forward shape of the caller's renders
+ * long tiles whole unless fgs_set_render_split says otherwise.  The autotuner
+ * (filtergs_b200/autotune.py) sets the shapes from measurements.
+ * cfg: int[4] out.                                                           */
 int fgs_set_render_config(int fwd_ppt, int fwd_batch, int bwd_ppt, int bwd_batch);
 int fgs_get_render_config(int *cfg);
 /* Forward: tiles with at least min_records tile/Gaussian pairs are rendered in bands of pixels, one
  * warp per band and four bands per CTA, longest tiles first, before the other tiles (min_records 0:
- * never).  Until this or fgs_set_render_config is called, the library chooses the tiles per view.
- * band_shape: 0 = 16x2, 1 = 8x4, 2 = 4x4, 3 = 4x2 pixels per band.  The outputs do not change; long
+ * never).  band_shape: 0 = 16x2, 1 = 8x4, 2 = 4x4, 3 = 4x2 pixels per band.  (0, -1), in force until this
+ * is called: while the forward's shape is the library's too, it chooses the long tiles per view and
+ * renders them in units of 8x4 pixels inside the tiles' launch.  The outputs do not change; long
  * tiles stop being the critical path of the forward.  Process-wide, like the above.
  * fgs_get_render_split: cfg int[2] out (min_records, band_shape).                                   */
 int fgs_set_render_split(int min_records, int band_shape);
