@@ -396,7 +396,7 @@ int fgs_batch_backward(void* handle, void* stream)
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t P = (size_t)B->P;
     if (!B->g_means3D || !B->g_opacity) return FGS_ERR_ARG;
-    // the shared outputs are zeroed by the compositing's launch (the fold writes the rows of
+    // the shared outputs are zeroed with the compositing (the fold writes the rows of
     // the Gaussians some view saw), as are the views' visibility bits
     const bool sh = B->views[0].pre.shs && B->g_sh;
     ZeroList zero;

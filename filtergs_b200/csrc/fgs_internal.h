@@ -182,8 +182,9 @@ void launch_ranges(const GeomState& g, const BinState& b, const ImageState& im, 
 void launch_render_fwd(const RenderConfig& c, int W, int H, const ImageState& im, const BinState& b, long long K,
                        const unsigned long long* totals, const float* bg, float* out_color, int* point_id,
                        float* pw_pixel, float* point_weight, bool stats, unsigned* err, cudaStream_t s);
-// zero: buffers the launch also zeroes (the gradient outputs: 568 MB at 2M Gaussians with SH 3, whose
-// writing then costs next to nothing beside compositing that is bound by instruction issue).
+// zero: buffers that are zeroed too (the gradient outputs: 568 MB at 2M Gaussians with SH 3): by the launch
+// itself, a share per tile, where that costs next to nothing beside compositing that is bound by
+// instruction issue; else by one of their own before it (zeroed_in_shares, render.cu).
 void launch_render_bwd(int W, int H, const ImageState& im, const BinState& b, const float* bg,
                        const float* dL_dpix, int consistent, const ZeroList& zero, unsigned* err, cudaStream_t s);
 // Densification statistics a training step keeps per Gaussian (null pointers: off).
@@ -273,7 +274,7 @@ struct TileArgs {
 void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const uint32_t* begin, int nviews,
                              uint32_t total_tiles, uint32_t* queue, uint32_t* long_list, uint32_t* long_ctr,
                              unsigned* err, cudaStream_t s);
-// zero: buffers that this launch zeroes, a share after each tile: its stores pass while others composite.
+// zero: as in launch_render_bwd (a share after each tile: its stores pass while others composite).
 void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
                              uint32_t* queue, const ZeroList& zero, int consistent, unsigned* err, cudaStream_t s);
 

@@ -1869,11 +1869,33 @@ constexpr int kBwdRulePpt = 2, kBwdBatch = 32;
         else FN<4, kBwdBatch>(__VA_ARGS__);                              \
     } while (0)
 
+// Whether the compositing launch zeroes the buffers, a share per tile, or a launch of its own before
+// it, at the memory's rate.  A block stores 15 to 50 GB/s, so with few tiles the shares are the
+// backward's time: 2M Gaussians with SH 3 (568 MB), one view, shares / own launch in us: 1 tile
+// 9606 / 176, 16 tiles 731 / 178, 64 tiles 238 / 186, 256 tiles 195 / 193, 1024 tiles 231 / 237, 8160 tiles
+// 660 / 737; two views in one launch, tiles of both: 32 852 / 178, 128 318 / 193, 512 218 / 215, 1024
+// 214 / 232.  200K Gaussians: 64 tiles (888 KB each) 61 / 56, 256 tiles (222 KB) 53 / 60; 20K: 4 tiles
+// (1.4 MB) 63 / 45, 16 (355 KB) 43 / 44, 64 (89 KB) 42 / 51.  From four tiles per SM on the blocks together
+// store at the memory's rate, and up to 256 KB a share costs less than the launch.
+bool zeroed_in_shares(const ZeroList& z, uint32_t tiles)
+{
+    size_t words = 0;
+    for (int b = 0; b < z.n; b++) words += z.words[b];
+    if (words * 4 <= (size_t)tiles * (256 << 10)) return true;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return tiles >= 4u * (uint32_t)sms;
+}
+
 void launch_render_bwd_multi(const TileArgs* views, const uint32_t* begin, int nviews, uint32_t total_tiles,
                              uint32_t* queue, const ZeroList& zero, int consistent, unsigned* err, cudaStream_t s)
 {
     cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
-    FGS_BWD_DISPATCH(bwd_multi_launch, views, begin, nviews, total_tiles, queue, zero, consistent, err, s);
+    const bool shares = zeroed_in_shares(zero, total_tiles);
+    if (!shares) launch_zero(zero, s);
+    FGS_BWD_DISPATCH(bwd_multi_launch, views, begin, nviews, total_tiles, queue, shares ? zero : ZeroList{}, consistent,
+                     err, s);
     note_launches(1);
 }
 
@@ -1881,7 +1903,9 @@ void launch_render_bwd(int W, int H, const ImageState& im, const BinState& b, co
                        const float* dL_dpix, int consistent, const ZeroList& zero, unsigned* err, cudaStream_t s)
 {
     const int gx = (W + kTileX - 1) / kTileX, gy = (H + kTileY - 1) / kTileY;
-    FGS_BWD_DISPATCH(bwd_launch, gx * gy, im, b, W, H, bg, dL_dpix, consistent, zero, err, s);
+    const bool shares = zeroed_in_shares(zero, (uint32_t)(gx * gy));
+    if (!shares) launch_zero(zero, s);
+    FGS_BWD_DISPATCH(bwd_launch, gx * gy, im, b, W, H, bg, dL_dpix, consistent, shares ? zero : ZeroList{}, err, s);
     note_launches(1);
 }
 
