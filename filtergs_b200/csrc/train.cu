@@ -338,10 +338,25 @@ __global__ void __launch_bounds__(kLossThreads)
             const float d = xv - yv;
             const float sgn = d > 0.f ? 1.f : (d < 0.f ? -1.f : 0.f);
             dpred[o] = f2_lo(a[rr]) + 2.f * xv * f2_hi(a[rr]) + yv * b[rr] + l1_grad_scale * sgn;
-            l1[rr / (kRowsPer / 2)] += fabsf(d);
         }
+        l1[rr / (kRowsPer / 2)] += fabsf(xs[rr] - ys[rr]);  // (0 outside the image)
     }
     tile_partials(l1[0], l1[1], red, H, partial);
+}
+
+// Thread t's sum of p[t], p[t + 1024], ... in turn, 16 loads in flight (1920x1080 has twelve per
+// thread; one at a time their latency is the kernel's time).
+__device__ __forceinline__ double partial_sum(const float* __restrict__ p, int n)
+{
+    double a = 0.0;
+    for (int i = threadIdx.x; i < n; i += 16 * 1024) {
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) v[k] = i + k * 1024 < n ? __ldg(p + i + k * 1024) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; k++) a += v[k];
+    }
+    return a;
 }
 
 // sums[0] += sum(l1 partials), sums[1] += sum(ssim partials), by one block in a
@@ -354,12 +369,7 @@ __global__ void __launch_bounds__(1024) loss_reduce_kernel(const float* __restri
                                                            double* __restrict__ sums)
 {
     __shared__ double s_a[32], s_b[32];
-    double a = 0.0, b = 0.0;
-    // (eight loads in flight at a time, added in turn)
-#pragma unroll 8
-    for (int i = threadIdx.x; i < nl1; i += 1024) a += l1p[i];
-#pragma unroll 8
-    for (int i = threadIdx.x; i < ns; i += 1024) b += sp[i];
+    double a = partial_sum(l1p, nl1), b = partial_sum(sp, ns);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
