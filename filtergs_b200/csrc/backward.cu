@@ -1,11 +1,12 @@
-// Per-Gaussian backward: 2D-covariance, projection, SH and scale/rotation
-// gradients in one kernel (antialias/cuda_rasterizer/backward.cu:20-396,
-// where computeCov2DCUDA and preprocessCUDA are two launches).
+// Per-Gaussian backward (antialias/cuda_rasterizer/backward.cu:20-396):
+// the per-pair gradients' sums (pair_grad_gather_kernel), then 2D-covariance,
+// projection and scale/rotation gradients in one kernel and the SH gradients
+// in two (fold_geo, fold_shcoef and fold_shdir), for one view or a batch.
 //
 // The 3D covariance is recomputed from scale/rotation (it is a pure function
-// of them) instead of being kept in the geometry buffer.  Every output row is
-// written, zeros for Gaussians the forward culled, so the caller needs no
-// zero-initialisation.
+// of them) instead of being kept in the geometry buffer.  The rows of the listed
+// Gaussians (the visible ones) are written; the launch that precedes these has
+// zeroed every output row, so those of the others are zero.
 //
 // mode FGS_BACKWARD_REF_COMPAT reproduces the reference: the 2D covariance is
 // dilated by +0.3 (backward.cu:197-199) whatever the forward did, and
@@ -150,7 +151,8 @@ __device__ __forceinline__ void load_sh_row(const float* __restrict__ shrow, int
 // in a run of 16 ranks the first block had seven of more than 512 rows, and the kernel
 // waited for it.  Row layout: dcolor r,g,b | dmean2D x,y | dconic x,y,w | dopacity.  vis
 // (optional): the view sets vis_bit in vis[idx] for every Gaussian it sees.
-// Bound by the latency of the copies and the scattered stores.  131K Gaussians with 2.1M rows
+// Bound by its barriers (a block waits for its copies, then for its sums) and by the issue of the
+// sums (65% of the slots).  131K Gaussians with 2.1M rows
 // (75 MB): 49 us, 10K with 90K rows 4; with a warp per Gaussian, a row per lane and a
 // shuffle tree per 32 rows 74 and 23.
 constexpr int kGatherRanks = 16, kGatherRun = 4, kGatherRows = 512, kGatherThreads = 160;

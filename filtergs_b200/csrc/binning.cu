@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(256)
 // latency of its ~11 dependent steps, where a pass over all pairs that compares
 // neighbours needs a zeroed table first and 16 bytes per pair of traffic (9.4 us plus the
 // memset for 1.75M pairs; this one 5 us for both).  The same warps list the tiles that the
-// launch rule renders in bands, one atomic per warp and bin.
+// launch rule renders in units, one atomic per warp and bin.
 __device__ __forceinline__ void find_ranges(const uint32_t* __restrict__ tile, uint32_t K, uint2* __restrict__ ranges,
                                             uint32_t num_tiles, uint32_t warp, const LongList& lng)
 {

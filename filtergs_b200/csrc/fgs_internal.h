@@ -67,8 +67,8 @@ struct ImageState {
     float* final_T;     // [N]
     uint32_t* n_contrib; // [N]
     uint2* ranges;      // [tiles]
-    uint32_t* long_list; // [32][tiles] tiles rendered in bands, binned by log2(records) (render.cu)
-    uint32_t* long_ctr;  // [34] 0: long tiles, 1: band queue, 2 + b: tiles in bin b
+    uint32_t* long_list; // [32][tiles] long tiles (units or bands), binned by log2(records) (render.cu)
+    uint32_t* long_ctr;  // [34] 0: long tiles, 1: their queue, 2 + b: tiles in bin b
 };
 ImageState image_views(void* base, int W, int H);
 size_t image_bytes(int W, int H);
@@ -162,7 +162,7 @@ __device__ __forceinline__ void zero_share(const ZeroList& z, uint32_t part)
 
 constexpr size_t kLongCtrBytes = 34 * sizeof(uint32_t);  // ImageState::long_ctr
 struct RenderConfig;
-// Where the tiles that the launch rule renders in bands are listed (render.cu): list [32][cap]
+// Where the tiles that the launch rule renders in units are listed (render.cu): list [32][cap]
 // binned by log2(records), ctr [34] (zeroed by the caller) and the first id of this view's tiles.
 // totals: the view's {pairs, visible} on the device; kv_*: zeroed for the listed tiles when given.
 struct LongList {
@@ -196,9 +196,9 @@ struct DensifyStats {
 // Per-Gaussian backward of one view.  Screen-space gradients come from the
 // per-pair gradients (pgrad, at the emission index), summed per Gaussian in
 // emission order: dmean2D / dconic / dcolor / dopac are the dense screen-space
-// outputs (rows of visible Gaussians written; the caller zeroes them), the rest are
-// written densely.  The Gaussians the forward found visible (radii > 0) receive
-// gradients.
+// outputs.  The Gaussians the forward found visible (radii > 0) receive gradients: their
+// rows are written, and the caller has zeroed all rows of all outputs (fgs_backward hands
+// them to launch_render_bwd for that).
 void launch_preprocess_bwd(const PreParams& p, const GeomState& g, const float* pgrad, float* dmean2D,
                            float* dconic, float* dcolor, float* dopac, float* dmean3D, float* dcov3D, float* dsh,
                            float* dscale, float* drot, int consistent, cudaStream_t s);
@@ -269,7 +269,7 @@ struct TileArgs {
 // Persistent multi-view compositing over the tiles of `nviews` views; begin[v]
 // is the first work item of view v (begin[nviews] == total_tiles); queue is a
 // device counter (zeroed here).
-// long_list: [32 * total_tiles], long_ctr: [34] (bands of long tiles; statistics must be off): scratch, or
+// long_list: [32 * total_tiles], long_ctr: [34] (the long tiles; statistics must be off): scratch, or
 // filled by the views' launch_ranges when the launch rule is in force.
 void launch_render_fwd_multi(const RenderConfig& c, const TileArgs* views, const uint32_t* begin, int nviews,
                              uint32_t total_tiles, uint32_t* queue, uint32_t* long_list, uint32_t* long_ctr,

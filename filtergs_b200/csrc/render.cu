@@ -9,7 +9,7 @@
 // record carries the mask of the tile's eight 8x4 blocks it can reach (block_mask,
 // written with it): one ballot per 32 records tells a warp which to composite.
 //
-// Both directions are bound by instruction issue (83% and 78% of the issue slots of
+// Both directions are bound by instruction issue (80% and 77% of the issue slots of
 // 1080p views), so two pixels of a lane are composited per instruction with packed
 // fma / mul / add.f32x2, which round each half as the scalar operation does, and a
 // record's masks are formed once, not once per warp and direction.  Sixteen 1080p views
@@ -1096,12 +1096,18 @@ __device__ __forceinline__ void unit_loop(unsigned char* dyn, const TileArgs* __
 }
 
 // ---------------------------------------------------------------- the launch rule's forward
-// Used until a caller sets a shape or a split: 2 pixels per lane and 128-record batches
-// (over all shapes within 5% of the best on views of 256x256 to 1080p, one or sixteen),
+// Used until a caller sets a shape or a split: 2 pixels per lane and 128-record batches,
 // and the long tiles (listed by place_kernel) in units by the same launch: its first
 // blocks, one resident set, take them from the queue before the tiles' own blocks start,
 // so a view without long tiles pays for no second kernel and no listing pass (10 us of
-// 300), only for blocks that leave at once.
+// 300), only for blocks that leave at once.  Against the best of the nine shapes without
+// long tiles, in us: a 1237x823 view of 300K Gaussians 199 / 194, one of 2M at 1080p 296 / 289
+// (4 pixels, 64 records), sixteen of these 3679 / 3486 (4, 64), six of mixed sizes 859 / 838, four
+// of 1600x900 692 / 677 (4, 64); 10K Gaussians at 256x256 53 / 35 (1, 256: more warps for few tiles).
+// In a batch the units share the tiles' registers: with every output per view, not the image
+// alone, sixteen 1080p views take 5365 against 4880 in the same shape without them, mixed sizes
+// 3054 / 2722; a tuned shape gets that back.  LoD views of 5.4M pairs 1.50 ms, 10.1 without long
+// tiles, 1.58 in the best bands.
 constexpr int kRulePpt = 2, kRuleBatch = 128;
 static_assert(kUnitThreads == 256 / kRulePpt, "one block size for tiles and units");
 static_assert(sizeof(UnitSmem) <= offsetof(FwdSmem<kRuleBatch>, ksum), "shared memory");
@@ -1172,7 +1178,8 @@ struct BwdPixels {
 // alpha T dL/dpixel (channels 0, 1), w dx, w dy, w dx dx, w dx dy, w dy dy, w and
 // alpha T dL/dpixel (channel 2): neighbours come from one packed instruction.  Pixels are
 // added one after the other, lanes by warp_transpose_sum9 and strips as (0 + 1) + (2 + 3),
-// whatever the block's shape: a training step carries the last bits of these sums on to the
+// at two and at four pixels per lane alike (one pixel per lane adds half strips in four
+// slots, in turn): a training step carries the last bits of these sums on to the
 // next one, where they decide comparisons.
 
 // 1 / x for x in [0.01, 1], with the bits of __fdividef(1, x) there, which spends its time on
@@ -1273,7 +1280,7 @@ __device__ __forceinline__ bool bwd_pair_step(BwdPixels<NP>& s, int q, const flo
 // each takes four sums of every fourth lane (128-bit loads, packed adds) through the first
 // three levels; two exchanges halve the four sums a lane still holds.  The two strips of one
 // record are added to each other first.  kAtomic: two warps share a slot.
-// What bounds the backward is instructions issued (78% of the slots; about 125 per step of 32
+// What bounds the backward is instructions issued (77% of the slots; about 125 per step of 32
 // lanes x 2 pixels).  A butterfly over one step's nine sums takes 12 shuffles and 46
 // instructions, this about 20 with the stores: with it, and with warps that do not wait for
 // one another at each batch, the backward of a 1237x823 view of 300K Gaussians takes 263 us
